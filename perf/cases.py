@@ -92,11 +92,11 @@ def draw(rng):
         return {"kind": kind, "system": "water" if water else "protein",
                 "atoms": rng.randint(150, 500) if water else _log(rng, 1500, 9000),
                 "conf_bias": _log(rng, 40, 1000), "steps": _log(rng, 12, 400), "proposal": proposal,
-                "mesh": rng.choice([0, 0, 32, 48, 54, 64])}
+                "mesh": rng.choice([0, 0, 0, 64])}
     proposal = rng.choice([0, 0, 1, 2])
     unique = rng.choice([1, 2, 5])
     return {"kind": kind, "system": "protein", "atoms": 0 if unique > 1 else _log(rng, 1500, 9000), "unique": unique,
-            "replicas": unique * rng.randint(1, max(1, 60 // unique)), "conf_bias": _log(rng, 100, 1000),
+            "replicas": unique * (2 * rng.randint(0, 30 // unique - 1) + 1), "conf_bias": _log(rng, 100, 1000),
             "steps": _log(rng, 12, 96), "proposal": proposal, "mesh": rng.choice([0, 0, 0, 48]),
             "tuned": rng.random() < 0.5}
 
