@@ -21,6 +21,7 @@ constexpr float kTwoPiF = 6.28318530717958647692f;
 constexpr int kMaxSites = 20;
 constexpr int kMaxPoses = 1024;  // poses per step (confBias limit)
 constexpr int kMaxWords = kMaxPoses / 32;
+constexpr unsigned kFull = 0xffffffffu;
 
 // RNG purposes: high half of the third counter word.
 enum : uint32_t { RP_INSERT = 1, RP_DELETE = 2, RP_MOVE = 3, RP_CLUSTER = 4, RP_PERM = 5, RP_GUMBEL = 6, RP_FB = 7 };
@@ -477,7 +478,9 @@ struct RepDev {
     double* pme_q;          // [n0 * n1 * n2] spread charges of the current state
     double2* pme_spec;      // [n0 * n1 * (n2 / 2 + 1)] transform workspace
     const double* pme_g;    // [n0 * n1 * (n2 / 2 + 1)] influence function
-    int* pme_dirty;         // 1: Q changed since phi was computed
+    const double2* pme_tw;  // roots of unity of the three axes, n0 + n1 + n2 (fft_twiddles)
+    int* pme_dirty;         // [0] 1: Q changed since phi was computed; [1] finished CTAs of the
+                            // mesh update's last pass (the last one clears the dirty marks)
     double pme_bgc;         // K pi / (2 V alpha^2): background energy -bgc Q^2
     double pme_qfix;        // total charge of the fixed atoms
 };
@@ -495,6 +498,38 @@ __device__ __forceinline__ int cell_of(const RepDev& R, float x, float y, float 
     int cy = cell_coord(y, R.start[1], R.invLc[1], R.nc[1]);
     int cz = cell_coord(z, R.start[2], R.invLc[2], R.nc[2]);
     return (cz * R.nc[1] + cy) * R.nc[0] + cx;
+}
+
+// pre[r] = work items of the replicas before r, pre[nrep] = all of them,
+// computed by the whole block (one replica per thread, warp scans, then the
+// warp totals) so that no thread walks the replica list alone.
+template <class Items>
+__device__ __forceinline__ void items_prefix(int nrep, int* pre, int* wtot, Items items) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+    int carry = 0;
+    for (int base = 0; base < nrep; base += blockDim.x) {
+        const int r = base + tid;
+        const int v = r < nrep ? items(r) : 0;
+        int inc = v;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int t = __shfl_up_sync(kFull, inc, off);
+            if (lane >= off) inc += t;
+        }
+        if (lane == 31) wtot[warp] = inc;
+        __syncthreads();
+        int before = 0, tot = 0;
+        for (int w = 0; w < nwarp; ++w) {
+            const int t = wtot[w];
+            if (w < warp) before += t;
+            tot += t;
+        }
+        if (r < nrep) pre[r] = carry + before + inc - v;
+        carry += tot;
+        __syncthreads();
+    }
+    if (tid == 0) pre[nrep] = carry;
+    __syncthreads();
 }
 
 // Centre of insertion pose i (gcmc/cpp/gcmc_energy.h:82-93): grid point + U(0,1]*dx.

@@ -26,7 +26,6 @@ namespace gcmc {
 constexpr int kWarpsE = 8;
 constexpr int kGCap = 128;
 constexpr int kACap = 512;
-constexpr unsigned kFull = 0xffffffffu;
 
 // Sites 2p and 2p+1 of a pose, component-interleaved for the packed (f32x2)
 // pair loop: negated centre-relative coordinates and Coulomb constant * charge.
@@ -998,38 +997,6 @@ __device__ __forceinline__ void nbr_share(const RepDev& R, const StepDesc& D, in
     } else {
         nbr_rows(R, D, i, zi, nsl, lane);
     }
-}
-
-// pre[r] = work items of the replicas before r, pre[nrep] = all of them,
-// computed by the whole block (one replica per thread, warp scans, then the
-// warp totals) so that no thread walks the replica list alone.
-template <class Items>
-__device__ __forceinline__ void items_prefix(int nrep, int* pre, int* wtot, Items items) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
-    int carry = 0;
-    for (int base = 0; base < nrep; base += blockDim.x) {
-        const int r = base + tid;
-        const int v = r < nrep ? items(r) : 0;
-        int inc = v;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int t = __shfl_up_sync(kFull, inc, off);
-            if (lane >= off) inc += t;
-        }
-        if (lane == 31) wtot[warp] = inc;
-        __syncthreads();
-        int before = 0, tot = 0;
-        for (int w = 0; w < nwarp; ++w) {
-            const int t = wtot[w];
-            if (w < warp) before += t;
-            tot += t;
-        }
-        if (r < nrep) pre[r] = carry + before + inc - v;
-        carry += tot;
-        __syncthreads();
-    }
-    if (tid == 0) pre[nrep] = carry;
-    __syncthreads();
 }
 
 // One item of a pose-energy launch (whole warp): item `it` of the replicas'

@@ -159,9 +159,11 @@ struct RepHost {
     double* pme_phi = nullptr;    // potential on the mesh
     double2* pme_spec = nullptr;  // half spectrum
     double* pme_g = nullptr;      // influence function on the half spectrum
-    int* pme_dirty = nullptr;     // 1: the spread charges changed since phi was computed
+    double2* pme_tw = nullptr;    // roots of unity of the three axes
+    int* pme_dirty = nullptr;     // [2] the spread charges changed since phi was computed; the passes' counter
     double pme_key[7] = {0, 0, 0, 0, 0, 0, 0};  // mesh, box and alpha the influence function in pme_g is for
-    const double* pme_g_for = nullptr;          // the buffer it was written to
+    const double* pme_g_for = nullptr;          // the buffers it and the roots were written to
+    const double2* pme_tw_for = nullptr;
 };
 
 }  // namespace
@@ -169,6 +171,7 @@ struct RepHost {
 struct gcmc_ctx {
     int nrep = 0;
     int device = 0;
+    int sms = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     std::vector<RepHost> reps;
@@ -250,7 +253,7 @@ void free_rep(RepHost& h) {
     dfree(h.raw_atoms); dfree(h.raw_groups); dfree(h.raw_grid); dfree(h.raw_bits); dfree(h.bits_blk);
     dfree(h.desc2); dfree(h.pcen2); dfree(h.pslot2); dfree(h.epart2); dfree(h.nbr2); dfree(h.pgum2); dfree(h.plnu2);
     dfree(h.psite2); dfree(h.valid2); dfree(h.abort2); dfree(h.sstep2); dfree(h.pending2); dfree(h.plnu); dfree(h.fpart); dfree(h.fbprop); dfree(h.fbcnt); dfree(h.logF);
-    dfree(h.pme_q); dfree(h.pme_phi); dfree(h.pme_spec); dfree(h.pme_g); dfree(h.pme_dirty);
+    dfree(h.pme_q); dfree(h.pme_phi); dfree(h.pme_spec); dfree(h.pme_g); dfree(h.pme_tw); dfree(h.pme_dirty);
     dfree(h.pbin); dfree(h.tiles); dfree(h.pbin2); dfree(h.tiles2);
     dfree(h.wcost); dfree(h.pnslab); dfree(h.pitem); dfree(h.pnslab2); dfree(h.pitem2);
     h.capn.clear();
@@ -766,6 +769,9 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
         // (a copy from pageable memory is staged before the call returns: tmp may go)
         CK(cudaMemcpyAsync(h.wcost, tmp.data(), sizeof(int) * h.ncell, cudaMemcpyHostToDevice, ctx->stream));
     }
+    AL(h.pme_dirty, 2);  // (every replica: the first of a launch holds the mesh passes' counter)
+    CK(cudaMemsetAsync(h.pme_dirty, 0, 2 * sizeof(int), ctx->stream));
+    d.pme_dirty = h.pme_dirty;
     // smooth PME: mesh and influence function
     h.pme = opt.pme > 0 || (opt.pme == 0 && I->PME != 0);
     d.pme = h.pme ? 1 : 0;
@@ -782,28 +788,33 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
             d.pme_n[a] = n[a];
         }
         const size_t nr = (size_t)n[0] * n[1] * n[2], nh = (size_t)n[0] * n[1] * (n[2] / 2 + 1);
-        AL(h.pme_q, nr); AL(h.pme_phi, nr); AL(h.pme_spec, nh); AL(h.pme_g, nh); AL(h.pme_dirty, 1);
+        AL(h.pme_q, nr); AL(h.pme_phi, nr); AL(h.pme_spec, nh); AL(h.pme_g, nh); AL(h.pme_tw, n[0] + n[1] + n[2]);
         // the influence function depends only on the mesh, the box and alpha: kept between refills
         const double key[7] = {(double)n[0], (double)n[1], (double)n[2], (double)I->cryst[0], (double)I->cryst[1],
                                (double)I->cryst[2], alpha};
-        if (h.pme_g_for != h.pme_g || std::memcmp(key, h.pme_key, sizeof(key)) != 0) {
+        if (h.pme_g_for != h.pme_g || h.pme_tw_for != h.pme_tw || std::memcmp(key, h.pme_key, sizeof(key)) != 0) {
             std::vector<double> G(nh);
             pme_influence(n, I->cryst, alpha, G.data());
             CK(cudaMemcpyAsync(h.pme_g, G.data(), sizeof(double) * nh, cudaMemcpyHostToDevice, ctx->stream));
+            std::vector<double2> tw(n[0] + n[1] + n[2]);
+            fft_twiddles(n[0], tw.data());
+            fft_twiddles(n[1], tw.data() + n[0]);
+            fft_twiddles(n[2], tw.data() + n[0] + n[1]);
+            CK(cudaMemcpyAsync(h.pme_tw, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice, ctx->stream));
             std::memcpy(h.pme_key, key, sizeof(key));
             h.pme_g_for = h.pme_g;
+            h.pme_tw_for = h.pme_tw;
         }
         CK(cudaMemsetAsync(h.pme_phi, 0, sizeof(double) * nr, ctx->stream));
-        const int fft_smem = 2 * kFftLines * kFftMax * (int)sizeof(double2);
-        CK(cudaFuncSetAttribute(k_pme_rows_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, fft_smem));
-        CK(cudaFuncSetAttribute(k_pme_axis, cudaFuncAttributeMaxDynamicSharedMemorySize, fft_smem));
-        CK(cudaFuncSetAttribute(k_pme_rows_c2r, cudaFuncAttributeMaxDynamicSharedMemorySize, fft_smem));
+        for (const void* k : {(const void*)k_pme_fwd_planes, (const void*)k_pme_inv_planes, (const void*)k_pme_axis,
+                              (const void*)k_pme_rows_r2c, (const void*)k_pme_rows_c2r})
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPmeSmemMax));
         for (int a = 0; a < 3; ++a) h.pme_n[a] = n[a];
         d.pme_phi = h.pme_phi;
         d.pme_q = h.pme_q;
         d.pme_spec = h.pme_spec;
         d.pme_g = h.pme_g;
-        d.pme_dirty = h.pme_dirty;
+        d.pme_tw = h.pme_tw;
         d.pme_bgc = (double)kCoulomb * M_PI / (2.0 * V * alpha * alpha);
         double qf = 0.0;
         for (int a = 0; a < h.nfix_atoms; ++a) qf += (double)in.atomInfo[a].charge;
@@ -980,26 +991,57 @@ int energy_warps(int device, int evar, int ebps, int spare_sms) {
 }
 
 
-// Replica r's PME mesh potential from its spread charges on stream s, when
-// they changed since the last update (every pass returns at once otherwise):
-// rows real-to-complex, axis 1, axis 0 with the influence function between
-// its forward and inverse transforms, axis 1 inverse, rows complex-to-real.
-int pme_update(gcmc_ctx* ctx, int r, cudaStream_t s) {
-    RepHost& h = ctx->reps[r];
-    if (!h.pme) return GCMC_OK;
-    const RepDev* rep = ctx->d_reps + r;
-    const int n0 = h.pme_n[0], n1 = h.pme_n[1], n2 = h.pme_n[2], M = n2 / 2 + 1;
-    const int kb = (M + kFftLines - 1) / kFftLines;
-    const int rows = (n0 * n1 + kFftLines - 1) / kFftLines;
-    const size_t sm2 = 2 * kFftLines * (size_t)n2 * sizeof(double2);
-    const size_t sm1 = 2 * kFftLines * (size_t)n1 * sizeof(double2);
-    const size_t sm0 = 2 * kFftLines * (size_t)n0 * sizeof(double2);
-    k_pme_rows_r2c<<<std::min(rows, 4096), kFftThreads, sm2, s>>>(rep);
-    k_pme_axis<<<std::min(n0 * kb, 4096), kFftThreads, sm1, s>>>(rep, 1, -1, 0);
-    k_pme_axis<<<std::min(n1 * kb, 4096), kFftThreads, sm0, s>>>(rep, 0, 0, 1);
-    k_pme_axis<<<std::min(n0 * kb, 4096), kFftThreads, sm1, s>>>(rep, 1, 1, 0);
-    k_pme_rows_c2r<<<std::min(rows, 4096), kFftThreads, sm2, s>>>(rep);
-    k_pme_done<<<1, 32, 0, s>>>(rep);
+// The replicas' mesh sizes (empty without Ewald): the captured mesh passes' grids
+// and shared memory are sized for them.
+std::vector<int> pme_meshes(const gcmc_ctx* ctx) {
+    std::vector<int> m;
+    if (ctx->pme_any)
+        for (const auto& h : ctx->reps)
+            for (int a = 0; a < 3; ++a) m.push_back(h.pme ? h.pme_n[a] : 0);
+    return m;
+}
+
+// The PME mesh potentials of replicas [r0, r0 + cnt) from their spread charges on
+// stream s, where they changed since the last update (the passes of pme.cuh; a
+// CTA that finds every mesh current returns at once).
+int pme_update(gcmc_ctx* ctx, int r0, int cnt, cudaStream_t s) {
+    size_t planes = 0, sm0 = 0, sm1 = 0, sm2 = 0;
+    int nplane = 0, nrow = 0, nax0 = 0, nax1 = 0;
+    for (int r = r0; r < r0 + cnt; ++r) {
+        const RepHost& h = ctx->reps[r];
+        if (!h.pme) continue;
+        const int n0 = h.pme_n[0], n1 = h.pme_n[1], n2 = h.pme_n[2], M = n2 / 2 + 1;
+        planes = std::max(planes, pme_plane_smem(n1, n2));
+        sm0 = std::max(sm0, pme_axis_smem(n0));
+        sm1 = std::max(sm1, pme_axis_smem(n1));
+        sm2 = std::max(sm2, pme_rows_smem(n2));
+        nplane += n0;
+        nrow += (n0 * n1 + 2 * kRowPairs - 1) / (2 * kRowPairs);
+        nax0 += (n1 * M + kAxisLines - 1) / kAxisLines;
+        nax1 += n0 * ((M + kAxisLines - 1) / kAxisLines);
+    }
+    if (nplane == 0) return GCMC_OK;
+    const RepDev* reps = ctx->d_reps + r0;
+    const int sms = std::max(1, ctx->sms);
+    // CTAs that share the items: what fits on the SMs at once, at most the items
+    auto grid = [&](int items, size_t smem, int threads) {
+        const int per_sm = std::max(1, std::min((int)(kPmeSmemMax / smem), 2048 / threads));
+        return std::max(1, std::min(items, sms * per_sm));
+    };
+    const bool whole = planes <= (size_t)kPmeSmemMax;
+    if (whole) {
+        k_pme_fwd_planes<<<grid(nplane, planes, kPlaneThreads), kPlaneThreads, planes, s>>>(reps, cnt);
+    } else {
+        k_pme_rows_r2c<<<grid(nrow, sm2, kAxisThreads), kAxisThreads, sm2, s>>>(reps, cnt);
+        k_pme_axis<<<grid(nax1, sm1, kAxisThreads), kAxisThreads, sm1, s>>>(reps, cnt, 1, -1, 0);
+    }
+    k_pme_axis<<<grid(nax0, sm0, kAxisThreads), kAxisThreads, sm0, s>>>(reps, cnt, 0, 0, 1);
+    if (whole) {
+        k_pme_inv_planes<<<grid(nplane, planes, kPlaneThreads), kPlaneThreads, planes, s>>>(reps, cnt);
+    } else {
+        k_pme_axis<<<grid(nax1, sm1, kAxisThreads), kAxisThreads, sm1, s>>>(reps, cnt, 1, 1, 0);
+        k_pme_rows_c2r<<<grid(nrow, sm2, kAxisThreads), kAxisThreads, sm2, s>>>(reps, cnt);
+    }
     CK(cudaGetLastError());
     return GCMC_OK;
 }
@@ -1242,8 +1284,7 @@ int build_graph(gcmc_ctx* ctx) {
             const int grid = ctx->gridE;
             const int gridf = ctx->gridF;
             for (int s = 0; s < kGraphSteps && e == cudaSuccess; ++s) {
-                for (int r = r0; r < r0 + cnt; ++r)
-                    if (pme_update(ctx, r, side[b]) != GCMC_OK) e = cudaErrorUnknown;
+                if (pme_update(ctx, r0, cnt, side[b]) != GCMC_OK) e = cudaErrorUnknown;
                 if (ctx->fb) {
                     fb_kernel(ctx)<<<gridf, kWarpsG * 32, 0, side[b]>>>(ctx->d_reps + r0, cnt, 1);
                     fb_kernel(ctx)<<<gridf, kWarpsG * 32, 0, side[b]>>>(ctx->d_reps + r0, cnt, 2);
@@ -1333,6 +1374,7 @@ int create_impl(int nrep, const gcmc_replica_in* ins, const gcmc_options* optp, 
     gcmc_ctx* ctx = new gcmc_ctx();
     ctx->nrep = nrep;
     cudaGetDevice(&ctx->device);
+    cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
     int st = GCMC_OK;
     if (stream) {
         ctx->stream = (cudaStream_t)stream;
@@ -1413,6 +1455,7 @@ int refill_impl(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins, const gcmc_
     const bool spec_changed = spec != ctx->spec;
     ctx->spec = spec;
     const bool tiled_before = ctx->tiled, pme_before = ctx->pme_any, dual_before = ctx->dual_any;
+    const std::vector<int> mesh_before = pme_meshes(ctx);
     st = for_each_rep(nrep, ctx->device, [&](int r) { return setup_rep(ctx, r, ins[r], opt); });
     if (st != GCMC_OK) return st;
     if (trace_on()) g_trace[1] = now_ms();
@@ -1432,7 +1475,8 @@ int refill_impl(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins, const gcmc_
     const bool had_graph = ctx->gexec || ctx->gexec_spec[0];
     const bool shape_changed = spec_changed || nb != ctx->branches || opt.energy_blocks_per_sm != ctx->ebps ||
                                fb != ctx->fb || evar != ctx->evar || ctx->tiled != tiled_before ||
-                               ctx->pme_any != pme_before || ctx->dual_any != dual_before ||
+                               ctx->pme_any != pme_before || pme_meshes(ctx) != mesh_before ||
+                               ctx->dual_any != dual_before ||
                                ctx->fb_mixed != mixed_before;
     ctx->fb = fb;
     ctx->evar = evar;
@@ -1887,10 +1931,8 @@ int gcmc_run_profiled(gcmc_ctx* ctx, int32_t nsteps, float* ms_energy, float* ms
     std::vector<cudaEvent_t> ev(3 * (size_t)need);
     for (auto& e : ev) CK(cudaEventCreate(&e));
     for (int i = 0; i < need; ++i) {
-        for (int r = 0; r < ctx->nrep; ++r) {
-            const int st = pme_update(ctx, r, ctx->stream);
-            if (st != GCMC_OK) return st;
-        }
+        const int st = pme_update(ctx, 0, ctx->nrep, ctx->stream);
+        if (st != GCMC_OK) return st;
         CK(cudaEventRecord(ev[3 * i], ctx->stream));
         if (ctx->fb) {
             fb_kernel(ctx)<<<ctx->gridF, kWarpsG * 32, 0, ctx->stream>>>(ctx->d_reps, ctx->nrep, 1);
@@ -2013,7 +2055,7 @@ int gcmc_pme_potential(gcmc_ctx* ctx, int32_t rep, const double* pts, int32_t n,
     if (!ctx || rep < 0 || rep >= ctx->nrep || n < 0 || (n > 0 && (!pts || !out))) return GCMC_ERR_ARG;
     if (!ctx->reps[rep].pme) return GCMC_ERR_ARG;
     if (n == 0) return GCMC_OK;
-    int st = pme_update(ctx, rep, ctx->stream);
+    int st = pme_update(ctx, rep, 1, ctx->stream);
     if (st != GCMC_OK) return st;
     double *dp = nullptr, *dout = nullptr;
     if ((st = dalloc(&dp, (size_t)3 * n)) || (st = dalloc(&dout, (size_t)n))) {
@@ -2089,7 +2131,7 @@ int gcmc_energy_poses(gcmc_ctx* ctx, int32_t rep, const float* xyz, const float*
             st = GCMC_ERR_CUDA;
             break;
         }
-        if ((st = pme_update(ctx, rep, s)) != GCMC_OK) break;
+        if ((st = pme_update(ctx, rep, 1, s)) != GCMC_OK) break;
         k_energy_explicit<<<ctx->gridE, kWarpsE * 32, 0, s>>>(ctx->repdev[rep], dxyz, dq, dt, nsites, dc, dself,
                                                               nposes, nslab, dout, dng);
         if (cudaGetLastError() != cudaSuccess ||
@@ -2257,7 +2299,7 @@ int gcmc_energy_poses_noalloc(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, co
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     if ((st = order_before(ctx, s)) != GCMC_OK) return st;
     {
-        const int pst = pme_update(ctx, rep, s);
+        const int pst = pme_update(ctx, rep, 1, s);
         if (pst != GCMC_OK) return pst;
     }
     k_energy_explicit<<<ctx->gridE, kWarpsE * 32, 0, s>>>(ctx->repdev[rep], d_xyz, d_site_q, d_site_type, nsites,

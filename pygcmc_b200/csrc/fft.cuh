@@ -4,25 +4,30 @@
 // each built from 1D passes over lines held in shared memory.
 //
 // A line of length n = 2^a 3^b (n <= kFftMax) is transformed by the
-// self-sorting Stockham algorithm, decimation in frequency: with the remaining
-// length l (initially n) and the stride s (initially 1, l s = n), a radix-r
-// stage maps x to y by
+// self-sorting Stockham algorithm, decimation in frequency: with the stride s
+// (the product of the radices so far, initially 1) and the remaining length
+// l = n / s, a radix-r stage maps x to y by
 //     y[q + s (r p + k)] = w_l^(p k) sum_j x[q + s (p + j l / r)] w_r^(j k),
-// p < l / r, q < s, k < r, w_m = exp(-+ 2 pi i / m), and continues on y with
-// l / r and r s; the output is in natural order.  Sign -1: forward
-// (exp(-2 pi i k x / n)), +1: inverse, unnormalised.  The twiddles come from
-// sincospi in FP64.
+// p < l / r, q < s, k < r, w_m = exp(-+ 2 pi i / m); the output is in natural
+// order.  Sign -1: forward (exp(-2 pi i k x / n)), +1: inverse, unnormalised.
+// Radices 8, 4, 2 and 3, so that 64 points take two stages and 128 three (a
+// stage costs one pass through shared memory and one barrier); the twiddles
+// w_l^(p k) = w_n^(p k s) come from a table of the n roots (fft_twiddles),
+// which sincospi per butterfly made the transforms' largest cost.
 //
-// The line transform (fft_line) is a __host__ __device__ function over a
-// "thread" index range, so the host test build runs the same arithmetic.
+// The lines of a batch are interleaved (element i of line b at x[i * ld + b],
+// consecutive threads take consecutive lines), so that the 16-byte shared
+// memory accesses of every stage are conflict-free whatever its stride.
+//
+// The stages are __host__ __device__ functions over a "thread" index range, so
+// the host test build runs the same arithmetic.
 #pragma once
+#include <cmath>
 #include <cuda_runtime.h>
 
 namespace gcmc {
 
-constexpr int kFftMax = 256;   // longest line
-constexpr int kFftLines = 8;   // lines per CTA in the batched passes
-constexpr int kFftThreads = 256;
+constexpr int kFftMax = 256;  // longest line
 
 __host__ __device__ inline bool fft_size_ok(int n) {
     if (n < 1 || n > kFftMax) return false;
@@ -31,80 +36,120 @@ __host__ __device__ inline bool fft_size_ok(int n) {
     return n == 1;
 }
 
-// The radices of n, radix 2 first, then 3 (stored in r[], returns the count).
-__host__ __device__ inline int fft_radices(int n, int r[16]) {
-    int c = 0;
-    while (n % 2 == 0) { r[c++] = 2; n /= 2; }
-    while (n % 3 == 0) { r[c++] = 3; n /= 3; }
-    return c;
+// The radix of the stage that leaves the remaining length l: 8 while the power
+// of two left is 8 or 32 and more (16 goes as 4 x 4), then 4, 2, 3.
+__host__ __device__ inline int fft_radix(int l) {
+    if ((l & 7) == 0 && (l & 31) != 16) return 8;
+    if ((l & 3) == 0) return 4;
+    return (l & 1) == 0 ? 2 : 3;
 }
 
 __host__ __device__ inline double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+__host__ __device__ inline double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__host__ __device__ inline double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+// a times sign i
+__host__ __device__ inline double2 cmuli(double2 a, double sign) { return make_double2(-sign * a.y, sign * a.x); }
 
-// exp(sign 2 pi i num / den)
-__host__ __device__ inline double2 twiddle(int num, int den, int sign) {
-    double sn, cs;
-#ifdef __CUDA_ARCH__
-    sincospi(2.0 * (double)num / (double)den, &sn, &cs);
-#else
-    sn = sin(2.0 * 3.14159265358979323846 * (double)num / (double)den);
-    cs = cos(2.0 * 3.14159265358979323846 * (double)num / (double)den);
-#endif
-    return make_double2(cs, sign * sn);
+// The n roots exp(-2 pi i k / n) (host; long double, rounded once).
+inline void fft_twiddles(int n, double2* tw) {
+    const long double two_pi = 6.283185307179586476925286766559005768L;
+    for (int k = 0; k < n; ++k) {
+        const long double th = two_pi * k / n;
+        tw[k] = make_double2((double)std::cos(th), (double)-std::sin(th));
+    }
 }
 
-// One Stockham stage on `nl` lines of length n (line b at x + b * ld), work
-// items t in [t0, t1) step dt (t = line * (n / r) + butterfly).
-__host__ __device__ inline void fft_stage(const double2* x, double2* y, int ld, int nl, int n, int l, int s, int r,
-                                          int sign, int t0, int dt) {
-    const int m = l / r;
-    const int per = n / r;  // butterflies per line (m * s)
+// v[k] <- sum_j v[j] w_R^(j k)
+__host__ __device__ inline void fft_dft2(double2* v) {
+    const double2 a = v[0], b = v[1];
+    v[0] = cadd(a, b);
+    v[1] = csub(a, b);
+}
+__host__ __device__ inline void fft_dft3(double2* v, double sign) {
+    // w3 = -1/2 + sign i sqrt(3)/2
+    const double2 cd = cadd(v[1], v[2]), cm = csub(v[1], v[2]);
+    const double2 base = make_double2(v[0].x - 0.5 * cd.x, v[0].y - 0.5 * cd.y);
+    const double2 rot = cmuli(make_double2(0.86602540378443864676 * cm.x, 0.86602540378443864676 * cm.y), sign);
+    v[0] = cadd(v[0], cd);
+    v[1] = cadd(base, rot);
+    v[2] = csub(base, rot);
+}
+__host__ __device__ inline void fft_dft4(double2* v, double sign) {
+    const double2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]);
+    const double2 c = cadd(v[1], v[3]), d = cmuli(csub(v[1], v[3]), sign);
+    v[0] = cadd(a, c);
+    v[1] = cadd(b, d);
+    v[2] = csub(a, c);
+    v[3] = csub(b, d);
+}
+__host__ __device__ inline void fft_dft8(double2* v, double sign) {
+    const double h = 0.70710678118654752440;
+    double2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+    fft_dft4(e, sign);
+    fft_dft4(o, sign);
+    // w8^k, k = 1..3: h (1 + sign i), sign i, h (-1 + sign i)
+    o[1] = make_double2(h * (o[1].x - sign * o[1].y), h * (o[1].y + sign * o[1].x));
+    o[2] = cmuli(o[2], sign);
+    o[3] = make_double2(-h * (o[3].x + sign * o[3].y), h * (sign * o[3].x - o[3].y));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        v[k] = cadd(e[k], o[k]);
+        v[k + 4] = csub(e[k], o[k]);
+    }
+}
+
+// One radix-R Stockham stage on nl interleaved lines, work items t in
+// [t0, nl * n / R) step dt (t = butterfly * nl + line).
+template <int R>
+__host__ __device__ inline void fft_stage(const double2* x, double2* y, int ld, int nl, int n, int s,
+                                          const double2* tw, int sign, int t0, int dt) {
+    const int per = n / R;  // butterflies per line
+    const bool last = s * R == n;  // p = 0: no twiddles
+    const double sg = (double)sign;
     for (int t = t0; t < nl * per; t += dt) {
-        const int b = t / per, u = t - b * per;
-        const int p = u / s, q = u - p * s;
-        const double2* xb = x + (size_t)b * ld;
-        double2* yb = y + (size_t)b * ld;
-        if (r == 2) {
-            const double2 a = xb[q + s * p], c = xb[q + s * (p + m)];
-            const double2 w = twiddle(p, l, sign);
-            yb[q + s * (2 * p)] = make_double2(a.x + c.x, a.y + c.y);
-            yb[q + s * (2 * p + 1)] = cmul(make_double2(a.x - c.x, a.y - c.y), w);
-        } else {  // r == 3
-            const double2 a = xb[q + s * p], c = xb[q + s * (p + m)], d = xb[q + s * (p + 2 * m)];
-            // w3 = exp(sign 2 pi i / 3) = -1/2 + sign i sqrt(3)/2
-            const double h = 0.86602540378443864676 * sign;
-            const double2 cd = make_double2(c.x + d.x, c.y + d.y);
-            const double2 cm = make_double2(c.x - d.x, c.y - d.y);  // (c - d)
-            const double2 t0v = make_double2(a.x + cd.x, a.y + cd.y);
-            const double2 base = make_double2(a.x - 0.5 * cd.x, a.y - 0.5 * cd.y);
-            // i h (c - d)
-            const double2 rot = make_double2(-h * cm.y, h * cm.x);
-            const double2 t1v = make_double2(base.x + rot.x, base.y + rot.y);
-            const double2 t2v = make_double2(base.x - rot.x, base.y - rot.y);
-            const double2 w1 = twiddle(p, l, sign);
-            const double2 w2 = twiddle(2 * p, l, sign);
-            yb[q + s * (3 * p)] = t0v;
-            yb[q + s * (3 * p + 1)] = cmul(t1v, w1);
-            yb[q + s * (3 * p + 2)] = cmul(t2v, w2);
+        const int u = (int)((unsigned)t / (unsigned)nl), b = t - u * nl;
+        const int p = (int)((unsigned)u / (unsigned)s), q = u - p * s;
+        double2 v[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) v[j] = x[(u + j * per) * ld + b];
+        if (R == 2) fft_dft2(v);
+        if (R == 3) fft_dft3(v, sg);
+        if (R == 4) fft_dft4(v, sg);
+        if (R == 8) fft_dft8(v, sg);
+        double2* out = y + (q + s * R * p) * ld + b;
+        out[0] = v[0];
+#pragma unroll
+        for (int k = 1; k < R; ++k) {
+            if (!last) {
+                double2 w = tw[k * p * s];
+                w.y *= -sg;
+                v[k] = cmul(v[k], w);
+            }
+            out[k * s * ld] = v[k];
         }
     }
 }
 
+__host__ __device__ inline void fft_any_stage(int r, const double2* x, double2* y, int ld, int nl, int n, int s,
+                                              const double2* tw, int sign, int t0, int dt) {
+    if (r == 8) fft_stage<8>(x, y, ld, nl, n, s, tw, sign, t0, dt);
+    else if (r == 4) fft_stage<4>(x, y, ld, nl, n, s, tw, sign, t0, dt);
+    else if (r == 3) fft_stage<3>(x, y, ld, nl, n, s, tw, sign, t0, dt);
+    else fft_stage<2>(x, y, ld, nl, n, s, tw, sign, t0, dt);
+}
+
 #ifdef __CUDACC__
-// nl lines of length n in shared memory (buf0, buf1: nl * ld each), whole
-// CTA; returns the buffer holding the result.
-__device__ __forceinline__ double2* fft_lines_block(double2* buf0, double2* buf1, int ld, int nl, int n, int sign) {
-    int rad[16];
-    const int nr = fft_radices(n, rad);
-    double2 *x = buf0, *y = buf1;
-    int l = n, s = 1;
-    for (int st = 0; st < nr; ++st) {
+// nl interleaved lines of length n in shared memory (x, y: n * ld each; tw the
+// n roots), whole CTA; returns the buffer holding the result.
+__device__ __forceinline__ double2* fft_lines_block(double2* x, double2* y, int ld, int nl, int n, const double2* tw,
+                                                    int sign) {
+    for (int s = 1; s < n;) {
+        const int r = fft_radix(n / s);
         __syncthreads();
-        fft_stage(x, y, ld, nl, n, l, s, rad[st], sign, threadIdx.x, blockDim.x);
-        l /= rad[st];
-        s *= rad[st];
+        fft_any_stage(r, x, y, ld, nl, n, s, tw, sign, threadIdx.x, blockDim.x);
+        s *= r;
         double2* t = x; x = y; y = t;
     }
     __syncthreads();
@@ -112,17 +157,15 @@ __device__ __forceinline__ double2* fft_lines_block(double2* buf0, double2* buf1
 }
 #endif
 
-// Host reference of one line (test build): returns the transform of x in x.
+// Host reference of one line (test build): the transform of x in x.
 inline void fft_line_host(double2* x, int n, int sign) {
-    double2 y[kFftMax];
-    int rad[16];
-    const int nr = fft_radices(n, rad);
+    double2 y[kFftMax], tw[kFftMax];
+    fft_twiddles(n, tw);
     double2 *a = x, *b = y;
-    int l = n, s = 1;
-    for (int st = 0; st < nr; ++st) {
-        fft_stage(a, b, n, 1, n, l, s, rad[st], sign, 0, 1);
-        l /= rad[st];
-        s *= rad[st];
+    for (int s = 1; s < n;) {
+        const int r = fft_radix(n / s);
+        fft_any_stage(r, a, b, 1, 1, n, s, tw, sign, 0, 1);
+        s *= r;
         double2* t = a; a = b; b = t;
     }
     if (a != x)

@@ -9,9 +9,7 @@
 // dirty.  Before a step's pose energies, a dirty mesh's potential is
 // recomputed, phi_mesh = IFFT(G * FFT(Q)) with G(m) = K exp(-pi^2 m^2 /
 // alpha^2) B(m) / (pi V m^2), B the B-spline moduli, by the hand-written FP64
-// transforms of fft.cuh (five passes: rows real-to-complex, axis 1, axis 0
-// with the G product between its forward and inverse transforms, axis 1,
-// rows complex-to-real); after a step that accepted nothing every pass
+// transforms of fft.cuh; after a step that accepted nothing every pass
 // returns at once.  The potential at a point is the same B-spline
 // interpolation of phi_mesh.
 //
@@ -126,109 +124,279 @@ __global__ void k_pme_spread_frag(const RepDev* __restrict__ rep, double* Q) {
     }
 }
 
-// ---- the mesh transforms (dynamic shared memory: 2 * kFftLines * n * 16 B,
-// n the pass's line length) ----
+// ---- the mesh transforms ----
+//
+// Planes (a context whose planes n1 x n2 fit, twice, in shared memory; 128 x 96
+// and 81 x 96 do, 128 x 128 does not): three passes over the mesh,
+//   1. k_pme_fwd_planes: a CTA per plane, rows real-to-complex, then axis 1;
+//   2. k_pme_axis: axis 0 forward, times G, axis 0 inverse;
+//   3. k_pme_inv_planes: a CTA per plane, axis 1 inverse, then rows to real.
+// Otherwise passes 1 and 3 are two each (k_pme_rows_r2c + k_pme_axis along
+// axis 1, and back).  Two real rows share one complex transform (one is the
+// real, the other the imaginary part), which halves the row work for odd and
+// even lengths alike.  All replicas of a launch are one list of items that the
+// CTAs share (a replica whose mesh is current contributes none), so a batch
+// takes as many launches as one replica.
+// Bound: shared-memory passes and barriers per CTA (a 64 x 64 plane: four
+// stages), then L2 traffic; the mesh of one replica stays in L2 between passes.
+// Measured (average launch, about half of them of clean meshes): one 64^3 mesh
+// 8.1 + 7.6 + 9.3 us, against 68 us for six launches with a sincospi per
+// butterfly, radix 2 and 3 and a complex transform per real row; 4 replicas
+// of a 128 x 128 x 96 mesh 75 + 73 + 78 us, against 4 x 228 us.
+constexpr int kPlaneThreads = 512;
+constexpr int kAxisThreads = 256;
+constexpr int kAxisLines = 16;   // columns (256 bytes of each row) per axis item
+constexpr int kRowPairs = 8;     // row pairs per item of the separate row passes
+constexpr int kPmeSmemMax = 220 * 1024;
 
-__device__ __forceinline__ bool pme_clean(const RepDev& R) {
-    return *reinterpret_cast<const volatile int*>(R.pme_dirty) == 0;
+// Complex elements of one of the plane passes' two buffers.
+__host__ __device__ inline size_t pme_plane_elems(int n1, int n2) {
+    const size_t rows = (size_t)n2 * (((n1 + 1) / 2) | 1), cols = (size_t)n1 * ((n2 / 2 + 1) | 1);
+    return rows > cols ? rows : cols;
+}
+__host__ __device__ inline size_t pme_plane_smem(int n1, int n2) {
+    return (2 * pme_plane_elems(n1, n2) + n1 + n2) * sizeof(double2);
+}
+__host__ __device__ inline size_t pme_axis_smem(int n) { return (size_t)(2 * kAxisLines + 1) * n * sizeof(double2); }
+__host__ __device__ inline size_t pme_rows_smem(int n2) {
+    return (size_t)(2 * (kRowPairs | 1) + 1) * n2 * sizeof(double2);
 }
 
-// Rows along axis 2: Q (real, n2 per row) -> spectrum rows (n2 / 2 + 1).
-__global__ void __launch_bounds__(kFftThreads) k_pme_rows_r2c(const RepDev* __restrict__ rep) {
-    const RepDev& R = *rep;
-    if (pme_clean(R)) return;
+__device__ __forceinline__ bool pme_stale(const RepDev& R) {
+    return R.pme && *reinterpret_cast<const volatile int*>(R.pme_dirty) != 0;
+}
+
+// The replica whose items hold `it` (pre[r] <= it < pre[r + 1]).
+__device__ __forceinline__ int prefix_find(const int* pre, int nrep, int it) {
+    int lo = 0, hi = nrep;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (pre[mid] <= it) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// The roots of axis a into shared memory (whole CTA, no barrier).
+__device__ __forceinline__ void load_roots(const RepDev& R, int a, double2* tw) {
+    const int off = a == 0 ? 0 : (a == 1 ? R.pme_n[0] : R.pme_n[0] + R.pme_n[1]);
+    for (int i = threadIdx.x; i < R.pme_n[a]; i += blockDim.x) tw[i] = R.pme_tw[off + i];
+}
+
+// nrow real rows of length n2 from `src`, in pairs: pair j = row 2j + i row 2j + 1
+// (0 past the last row), element i of pair j at b[i * ld + j].
+__device__ __forceinline__ void load_row_pairs(const double* __restrict__ src, int nrow, int n2, double2* b, int ld) {
+    const int np = (nrow + 1) >> 1;
+    for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
+        const int j = (int)((unsigned)e / (unsigned)n2), i = e - j * n2;
+        const double* p = src + (size_t)(2 * j) * n2 + i;
+        b[i * ld + j] = make_double2(p[0], 2 * j + 1 < nrow ? p[n2] : 0.0);
+    }
+}
+
+// Half spectra of the two rows of a transformed pair, Z[k] and Z[n - k]:
+// X_a = (Z[k] + conj Z[n - k]) / 2, X_b = (Z[k] - conj Z[n - k]) / 2i.
+__device__ __forceinline__ void split_pair(double2 z, double2 w, double2& xa, double2& xb) {
+    xa = make_double2(0.5 * (z.x + w.x), 0.5 * (z.y - w.y));
+    xb = make_double2(0.5 * (z.y + w.y), 0.5 * (w.x - z.x));
+}
+// X_a + i X_b at k, from the half spectra (Hermitian extension past n / 2).
+__device__ __forceinline__ double2 join_pair(double2 xa, double2 xb, bool mirrored) {
+    return mirrored ? make_double2(xa.x + xb.y, xb.x - xa.y) : make_double2(xa.x - xb.y, xa.y + xb.x);
+}
+
+__global__ void __launch_bounds__(kPlaneThreads) k_pme_fwd_planes(const RepDev* __restrict__ reps, int nrep) {
     extern __shared__ __align__(16) double2 fbuf[];
-    const int n0 = R.pme_n[0], n1 = R.pme_n[1], n2 = R.pme_n[2], M = n2 / 2 + 1;
-    const int rows = n0 * n1;
-    double2 *b0 = fbuf, *b1 = fbuf + kFftLines * n2;
-    for (int r0 = blockIdx.x * kFftLines; r0 < rows; r0 += gridDim.x * kFftLines) {
-        const int nl = min(kFftLines, rows - r0);
+    __shared__ int pre[257];
+    __shared__ int wtot[32];
+    items_prefix(nrep, pre, wtot, [&](int r) { return pme_stale(reps[r]) ? reps[r].pme_n[0] : 0; });
+    for (int it = blockIdx.x; it < pre[nrep]; it += gridDim.x) {
+        const int r = prefix_find(pre, nrep, it), i0 = it - pre[r];
+        const RepDev& R = reps[r];
+        const int n1 = R.pme_n[1], n2 = R.pme_n[2], M = n2 / 2 + 1, np = (n1 + 1) >> 1;
+        const int ldp = np | 1, ldc = M | 1;
+        const size_t S = pme_plane_elems(n1, n2);
+        double2 *b0 = fbuf, *b1 = fbuf + S, *tw1 = fbuf + 2 * S, *tw2 = tw1 + n1;
         __syncthreads();
-        for (int e = threadIdx.x; e < nl * n2; e += blockDim.x)
-            b0[e] = make_double2(R.pme_q[(size_t)r0 * n2 + e], 0.0);
-        const double2* out = fft_lines_block(b0, b1, n2, nl, n2, -1);
-        for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
-            const int b = e / M, k = e - b * M;
-            R.pme_spec[(size_t)(r0 + b) * M + k] = out[b * n2 + k];
+        load_roots(R, 1, tw1);
+        load_roots(R, 2, tw2);
+        load_row_pairs(R.pme_q + (size_t)i0 * n1 * n2, n1, n2, b0, ldp);
+        double2* z = fft_lines_block(b0, b1, ldp, np, n2, tw2, -1);
+        double2* c = z == b0 ? b1 : b0;
+        for (int e = threadIdx.x; e < np * M; e += blockDim.x) {  // [i1][k2]
+            const int k = (int)((unsigned)e / (unsigned)np), j = e - k * np;
+            double2 xa, xb;
+            split_pair(z[k * ldp + j], z[(k ? n2 - k : 0) * ldp + j], xa, xb);
+            c[2 * j * ldc + k] = xa;
+            if (2 * j + 1 < n1) c[(2 * j + 1) * ldc + k] = xb;
+        }
+        const double2* out = fft_lines_block(c, z, ldc, M, n1, tw1, -1);
+        double2* dst = R.pme_spec + (size_t)i0 * n1 * M;
+        for (int e = threadIdx.x; e < n1 * M; e += blockDim.x) {
+            const int i = (int)((unsigned)e / (unsigned)M), k = e - i * M;
+            dst[e] = out[i * ldc + k];
         }
     }
 }
 
-// Lines along axis `axis` (0 or 1) of the half spectrum, kFftLines consecutive
-// k2 per CTA: sign -1 forward, +1 inverse; fuse_g: forward, times G, inverse.
-__global__ void __launch_bounds__(kFftThreads) k_pme_axis(const RepDev* __restrict__ rep, int axis, int sign,
-                                                          int fuse_g) {
-    const RepDev& R = *rep;
-    if (pme_clean(R)) return;
+// After the last pass over the meshes of a launch: the last CTA to finish marks
+// them current (every CTA has read the marks at its start).
+__device__ __forceinline__ void pme_finish(const RepDev* __restrict__ reps, int nrep) {
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&reps[0].pme_dirty[1], 1) == (int)gridDim.x - 1) {
+        for (int r = 0; r < nrep; ++r)
+            if (reps[r].pme) reps[r].pme_dirty[0] = 0;
+        reps[0].pme_dirty[1] = 0;
+    }
+}
+
+__global__ void __launch_bounds__(kPlaneThreads) k_pme_inv_planes(const RepDev* __restrict__ reps, int nrep) {
     extern __shared__ __align__(16) double2 fbuf[];
-    const int n0 = R.pme_n[0], n1 = R.pme_n[1], M = R.pme_n[2] / 2 + 1;
-    const int n = axis == 0 ? n0 : n1, other = axis == 0 ? n1 : n0;
-    const size_t stride = axis == 0 ? (size_t)n1 * M : (size_t)M;
-    const int kb = (M + kFftLines - 1) / kFftLines;
-    double2 *b0 = fbuf, *b1 = fbuf + kFftLines * n;
-    for (int w = blockIdx.x; w < other * kb; w += gridDim.x) {
-        const int o = w / kb, k0 = (w - o * kb) * kFftLines;
-        const int nl = min(kFftLines, M - k0);
-        const size_t base = (axis == 0 ? (size_t)o * M : (size_t)o * n1 * M) + k0;
+    __shared__ int pre[257];
+    __shared__ int wtot[32];
+    items_prefix(nrep, pre, wtot, [&](int r) { return pme_stale(reps[r]) ? reps[r].pme_n[0] : 0; });
+    for (int it = blockIdx.x; it < pre[nrep]; it += gridDim.x) {
+        const int r = prefix_find(pre, nrep, it), i0 = it - pre[r];
+        const RepDev& R = reps[r];
+        const int n1 = R.pme_n[1], n2 = R.pme_n[2], M = n2 / 2 + 1, np = (n1 + 1) >> 1;
+        const int ldp = np | 1, ldc = M | 1;
+        const size_t S = pme_plane_elems(n1, n2);
+        double2 *b0 = fbuf, *b1 = fbuf + S, *tw1 = fbuf + 2 * S, *tw2 = tw1 + n1;
         __syncthreads();
-        for (int e = threadIdx.x; e < n * kFftLines; e += blockDim.x) {  // consecutive threads: consecutive k2
-            const int i = e / kFftLines, b = e - i * kFftLines;
-            if (b < nl) b0[b * n + i] = R.pme_spec[base + (size_t)i * stride + b];
+        load_roots(R, 1, tw1);
+        load_roots(R, 2, tw2);
+        const double2* src = R.pme_spec + (size_t)i0 * n1 * M;
+        for (int e = threadIdx.x; e < n1 * M; e += blockDim.x) {
+            const int i = (int)((unsigned)e / (unsigned)M), k = e - i * M;
+            b0[i * ldc + k] = src[e];
         }
-        double2* out = fft_lines_block(b0, b1, n, nl, n, fuse_g ? -1 : sign);
+        double2* c = fft_lines_block(b0, b1, ldc, M, n1, tw1, 1);
+        double2* z = c == b0 ? b1 : b0;
+        for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
+            const int k = (int)((unsigned)e / (unsigned)np), j = e - k * np;
+            const bool mir = k >= M;
+            const int kk = mir ? n2 - k : k;
+            const double2 xb = 2 * j + 1 < n1 ? c[(2 * j + 1) * ldc + kk] : make_double2(0.0, 0.0);
+            z[k * ldp + j] = join_pair(c[2 * j * ldc + kk], xb, mir);
+        }
+        const double2* out = fft_lines_block(z, c, ldp, np, n2, tw2, 1);
+        double* phi = const_cast<double*>(R.pme_phi) + (size_t)i0 * n1 * n2;
+        for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
+            const int j = (int)((unsigned)e / (unsigned)n2), i = e - j * n2;
+            const double2 v = out[i * ldp + j];
+            phi[(size_t)(2 * j) * n2 + i] = v.x;
+            if (2 * j + 1 < n1) phi[(size_t)(2 * j + 1) * n2 + i] = v.y;
+        }
+    }
+    pme_finish(reps, nrep);
+}
+
+// Transforms along axis 0 or 1 of the half spectrum: the mesh is `outer`
+// matrices of n rows and C contiguous columns (axis 0: one, n0 x (n1 M); axis
+// 1: n0, n1 x M), an item is kAxisLines columns of one of them.  sign -1
+// forward, +1 inverse; fuse_g: forward, times G, inverse.
+__global__ void __launch_bounds__(kAxisThreads) k_pme_axis(const RepDev* __restrict__ reps, int nrep, int axis,
+                                                           int sign, int fuse_g) {
+    extern __shared__ __align__(16) double2 fbuf[];
+    __shared__ int pre[257];
+    __shared__ int wtot[32];
+    auto columns = [&](const RepDev& R) { return (axis == 0 ? R.pme_n[1] : 1) * (R.pme_n[2] / 2 + 1); };
+    items_prefix(nrep, pre, wtot, [&](int r) {
+        if (!pme_stale(reps[r])) return 0;
+        return (axis == 0 ? 1 : reps[r].pme_n[0]) * ((columns(reps[r]) + kAxisLines - 1) / kAxisLines);
+    });
+    for (int it = blockIdx.x; it < pre[nrep]; it += gridDim.x) {
+        const int r = prefix_find(pre, nrep, it);
+        const RepDev& R = reps[r];
+        const int n = R.pme_n[axis], C = columns(R), cb = (C + kAxisLines - 1) / kAxisLines;
+        const int o = (it - pre[r]) / cb, c0 = (it - pre[r] - o * cb) * kAxisLines;
+        const int nl = min(kAxisLines, C - c0);
+        const size_t base = (size_t)o * n * C + c0;
+        double2 *b0 = fbuf, *b1 = fbuf + kAxisLines * n, *tw = b1 + kAxisLines * n;
+        __syncthreads();
+        load_roots(R, axis, tw);
+        for (int e = threadIdx.x; e < n * kAxisLines; e += blockDim.x) {
+            const int i = e / kAxisLines, b = e % kAxisLines;
+            if (b < nl) b0[e] = R.pme_spec[base + (size_t)i * C + b];
+        }
+        double2* out = fft_lines_block(b0, b1, kAxisLines, nl, n, tw, fuse_g ? -1 : sign);
         if (fuse_g) {
-            for (int e = threadIdx.x; e < n * kFftLines; e += blockDim.x) {
-                const int i = e / kFftLines, b = e - i * kFftLines;
+            for (int e = threadIdx.x; e < n * kAxisLines; e += blockDim.x) {
+                const int i = e / kAxisLines, b = e % kAxisLines;
                 if (b < nl) {
-                    const double g = R.pme_g[base + (size_t)i * stride + b];
-                    double2& v = out[b * n + i];
-                    v.x *= g;
-                    v.y *= g;
+                    const double g = R.pme_g[base + (size_t)i * C + b];
+                    out[e] = make_double2(g * out[e].x, g * out[e].y);
                 }
             }
-            double2* other_buf = out == b0 ? b1 : b0;
-            out = fft_lines_block(out, other_buf, n, nl, n, 1);
+            out = fft_lines_block(out, out == b0 ? b1 : b0, kAxisLines, nl, n, tw, 1);
         }
-        for (int e = threadIdx.x; e < n * kFftLines; e += blockDim.x) {
-            const int i = e / kFftLines, b = e - i * kFftLines;
-            if (b < nl) R.pme_spec[base + (size_t)i * stride + b] = out[b * n + i];
+        for (int e = threadIdx.x; e < n * kAxisLines; e += blockDim.x) {
+            const int i = e / kAxisLines, b = e % kAxisLines;
+            if (b < nl) R.pme_spec[base + (size_t)i * C + b] = out[e];
         }
     }
 }
 
-// Rows along axis 2: half spectrum -> phi (real): the row's full Hermitian
-// extension, inverse transform, real part.
-__global__ void __launch_bounds__(kFftThreads) k_pme_rows_c2r(const RepDev* __restrict__ rep) {
-    const RepDev& R = *rep;
-    if (pme_clean(R)) return;
+// The row passes alone (planes that do not fit in shared memory): an item is
+// kRowPairs pairs of consecutive rows.
+__device__ __forceinline__ int row_items(const RepDev& R) {
+    return (R.pme_n[0] * R.pme_n[1] + 2 * kRowPairs - 1) / (2 * kRowPairs);
+}
+__global__ void __launch_bounds__(kAxisThreads) k_pme_rows_r2c(const RepDev* __restrict__ reps, int nrep) {
     extern __shared__ __align__(16) double2 fbuf[];
-    const int n0 = R.pme_n[0], n1 = R.pme_n[1], n2 = R.pme_n[2], M = n2 / 2 + 1;
-    const int rows = n0 * n1;
-    double2 *b0 = fbuf, *b1 = fbuf + kFftLines * n2;
-    double* phi = const_cast<double*>(R.pme_phi);
-    for (int r0 = blockIdx.x * kFftLines; r0 < rows; r0 += gridDim.x * kFftLines) {
-        const int nl = min(kFftLines, rows - r0);
+    __shared__ int pre[257];
+    __shared__ int wtot[32];
+    items_prefix(nrep, pre, wtot, [&](int r) { return pme_stale(reps[r]) ? row_items(reps[r]) : 0; });
+    for (int it = blockIdx.x; it < pre[nrep]; it += gridDim.x) {
+        const int r = prefix_find(pre, nrep, it);
+        const RepDev& R = reps[r];
+        const int n2 = R.pme_n[2], M = n2 / 2 + 1, ld = kRowPairs | 1;
+        const int r0 = (it - pre[r]) * 2 * kRowPairs, nrow = min(2 * kRowPairs, R.pme_n[0] * R.pme_n[1] - r0);
+        const int np = (nrow + 1) >> 1;
+        double2 *b0 = fbuf, *b1 = fbuf + ld * n2, *tw = b1 + ld * n2;
         __syncthreads();
-        for (int e = threadIdx.x; e < nl * n2; e += blockDim.x) {
-            const int b = e / n2, k = e - b * n2;
-            const double2* row = R.pme_spec + (size_t)(r0 + b) * M;
-            double2 v;
-            if (k < M) {
-                v = row[k];
-            } else {
-                v = row[n2 - k];
-                v.y = -v.y;
-            }
-            b0[e] = v;
+        load_roots(R, 2, tw);
+        load_row_pairs(R.pme_q + (size_t)r0 * n2, nrow, n2, b0, ld);
+        const double2* z = fft_lines_block(b0, b1, ld, np, n2, tw, -1);
+        for (int e = threadIdx.x; e < np * M; e += blockDim.x) {
+            const int j = (int)((unsigned)e / (unsigned)M), k = e - j * M;
+            double2 xa, xb;
+            split_pair(z[k * ld + j], z[(k ? n2 - k : 0) * ld + j], xa, xb);
+            double2* dst = R.pme_spec + (size_t)(r0 + 2 * j) * M + k;
+            dst[0] = xa;
+            if (2 * j + 1 < nrow) dst[M] = xb;
         }
-        const double2* out = fft_lines_block(b0, b1, n2, nl, n2, 1);
-        for (int e = threadIdx.x; e < nl * n2; e += blockDim.x) phi[(size_t)r0 * n2 + e] = out[e].x;
     }
 }
-
-// The mesh potential is current again.
-__global__ void k_pme_done(const RepDev* __restrict__ rep) {
-    if (threadIdx.x == 0) *rep->pme_dirty = 0;
+__global__ void __launch_bounds__(kAxisThreads) k_pme_rows_c2r(const RepDev* __restrict__ reps, int nrep) {
+    extern __shared__ __align__(16) double2 fbuf[];
+    __shared__ int pre[257];
+    __shared__ int wtot[32];
+    items_prefix(nrep, pre, wtot, [&](int r) { return pme_stale(reps[r]) ? row_items(reps[r]) : 0; });
+    for (int it = blockIdx.x; it < pre[nrep]; it += gridDim.x) {
+        const int r = prefix_find(pre, nrep, it);
+        const RepDev& R = reps[r];
+        const int n2 = R.pme_n[2], M = n2 / 2 + 1, ld = kRowPairs | 1;
+        const int r0 = (it - pre[r]) * 2 * kRowPairs, nrow = min(2 * kRowPairs, R.pme_n[0] * R.pme_n[1] - r0);
+        const int np = (nrow + 1) >> 1;
+        double2 *b0 = fbuf, *b1 = fbuf + ld * n2, *tw = b1 + ld * n2;
+        __syncthreads();
+        load_roots(R, 2, tw);
+        for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
+            const int j = (int)((unsigned)e / (unsigned)n2), k = e - j * n2;
+            const bool mir = k >= M;
+            const double2* src = R.pme_spec + (size_t)(r0 + 2 * j) * M + (mir ? n2 - k : k);
+            b0[k * ld + j] = join_pair(src[0], 2 * j + 1 < nrow ? src[M] : make_double2(0.0, 0.0), mir);
+        }
+        const double2* out = fft_lines_block(b0, b1, ld, np, n2, tw, 1);
+        double* phi = const_cast<double*>(R.pme_phi) + (size_t)r0 * n2;
+        for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
+            const int j = (int)((unsigned)e / (unsigned)n2), i = e - j * n2;
+            const double2 v = out[i * ld + j];
+            phi[(size_t)(2 * j) * n2 + i] = v.x;
+            if (2 * j + 1 < nrow) phi[(size_t)(2 * j + 1) * n2 + i] = v.y;
+        }
+    }
+    pme_finish(reps, nrep);
 }
 
 // Spread the change of an accepted move's site: charge q leaves (x0, y0, z0)
