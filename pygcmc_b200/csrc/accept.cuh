@@ -632,25 +632,33 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
     }
 
     if (D.move == MV_DELETE) {
+        bool acc = false;
+        if (tid == 0 && k == 1) {
+            const double lnp = log((double)D.n) - F.B + kBeta * S.E[0];
+            const U4 r = rng(R.seed, R.replica, R.step_base + (uint32_t)D.step, 0u, RP_DELETE, 0);
+            const double u = u53(r.y, r.z);
+            acc = !isnan(lnp) && (lnp >= 0.0 || u < exp(lnp));
+            S.misc[0] = acc ? 1 : 0;
+            if (acc && spec) void_next(R, D.step + 1);
+        }
+        if (Pme && R.pme && k == 1) {  // the leaving molecule's charges leave the mesh, a site per warp
+            __syncthreads();
+            if (S.misc[0]) {
+                const int2 sd = R.gspan[F.startRes + D.del_slot];
+                for (int s = warp; s < ns; s += nwarps) {
+                    const float4 a = R.xyzq[sd.x + s];
+                    if (a.w != 0.0f) pme_spread_warp(R, R.pme_q, a.x, a.y, a.z, -(double)a.w, lane);
+                }
+                if (tid == 0) *R.pme_dirty = 1;
+            }
+            __syncthreads();  // before the slot is overwritten
+        }
         if (tid == 0 && k == 1) {
             const double E = S.E[0];
             const int n = D.n;
-            const double lnp = log((double)n) - F.B + kBeta * E;
-            const U4 r = rng(R.seed, R.replica, R.step_base + (uint32_t)D.step, 0u, RP_DELETE, 0);
-            const double u = u53(r.y, r.z);
-            const bool acc = !isnan(lnp) && (lnp >= 0.0 || u < exp(lnp));
             if (acc) {
-                if (spec) void_next(R, D.step + 1);
                 const int slot = D.del_slot, last = n - 1;
                 const int gs = F.startRes + slot, gl = F.startRes + last;
-                if (Pme && R.pme) {  // the leaving molecule's charges leave the mesh
-                    const int2 sd = R.gspan[gs];
-                    for (int s = 0; s < ns; ++s) {
-                        const float4 a = R.xyzq[sd.x + s];
-                        pme_move_site(R, true, a.x, a.y, a.z, false, 0.f, 0.f, 0.f, a.w);
-                    }
-                    *R.pme_dirty = 1;
-                }
                 cell_remove(R, gs);
                 if (slot != last) {
                     const int2 ss = R.gspan[gs], sl = R.gspan[gl];
@@ -665,7 +673,6 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
                 R.totalNum[D.ftype] = n - 1;
                 *R.energy -= E;
             }
-            S.misc[0] = acc ? 1 : 0;
             S.misc[1] = 1;
             S.misc[2] = acc ? 0 : -1;
             S.misc[3] = acc ? n - 1 : n;
@@ -846,10 +853,16 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
                     const float4 p = R.psite[i * kMaxSites + lane];
                     R.xyzq[sp.x + lane] = p;
                     R.atype[sp.x + lane] = F.stype[lane];
-                    if (Pme && R.pme) pme_move_site(R, false, 0.f, 0.f, 0.f, true, p.x, p.y, p.z, p.w);
                 }
                 if (lane == 0) R.gcen[res] = make_float4(c.x, c.y, c.z, 0.0f);
             }
+            if (Pme && R.pme)  // the new molecules' charges onto the mesh, a site per warp
+                for (int x = warp; x < na * ns; x += nwarps) {
+                    const int a = x / ns;
+                    if (S.acc_slot[a] < 0) continue;
+                    const float4 p = R.psite[S.acc_list[a] * kMaxSites + (x - a * ns)];
+                    if (p.w != 0.0f) pme_spread_warp(R, R.pme_q, p.x, p.y, p.z, (double)p.w, lane);
+                }
             __syncthreads();
             if (warp == 0) {
                 for (int a0 = 0; a0 < na; a0 += 32) {
@@ -866,6 +879,17 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
                 if (lane == 0) R.totalNum[D.ftype] = S.misc[3];
             }
         } else {
+            if (Pme && R.pme) {  // the moved charges: off their old places, onto the new ones, a site per warp
+                for (int x = warp; x < na * ns; x += nwarps) {
+                    const int a = x / ns, s = x - a * ns, i = S.acc_list[a];
+                    const float4 o = R.xyzq[R.gspan[F.startRes + R.pslot[i]].x + s];
+                    if (o.w == 0.0f) continue;
+                    const float4 p = R.psite[i * kMaxSites + s];
+                    pme_spread_warp(R, R.pme_q, o.x, o.y, o.z, -(double)o.w, lane);
+                    pme_spread_warp(R, R.pme_q, p.x, p.y, p.z, (double)o.w, lane);
+                }
+                __syncthreads();  // before the old sites are overwritten
+            }
             for (int a = warp; a < na; a += nwarps) {
                 const int i = S.acc_list[a];
                 const int res = F.startRes + R.pslot[i];
@@ -873,10 +897,6 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
                 if (lane < ns) {  // moved sites as built by the pose-energy kernel; the charge stays
                     const float4 p = R.psite[i * kMaxSites + lane];
                     float* dst = reinterpret_cast<float*>(R.xyzq + sp.x + lane);
-                    if (Pme && R.pme) {
-                        const float4 o = R.xyzq[sp.x + lane];
-                        pme_move_site(R, true, o.x, o.y, o.z, true, p.x, p.y, p.z, o.w);
-                    }
                     dst[0] = p.x;
                     dst[1] = p.y;
                     dst[2] = p.z;

@@ -1051,10 +1051,7 @@ __device__ __forceinline__ void energy_item(const RepDev* __restrict__ reps, int
         // range samples the whole cutoff sphere and the ranges of a pose take equal time)
         energy_cells<Ew>(R, B, R.frag[D.ftype].nsites, cx, cy, cz, self, zi, nwin, lane, acc, ng, npair,
                          mode == 1 ? R.abort : nullptr, D.step, nsl);
-        if (Ew && R.pme && zi == 0) {
-            const float4 a = B.site_abs[lane < kMaxSites ? lane : 0];
-            acc += pme_pose_lane(R, R.frag[D.ftype].nsites, lane, a.x, a.y, a.z, a.w, self);
-        }
+        if (Ew && R.pme && zi == 0) acc += pme_pose_warp(R, R.frag[D.ftype].nsites, lane, B.site_abs, self);
     }
     acc = warp_sum(acc);
     if (lane == 0) {
@@ -1246,10 +1243,7 @@ __global__ void __launch_bounds__(kWarpsE * 32)
         const int nwin = R.span[0] * R.span[1] * R.span[2];
         energy_cells(R, B, ns, centres[3 * p], centres[3 * p + 1], centres[3 * p + 2], self ? self[p] : -1,
                      z * nwin / nslab, (z + 1) * nwin / nslab, lane, acc, ng, npair);
-        if (R.pme && z == 0) {
-            const float4 a = B.site_abs[lane < kMaxSites ? lane : 0];
-            acc += pme_pose_lane(R, ns, lane, a.x, a.y, a.z, a.w, self ? self[p] : -1);
-        }
+        if (R.pme && z == 0) acc += pme_pose_warp(R, ns, lane, B.site_abs, self ? self[p] : -1);
         acc = warp_sum(acc);
         if (lane == 0) {
             out[it] = acc;

@@ -300,9 +300,8 @@ __global__ void __launch_bounds__(kWarpsG * 32, 5) k_energy_fb(const RepDev* __r
             double epme = 0.0;
             float pgx = 0.f, pgy = 0.f, pgz = 0.f;
             if (R.pme && zi == 0) {  // Ewald reciprocal and molecular terms of the pose, once (slab 0)
-                const float4 a = B.site_abs[lane < kMaxSites ? lane : 0];
-                epme = pme_pose_lane(R, ns, lane, a.x, a.y, a.z, a.w, self);
-                pme_grad_lane(R, ns, lane, a.x, a.y, a.z, a.w, self, pgx, pgy, pgz);
+                epme = pme_pose_warp(R, ns, lane, B.site_abs, self);
+                pme_grad_warp(R, ns, lane, B.site_abs, self, pgx, pgy, pgz);
             }
             acc = warp_sum((double)sink.e + epme);
             // per-site gradient (lanes < ns after summing the atom subsets), then

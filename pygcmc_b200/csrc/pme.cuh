@@ -399,13 +399,40 @@ __global__ void __launch_bounds__(kAxisThreads) k_pme_rows_c2r(const RepDev* __r
     pme_finish(reps, nrep);
 }
 
-// Spread the change of an accepted move's site: charge q leaves (x0, y0, z0)
-// and arrives at (x1, y1, z1) (either side skipped when its flag is false).
-__device__ __forceinline__ void pme_move_site(const RepDev& R, bool from, float x0, float y0, float z0, bool to,
-                                              float x1, float y1, float z1, float q) {
-    if (q == 0.0f) return;
-    if (from) pme_spread_one(R, R.pme_q, x0, y0, z0, -(double)q);
-    if (to) pme_spread_one(R, R.pme_q, x1, y1, z1, (double)q);
+// Order-4 B-spline weight j of the fraction w (bspline4's m[j]) and its derivative.
+__device__ __forceinline__ double bspline4_at(double w, int j) {
+    double m[4];
+    bspline4(w, m);
+    return j & 2 ? (j & 1 ? m[3] : m[2]) : (j & 1 ? m[1] : m[0]);
+}
+__device__ __forceinline__ double bspline4_d_at(double w, int j) {
+    double d[4];
+    bspline4_d(w, d);
+    return j & 2 ? (j & 1 ? d[3] : d[2]) : (j & 1 ? d[1] : d[0]);
+}
+
+// Mesh index of the spline's point j at mesh coordinate floor f (any period).
+__device__ __forceinline__ int mesh_index(double f, int j, int n) {
+    int k = (int)f;
+    if ((unsigned)k >= (unsigned)n) k = wrapm(k, n);
+    k -= j;
+    return k < 0 ? wrapm(k, n) : k;
+}
+
+// Charge q at (x, y, z) spread onto Q by a whole warp: lane l adds the points
+// (l / 8, (l / 2) % 4, 2 (l % 2) + {0, 1}).  One site per warp instead of one per
+// lane: a lane's 64 adds in a row took 10 to 20 us of the accept kernel (3-site
+// water, 64^3 mesh; 70 to 120 us in the slab's steps of 30 to 70 accepted moves).
+__device__ __forceinline__ void pme_spread_warp(const RepDev& R, double* Q, float x, float y, float z, double q,
+                                                int lane) {
+    const int a = lane >> 3, b = (lane >> 1) & 3, c = (lane & 1) * 2;
+    const double ux = mesh_u(R, x, 0), uy = mesh_u(R, y, 1), uz = mesh_u(R, z, 2);
+    const double fx = floor(ux), fy = floor(uy), fz = floor(uz);
+    const double wab = q * bspline4_at(ux - fx, a) * bspline4_at(uy - fy, b);
+    const int n1 = R.pme_n[1], n2 = R.pme_n[2];
+    double* row = Q + ((size_t)mesh_index(fx, a, R.pme_n[0]) * n1 + mesh_index(fy, b, n1)) * n2;
+    atomicAdd(row + mesh_index(fz, c, n2), wab * bspline4_at(uz - fz, c));
+    atomicAdd(row + mesh_index(fz, c + 1, n2), wab * bspline4_at(uz - fz, c + 1));
 }
 
 // phi at caller points (diagnostics)
@@ -419,67 +446,102 @@ __device__ __forceinline__ float ewald_g(float r, float alpha) {
     return r < 1e-6f ? 2.0f * alpha * 0.564189584f : erff(alpha * r) / r;
 }
 
-// Reciprocal-space and molecular terms of a pose for lane `lane` (< ns; 0
-// otherwise): q_s phi(r_s) - K q_s sum_t q_t g(|r_s - x_t|) (the latter when
-// the pose replaces group `self`).  Sites at absolute positions (sx, sy, sz).
-__device__ __forceinline__ double pme_pose_lane(const RepDev& R, int ns, int lane, float sx, float sy, float sz,
-                                                float q, int self) {
-    if (lane >= ns) return 0.0;
-    double e = (double)q * pme_phi_at(R, sx, sy, sz);
-    if (self >= 0) {
+// Lanes that share one site's 16 mesh rows (of 4 points) when ns sites are
+// interpolated by a warp: the largest power of two with ns lanes' groups in 32.
+__device__ __forceinline__ int mesh_lanes(int ns) {
+    return ns <= 2 ? 16 : (ns <= 4 ? 8 : (ns <= 8 ? 4 : (ns <= 16 ? 2 : 1)));
+}
+
+// Reciprocal-space and molecular terms of a pose, whole warp; the sum over the
+// lanes of the results is
+//   sum_s q_s phi(r_s) - K q_s sum_t q_t g(|r_s - x_t|)
+// (the latter when the pose replaces group `self`).  Site s at sites[s]
+// (absolute position, charge) in shared memory.  phi is interpolated by
+// mesh_lanes lanes per site, each taking its share of the 16 mesh rows: with one
+// lane per site a 3-site pose kept 3 lanes busy with 64 loads each.
+__device__ __forceinline__ double pme_pose_warp(const RepDev& R, int ns, int lane, const float4* sites, int self) {
+    const int P = mesh_lanes(ns), s = lane / P, sub = lane - s * P;
+    double e = 0.0;
+    if (s < ns) {
+        const float4 p = sites[s];
+        const double ux = mesh_u(R, p.x, 0), uy = mesh_u(R, p.y, 1), uz = mesh_u(R, p.z, 2);
+        const double fx = floor(ux), fy = floor(uy), fz = floor(uz);
+        double mz[4];
+        bspline4(uz - fz, mz);
+        const int n1 = R.pme_n[1], n2 = R.pme_n[2];
+        const int z0 = mesh_index(fz, 0, n2), z1 = mesh_index(fz, 1, n2), z2 = mesh_index(fz, 2, n2),
+                  z3 = mesh_index(fz, 3, n2);
+        for (int r = sub; r < 16; r += P) {
+            const int a = r >> 2, b = r & 3;
+            const double* row = R.pme_phi + ((size_t)mesh_index(fx, a, R.pme_n[0]) * n1 + mesh_index(fy, b, n1)) * n2;
+            const double t = mz[0] * row[z0] + mz[1] * row[z1] + mz[2] * row[z2] + mz[3] * row[z3];
+            e += bspline4_at(ux - fx, a) * bspline4_at(uy - fy, b) * t;
+        }
+        e *= (double)p.w;
+    }
+    if (self >= 0 && lane < ns) {
+        const float4 p = sites[lane];
         const int2 sp = R.gspan[self];
         float m = 0.0f;
         for (int t = 0; t < sp.y; ++t) {
             const float4 a = R.xyzq[sp.x + t];
-            float dx = sx - a.x, dy = sy - a.y, dz = sz - a.z;
+            float dx = p.x - a.x, dy = p.y - a.y, dz = p.z - a.z;
             dx -= rintf(dx * R.invL[0]) * R.L[0];
             dy -= rintf(dy * R.invL[1]) * R.L[1];
             dz -= rintf(dz * R.invL[2]) * R.L[2];
             m += a.w * ewald_g(sqrtf(dx * dx + dy * dy + dz * dz), R.pme_alpha);
         }
-        e -= (double)kCoulomb * (double)q * (double)m;
+        e -= (double)kCoulomb * (double)p.w * (double)m;
     }
     return e;
 }
 
-// Gradient of pme_pose_lane's terms with respect to lane `lane`'s site
-// position (< ns; zero otherwise): q grad phi(r_s) from the derivative of the
-// B-spline interpolation (d/dx = (n / L) d/du), minus K q sum_t q_t g'(d) d/|d|
-// over the replaced group's atoms (d = r_s - x_t, minimum image).
-__device__ __forceinline__ void pme_grad_lane(const RepDev& R, int ns, int lane, float sx, float sy, float sz,
-                                              float q, int self, float& gx, float& gy, float& gz) {
-    gx = gy = gz = 0.0f;
-    if (lane >= ns || q == 0.0f) return;
-    double mx[4], my[4], mz[4], dx[4], dy[4], dz[4];
-    const double ux = mesh_u(R, sx, 0), uy = mesh_u(R, sy, 1), uz = mesh_u(R, sz, 2);
-    const double fx = floor(ux), fy = floor(uy), fz = floor(uz);
-    bspline4(ux - fx, mx);
-    bspline4(uy - fy, my);
-    bspline4(uz - fz, mz);
-    bspline4_d(ux - fx, dx);
-    bspline4_d(uy - fy, dy);
-    bspline4_d(uz - fz, dz);
-    const int n0 = R.pme_n[0], n1 = R.pme_n[1], n2 = R.pme_n[2];
+// Gradient of pme_pose_warp's terms with respect to lane `lane`'s site position
+// (lanes < ns; zero otherwise), whole warp: q grad phi(r_s) from the derivative of
+// the B-spline interpolation (d/dx = (n / L) d/du), the mesh rows shared out as
+// there, minus K q sum_t q_t g'(d) d/|d| over the replaced group's atoms
+// (d = r_s - x_t, minimum image).
+__device__ __forceinline__ void pme_grad_warp(const RepDev& R, int ns, int lane, const float4* sites, int self,
+                                              float& gx, float& gy, float& gz) {
+    const int P = mesh_lanes(ns), ms = lane / P, sub = lane - ms * P;
     double px = 0.0, py = 0.0, pz = 0.0;
-    for (int a = 0; a < 4; ++a) {
-        const int i0 = wrapm((int)fx - a, n0);
-        for (int b = 0; b < 4; ++b) {
-            const int i1 = wrapm((int)fy - b, n1);
-            const double* row = R.pme_phi + ((size_t)i0 * n1 + i1) * n2;
-            double t = 0.0, tz = 0.0;
-            for (int c = 0; c < 4; ++c) {
-                const double v = row[wrapm((int)fz - c, n2)];
-                t += mz[c] * v;
-                tz += dz[c] * v;
-            }
-            px += dx[a] * my[b] * t;
-            py += mx[a] * dy[b] * t;
-            pz += mx[a] * my[b] * tz;
+    if (ms < ns) {
+        const float4 p = sites[ms];
+        const double ux = mesh_u(R, p.x, 0), uy = mesh_u(R, p.y, 1), uz = mesh_u(R, p.z, 2);
+        const double fx = floor(ux), fy = floor(uy), fz = floor(uz);
+        double mz[4], dz[4];
+        bspline4(uz - fz, mz);
+        bspline4_d(uz - fz, dz);
+        const int n1 = R.pme_n[1], n2 = R.pme_n[2];
+        const int z0 = mesh_index(fz, 0, n2), z1 = mesh_index(fz, 1, n2), z2 = mesh_index(fz, 2, n2),
+                  z3 = mesh_index(fz, 3, n2);
+        for (int r = sub; r < 16; r += P) {
+            const int a = r >> 2, b = r & 3;
+            const double* row = R.pme_phi + ((size_t)mesh_index(fx, a, R.pme_n[0]) * n1 + mesh_index(fy, b, n1)) * n2;
+            const double v0 = row[z0], v1 = row[z1], v2 = row[z2], v3 = row[z3];
+            const double t = mz[0] * v0 + mz[1] * v1 + mz[2] * v2 + mz[3] * v3;
+            const double tz = dz[0] * v0 + dz[1] * v1 + dz[2] * v2 + dz[3] * v3;
+            const double wx = bspline4_at(ux - fx, a), wy = bspline4_at(uy - fy, b);
+            px += bspline4_d_at(ux - fx, a) * wy * t;
+            py += wx * bspline4_d_at(uy - fy, b) * t;
+            pz += wx * wy * tz;
         }
     }
-    double g0 = (double)q * px * n0 / (double)R.L[0];
-    double g1 = (double)q * py * n1 / (double)R.L[1];
-    double g2 = (double)q * pz * n2 / (double)R.L[2];
+    for (int off = P >> 1; off > 0; off >>= 1) {
+        px += __shfl_xor_sync(kFull, px, off);
+        py += __shfl_xor_sync(kFull, py, off);
+        pz += __shfl_xor_sync(kFull, pz, off);
+    }
+    const int from = min(lane * P, 31);  // lane s: the sum of the lanes of site s
+    px = __shfl_sync(kFull, px, from);
+    py = __shfl_sync(kFull, py, from);
+    pz = __shfl_sync(kFull, pz, from);
+    gx = gy = gz = 0.0f;
+    if (lane >= ns || sites[lane].w == 0.0f) return;
+    const float sx = sites[lane].x, sy = sites[lane].y, sz = sites[lane].z, q = sites[lane].w;
+    double g0 = (double)q * px * R.pme_n[0] / (double)R.L[0];
+    double g1 = (double)q * py * R.pme_n[1] / (double)R.L[1];
+    double g2 = (double)q * pz * R.pme_n[2] / (double)R.L[2];
     if (self >= 0) {  // d/dr_s of -K q sum_t q_t g(|r_s - x_t|), g(r) = erf(alpha r) / r
         const int2 sp = R.gspan[self];
         const double al = (double)R.pme_alpha, c = 1.1283791670955126 * al;  // 2 alpha / sqrt(pi)
