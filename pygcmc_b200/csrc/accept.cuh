@@ -603,20 +603,38 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
         }
         e += bg;
         S.ephys[i] = e;
-        if (D.fb) {  // Metropolis-Hastings: exp(-beta dE) q(new -> old) / q(old -> new)
-            float fo[6], fn[6];
-            fb_force(R, D, i, 1, fo, false);
-            fb_force(R, D, i, 0, fn, false);
-            const float4 d = R.fbprop[2 * i], ao = R.fbprop[2 * i + 1];
-            double eff = INFINITY;
-            if (d.w == 0.0f && isfinite(e)) eff = __dsub_rn(e, __ddiv_rn(fb_ln_ratio(R, D, d, ao, fn), kBeta));
-            S.E[i] = eff;
-            if (logging && R.logF && i < R.log_kmax) {
-                float* o = R.logF + ((size_t)D.step * R.log_kmax + i) * 12;
-                for (int c = 0; c < 6; ++c) { o[c] = fo[c]; o[6 + c] = fn[c]; }
+        S.E[i] = e;
+    }
+    if (D.fb) {
+        // Metropolis-Hastings, exp(-beta dE) q(new -> old) / q(old -> new): a half-warp per
+        // pose, lanes 0..5 sum the old pose's force and torque components over the slabs,
+        // 6..11 the new pose's, lanes 0..2 form the components of the ratio.  (One thread
+        // per pose left 60 threads with 12 sums of 15 terms each: 22 us of a 65-pose step,
+        // 7 us now.)
+        __syncthreads();  // ephys of the half-warp's pose
+        const int sub = lane & 15;
+        const bool trn = D.move == MV_TRANSLATE;
+        for (int base = 2 * warp; base < k; base += 2 * nwarps) {
+            const int i = base + (lane >> 4);
+            const bool on = i < k;
+            float f = 0.0f;
+            if (on && sub < 12) f = fb_force_at(R, D, i, sub < 6 ? 1 : 0, sub < 6 ? sub : sub - 6, false);
+            const float fn = __shfl_sync(kFull, f, (lane & 16) + 6 + (trn ? 0 : 3) + min(sub, 2));
+            double t = 0.0;
+            bool valid = false;
+            if (on) {
+                const float4 d = R.fbprop[2 * i], ao = R.fbprop[2 * i + 1];
+                valid = d.w == 0.0f;
+                t = fb_ln_term(R, D, sub == 0 ? d.x : (sub == 1 ? d.y : d.z),
+                               sub == 0 ? ao.x : (sub == 1 ? ao.y : ao.z), fn);
             }
-        } else {
-            S.E[i] = e;
+            const double t1 = __shfl_sync(kFull, t, (lane & 16) + 1), t2 = __shfl_sync(kFull, t, (lane & 16) + 2);
+            if (on && sub == 0) {
+                const double e = S.ephys[i], s = __dadd_rn(__dadd_rn(__dadd_rn(0.0, t), t1), t2);
+                S.E[i] = (valid && isfinite(e)) ? __dsub_rn(e, __ddiv_rn(s, kBeta)) : INFINITY;
+            }
+            if (on && sub < 12 && logging && R.logF && i < R.log_kmax)
+                R.logF[((size_t)D.step * R.log_kmax + i) * 12 + sub] = f;
         }
     }
     if (tid == 0) { S.misc[0] = 0; S.misc[1] = 0; S.misc[2] = -1; S.misc[3] = D.n; }

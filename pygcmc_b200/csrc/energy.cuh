@@ -677,21 +677,18 @@ __device__ __forceinline__ void moved_site(const RepDev& R, const StepDesc& D, i
 // old pose (fb_tilted).  A translate moves the sites by d wrapped so the new
 // centre lies in the box.  The reverse move is -d from the new pose with its
 // own force, and the ratio of the two proposal densities enters the
-// acceptance (fb_ln_ratio).  All float steps are explicit round-to-nearest
+// acceptance (fb_ln_term).  All float steps are explicit round-to-nearest
 // operations so the host oracle reproduces them bit for bit.
 
-// Force and torque partials of pose i, variant v, summed over the slabs in
-// order (FP64) and rounded to float.  cg: read through L2 only (partials
-// written by other CTAs of the running launch).
-__device__ __forceinline__ void fb_force(const RepDev& R, const StepDesc& D, int i, int v, float f[6], bool cg) {
-    for (int c = 0; c < 6; ++c) {
-        double a = 0.0;
-        for (int z = 0; z < D.nslab; ++z) {
-            const float* p = R.fpart + ((size_t)(i * 2 + v) * D.nslab + z) * 6 + c;
-            a += (double)(cg ? __ldcg(p) : *p);
-        }
-        f[c] = (float)a;
-    }
+// Component c of the force (0..2) and torque (3..5) of pose i, variant v: the
+// slabs' partials summed in order (FP64) and rounded to float.  cg: read through
+// L2 only (partials written by other CTAs of the running launch).
+__device__ __forceinline__ float fb_force_at(const RepDev& R, const StepDesc& D, int i, int v, int c, bool cg) {
+    const float* p = R.fpart + (size_t)(i * 2 + v) * D.nslab * 6 + c;
+    double a = 0.0;
+#pragma unroll 4
+    for (int z = 0; z < D.nslab; ++z) a += (double)(cg ? __ldcg(p + 6 * z) : p[6 * z]);
+    return (float)a;
 }
 
 // Shift of the centre coordinate c by d, wrapped into [start, start + L).
@@ -755,24 +752,16 @@ __device__ __forceinline__ void fb_moved_site(const RepDev& R, const StepDesc& D
     pz = fadd(z, mz);
 }
 
-// ln q(new -> old) - ln q(old -> new) for pose i: per component
-// g(a') - g(a) - (a' + a) d with g = fb_lnorm, a (stored) the old tilt and
-// a' = lambda beta f' from the new pose's force/torque fn; the rotation-vector
-// Jacobian is even in v and cancels.  Float terms, FP64 sum.
-__device__ __forceinline__ double fb_ln_ratio(const RepDev& R, const StepDesc& D, const float4& d, const float4& a,
-                                              const float fn[6]) {
+// Component c of ln q(new -> old) - ln q(old -> new) of a pose, whose terms are
+// summed in order: g(a') - g(a) - (a' + a) d with g = fb_lnorm, a (stored) the old
+// tilt and a' = lambda beta f' from the component f' of the new pose's force /
+// torque; the rotation-vector Jacobian is even in v and cancels.  Float terms, FP64 sum.
+__device__ __forceinline__ double fb_ln_term(const RepDev& R, const StepDesc& D, float d, float a, float fn) {
     const bool trn = D.move == MV_TRANSLATE;
-    const float* g = trn ? fn : fn + 3;
     const float lb = trn ? R.fb_at : R.fb_ar, h = trn ? R.fb_ht : R.fb_hr;
-    const float dd[3] = {d.x, d.y, d.z}, ao[3] = {a.x, a.y, a.z};
-    double s = 0.0;
-    for (int c = 0; c < 3; ++c) {
-        const float an = fmul(lb, g[c]);
-        const double t = __dsub_rn(__dsub_rn((double)fb_lnorm(an, h), (double)fb_lnorm(ao[c], h)),
-                                   __dmul_rn(__dadd_rn((double)an, (double)ao[c]), (double)dd[c]));
-        s = __dadd_rn(s, t);
-    }
-    return s;
+    const float an = fmul(lb, fn);
+    return __dsub_rn(__dsub_rn((double)fb_lnorm(an, h), (double)fb_lnorm(a, h)),
+                     __dmul_rn(__dadd_rn((double)an, (double)a), (double)d));
 }
 
 // Load the pose of item (i, variant v) of step D into B.site; returns the

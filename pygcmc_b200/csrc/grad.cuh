@@ -346,12 +346,16 @@ __global__ void __launch_bounds__(kWarpsG * 32, 5) k_energy_fb(const RepDev* __r
                 if (last) R.fbcnt[i] = 0;
             }
             last = __shfl_sync(kFull, last, 0);
-            if (last && lane == 0) {
+            if (last) {  // a lane per component sums, then lane 0 draws
                 __threadfence();
+                const float fc = lane < 6 ? fb_force_at(R, D, i, 1, lane, true) : 0.0f;
                 float fo[6];
-                fb_force(R, D, i, 1, fo, true);
-                const float4 gc = R.gcen[R.frag[D.ftype].startRes + R.pslot[i]];
-                R.pcen[i] = fb_propose(R, D, i, fo, gc, R.fbprop + 2 * i);
+#pragma unroll
+                for (int c = 0; c < 6; ++c) fo[c] = __shfl_sync(kFull, fc, c);
+                if (lane == 0) {
+                    const float4 gc = R.gcen[R.frag[D.ftype].startRes + R.pslot[i]];
+                    R.pcen[i] = fb_propose(R, D, i, fo, gc, R.fbprop + 2 * i);
+                }
             }
         } else if (v == 0 && D.nw > 0) {  // this item's share of the neighbour bit matrix
             nbr_share(R, D, i, zi, D.nslab, i * D.nslab + zi, lane, sym);
