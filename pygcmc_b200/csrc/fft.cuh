@@ -61,6 +61,22 @@ inline void fft_twiddles(int n, double2* tw) {
     }
 }
 
+// Division by d of 0 <= t < 2^32 / d with one multiplication (m = ceil(2^32 / d),
+// d > 1): the index arithmetic of a butterfly costs as much as its sums with the
+// compiler's general division.
+struct FastDiv {
+    unsigned m, d;
+    __host__ __device__ explicit FastDiv(int d_) : m(0xffffffffu / (unsigned)d_ + 1u), d((unsigned)d_) {}
+    __host__ __device__ int quot(int t) const {
+        if (d == 1u) return t;
+#ifdef __CUDA_ARCH__
+        return (int)__umulhi((unsigned)t, m);
+#else
+        return (int)(((unsigned long long)(unsigned)t * m) >> 32);
+#endif
+    }
+};
+
 // v[k] <- sum_j v[j] w_R^(j k)
 __host__ __device__ inline void fft_dft2(double2* v) {
     const double2 a = v[0], b = v[1];
@@ -108,9 +124,10 @@ __host__ __device__ inline void fft_stage(const double2* x, double2* y, int ld, 
     const int per = n / R;  // butterflies per line
     const bool last = s * R == n;  // p = 0: no twiddles
     const double sg = (double)sign;
+    const FastDiv by_nl(nl), by_s(s);
     for (int t = t0; t < nl * per; t += dt) {
-        const int u = (int)((unsigned)t / (unsigned)nl), b = t - u * nl;
-        const int p = (int)((unsigned)u / (unsigned)s), q = u - p * s;
+        const int u = by_nl.quot(t), b = t - u * nl;
+        const int p = by_s.quot(u), q = u - p * s;
         double2 v[R];
 #pragma unroll
         for (int j = 0; j < R; ++j) v[j] = x[(u + j * per) * ld + b];

@@ -32,11 +32,11 @@ namespace gcmc {
 
 // order-4 B-spline weights of the four mesh points floor(u) - j, j = 0..3
 __device__ __forceinline__ void bspline4(double w, double m[4]) {
-    const double w2 = w * w, w3 = w2 * w, c = 1.0 - w;
-    m[0] = w3 / 6.0;
-    m[1] = (-3.0 * w3 + 3.0 * w2 + 3.0 * w + 1.0) / 6.0;
-    m[2] = (3.0 * w3 - 6.0 * w2 + 4.0) / 6.0;
-    m[3] = c * c * c / 6.0;
+    const double w2 = w * w, w3 = w2 * w, c = 1.0 - w, sixth = 1.0 / 6.0;
+    m[0] = w3 * sixth;
+    m[1] = (-3.0 * w3 + 3.0 * w2 + 3.0 * w + 1.0) * sixth;
+    m[2] = (3.0 * w3 - 6.0 * w2 + 4.0) * sixth;
+    m[3] = c * c * c * sixth;
 }
 
 __device__ __forceinline__ int wrapm(int k, int n) {
@@ -186,8 +186,10 @@ __device__ __forceinline__ void load_roots(const RepDev& R, int a, double2* tw) 
 // (0 past the last row), element i of pair j at b[i * ld + j].
 __device__ __forceinline__ void load_row_pairs(const double* __restrict__ src, int nrow, int n2, double2* b, int ld) {
     const int np = (nrow + 1) >> 1;
+    const FastDiv by_n2(n2);
+#pragma unroll 4
     for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
-        const int j = (int)((unsigned)e / (unsigned)n2), i = e - j * n2;
+        const int j = by_n2.quot(e), i = e - j * n2;
         const double* p = src + (size_t)(2 * j) * n2 + i;
         b[i * ld + j] = make_double2(p[0], 2 * j + 1 < nrow ? p[n2] : 0.0);
     }
@@ -222,8 +224,9 @@ __global__ void __launch_bounds__(kPlaneThreads) k_pme_fwd_planes(const RepDev* 
         load_row_pairs(R.pme_q + (size_t)i0 * n1 * n2, n1, n2, b0, ldp);
         double2* z = fft_lines_block(b0, b1, ldp, np, n2, tw2, -1);
         double2* c = z == b0 ? b1 : b0;
+        const FastDiv by_np(np), by_M(M);
         for (int e = threadIdx.x; e < np * M; e += blockDim.x) {  // [i1][k2]
-            const int k = (int)((unsigned)e / (unsigned)np), j = e - k * np;
+            const int k = by_np.quot(e), j = e - k * np;
             double2 xa, xb;
             split_pair(z[k * ldp + j], z[(k ? n2 - k : 0) * ldp + j], xa, xb);
             c[2 * j * ldc + k] = xa;
@@ -231,8 +234,9 @@ __global__ void __launch_bounds__(kPlaneThreads) k_pme_fwd_planes(const RepDev* 
         }
         const double2* out = fft_lines_block(c, z, ldc, M, n1, tw1, -1);
         double2* dst = R.pme_spec + (size_t)i0 * n1 * M;
+#pragma unroll 4
         for (int e = threadIdx.x; e < n1 * M; e += blockDim.x) {
-            const int i = (int)((unsigned)e / (unsigned)M), k = e - i * M;
+            const int i = by_M.quot(e), k = e - i * M;
             dst[e] = out[i * ldc + k];
         }
     }
@@ -265,14 +269,16 @@ __global__ void __launch_bounds__(kPlaneThreads) k_pme_inv_planes(const RepDev* 
         load_roots(R, 1, tw1);
         load_roots(R, 2, tw2);
         const double2* src = R.pme_spec + (size_t)i0 * n1 * M;
+        const FastDiv by_np(np), by_M(M), by_n2(n2);
+#pragma unroll 4
         for (int e = threadIdx.x; e < n1 * M; e += blockDim.x) {
-            const int i = (int)((unsigned)e / (unsigned)M), k = e - i * M;
+            const int i = by_M.quot(e), k = e - i * M;
             b0[i * ldc + k] = src[e];
         }
         double2* c = fft_lines_block(b0, b1, ldc, M, n1, tw1, 1);
         double2* z = c == b0 ? b1 : b0;
         for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
-            const int k = (int)((unsigned)e / (unsigned)np), j = e - k * np;
+            const int k = by_np.quot(e), j = e - k * np;
             const bool mir = k >= M;
             const int kk = mir ? n2 - k : k;
             const double2 xb = 2 * j + 1 < n1 ? c[(2 * j + 1) * ldc + kk] : make_double2(0.0, 0.0);
@@ -280,8 +286,9 @@ __global__ void __launch_bounds__(kPlaneThreads) k_pme_inv_planes(const RepDev* 
         }
         const double2* out = fft_lines_block(z, c, ldp, np, n2, tw2, 1);
         double* phi = const_cast<double*>(R.pme_phi) + (size_t)i0 * n1 * n2;
+#pragma unroll 4
         for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
-            const int j = (int)((unsigned)e / (unsigned)n2), i = e - j * n2;
+            const int j = by_n2.quot(e), i = e - j * n2;
             const double2 v = out[i * ldp + j];
             phi[(size_t)(2 * j) * n2 + i] = v.x;
             if (2 * j + 1 < n1) phi[(size_t)(2 * j + 1) * n2 + i] = v.y;
@@ -314,6 +321,7 @@ __global__ void __launch_bounds__(kAxisThreads) k_pme_axis(const RepDev* __restr
         double2 *b0 = fbuf, *b1 = fbuf + kAxisLines * n, *tw = b1 + kAxisLines * n;
         __syncthreads();
         load_roots(R, axis, tw);
+#pragma unroll 4
         for (int e = threadIdx.x; e < n * kAxisLines; e += blockDim.x) {
             const int i = e / kAxisLines, b = e % kAxisLines;
             if (b < nl) b0[e] = R.pme_spec[base + (size_t)i * C + b];
@@ -357,8 +365,9 @@ __global__ void __launch_bounds__(kAxisThreads) k_pme_rows_r2c(const RepDev* __r
         load_roots(R, 2, tw);
         load_row_pairs(R.pme_q + (size_t)r0 * n2, nrow, n2, b0, ld);
         const double2* z = fft_lines_block(b0, b1, ld, np, n2, tw, -1);
+        const FastDiv by_M(M);
         for (int e = threadIdx.x; e < np * M; e += blockDim.x) {
-            const int j = (int)((unsigned)e / (unsigned)M), k = e - j * M;
+            const int j = by_M.quot(e), k = e - j * M;
             double2 xa, xb;
             split_pair(z[k * ld + j], z[(k ? n2 - k : 0) * ld + j], xa, xb);
             double2* dst = R.pme_spec + (size_t)(r0 + 2 * j) * M + k;
@@ -381,8 +390,9 @@ __global__ void __launch_bounds__(kAxisThreads) k_pme_rows_c2r(const RepDev* __r
         double2 *b0 = fbuf, *b1 = fbuf + ld * n2, *tw = b1 + ld * n2;
         __syncthreads();
         load_roots(R, 2, tw);
+        const FastDiv by_n2(n2);
         for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
-            const int j = (int)((unsigned)e / (unsigned)n2), k = e - j * n2;
+            const int j = by_n2.quot(e), k = e - j * n2;
             const bool mir = k >= M;
             const double2* src = R.pme_spec + (size_t)(r0 + 2 * j) * M + (mir ? n2 - k : k);
             b0[k * ld + j] = join_pair(src[0], 2 * j + 1 < nrow ? src[M] : make_double2(0.0, 0.0), mir);
@@ -390,7 +400,7 @@ __global__ void __launch_bounds__(kAxisThreads) k_pme_rows_c2r(const RepDev* __r
         const double2* out = fft_lines_block(b0, b1, ld, np, n2, tw, 1);
         double* phi = const_cast<double*>(R.pme_phi) + (size_t)r0 * n2;
         for (int e = threadIdx.x; e < np * n2; e += blockDim.x) {
-            const int j = (int)((unsigned)e / (unsigned)n2), i = e - j * n2;
+            const int j = by_n2.quot(e), i = e - j * n2;
             const double2 v = out[i * ld + j];
             phi[(size_t)(2 * j) * n2 + i] = v.x;
             if (2 * j + 1 < nrow) phi[(size_t)(2 * j + 1) * n2 + i] = v.y;
@@ -399,16 +409,8 @@ __global__ void __launch_bounds__(kAxisThreads) k_pme_rows_c2r(const RepDev* __r
     pme_finish(reps, nrep);
 }
 
-// Order-4 B-spline weight j of the fraction w (bspline4's m[j]) and its derivative.
-__device__ __forceinline__ double bspline4_at(double w, int j) {
-    double m[4];
-    bspline4(w, m);
+__device__ __forceinline__ double sel4(const double m[4], int j) {
     return j & 2 ? (j & 1 ? m[3] : m[2]) : (j & 1 ? m[1] : m[0]);
-}
-__device__ __forceinline__ double bspline4_d_at(double w, int j) {
-    double d[4];
-    bspline4_d(w, d);
-    return j & 2 ? (j & 1 ? d[3] : d[2]) : (j & 1 ? d[1] : d[0]);
 }
 
 // Mesh index of the spline's point j at mesh coordinate floor f (any period).
@@ -420,19 +422,28 @@ __device__ __forceinline__ int mesh_index(double f, int j, int n) {
 }
 
 // Charge q at (x, y, z) spread onto Q by a whole warp: lane l adds the points
-// (l / 8, (l / 2) % 4, 2 (l % 2) + {0, 1}).  One site per warp instead of one per
-// lane: a lane's 64 adds in a row took 10 to 20 us of the accept kernel (3-site
-// water, 64^3 mesh; 70 to 120 us in the slab's steps of 30 to 70 accepted moves).
+// (l / 8, (l / 2) % 4, 2 (l % 2) + {0, 1}); lane 4 a + j forms axis a's weight and
+// index j, which the others fetch (with every lane forming all twelve weights the
+// single SM's FP64 rate bounded it, 3.8 us a site).  One site per warp instead of
+// one per lane: a lane's 64 adds in a row took 10 to 20 us of the accept kernel
+// (3-site water, 64^3 mesh; 70 to 120 us in the slab's steps of 30 to 70 accepted
+// moves).
 __device__ __forceinline__ void pme_spread_warp(const RepDev& R, double* Q, float x, float y, float z, double q,
                                                 int lane) {
-    const int a = lane >> 3, b = (lane >> 1) & 3, c = (lane & 1) * 2;
-    const double ux = mesh_u(R, x, 0), uy = mesh_u(R, y, 1), uz = mesh_u(R, z, 2);
-    const double fx = floor(ux), fy = floor(uy), fz = floor(uz);
-    const double wab = q * bspline4_at(ux - fx, a) * bspline4_at(uy - fy, b);
-    const int n1 = R.pme_n[1], n2 = R.pme_n[2];
-    double* row = Q + ((size_t)mesh_index(fx, a, R.pme_n[0]) * n1 + mesh_index(fy, b, n1)) * n2;
-    atomicAdd(row + mesh_index(fz, c, n2), wab * bspline4_at(uz - fz, c));
-    atomicAdd(row + mesh_index(fz, c + 1, n2), wab * bspline4_at(uz - fz, c + 1));
+    const int ax = (lane >> 2) % 3;
+    const double u = mesh_u(R, ax == 0 ? x : (ax == 1 ? y : z), ax), f = floor(u);
+    double m[4];
+    bspline4(u - f, m);
+    const double w = sel4(m, lane & 3);
+    const int k = mesh_index(f, lane & 3, R.pme_n[ax]);
+    const int a = lane >> 3, b = 4 + ((lane >> 1) & 3), c = 8 + (lane & 1) * 2;
+    const double wab = q * __shfl_sync(kFull, w, a) * __shfl_sync(kFull, w, b);
+    const double w0 = __shfl_sync(kFull, w, c), w1 = __shfl_sync(kFull, w, c + 1);
+    const int ka = __shfl_sync(kFull, k, a), kb = __shfl_sync(kFull, k, b);
+    const int k0 = __shfl_sync(kFull, k, c), k1 = __shfl_sync(kFull, k, c + 1);
+    double* row = Q + ((size_t)ka * R.pme_n[1] + kb) * R.pme_n[2];
+    atomicAdd(row + k0, wab * w0);
+    atomicAdd(row + k1, wab * w1);
 }
 
 // phi at caller points (diagnostics)
@@ -466,7 +477,9 @@ __device__ __forceinline__ double pme_pose_warp(const RepDev& R, int ns, int lan
         const float4 p = sites[s];
         const double ux = mesh_u(R, p.x, 0), uy = mesh_u(R, p.y, 1), uz = mesh_u(R, p.z, 2);
         const double fx = floor(ux), fy = floor(uy), fz = floor(uz);
-        double mz[4];
+        double mx[4], my[4], mz[4];
+        bspline4(ux - fx, mx);
+        bspline4(uy - fy, my);
         bspline4(uz - fz, mz);
         const int n1 = R.pme_n[1], n2 = R.pme_n[2];
         const int z0 = mesh_index(fz, 0, n2), z1 = mesh_index(fz, 1, n2), z2 = mesh_index(fz, 2, n2),
@@ -475,7 +488,7 @@ __device__ __forceinline__ double pme_pose_warp(const RepDev& R, int ns, int lan
             const int a = r >> 2, b = r & 3;
             const double* row = R.pme_phi + ((size_t)mesh_index(fx, a, R.pme_n[0]) * n1 + mesh_index(fy, b, n1)) * n2;
             const double t = mz[0] * row[z0] + mz[1] * row[z1] + mz[2] * row[z2] + mz[3] * row[z3];
-            e += bspline4_at(ux - fx, a) * bspline4_at(uy - fy, b) * t;
+            e += sel4(mx, a) * sel4(my, b) * t;
         }
         e *= (double)p.w;
     }
@@ -509,8 +522,12 @@ __device__ __forceinline__ void pme_grad_warp(const RepDev& R, int ns, int lane,
         const float4 p = sites[ms];
         const double ux = mesh_u(R, p.x, 0), uy = mesh_u(R, p.y, 1), uz = mesh_u(R, p.z, 2);
         const double fx = floor(ux), fy = floor(uy), fz = floor(uz);
-        double mz[4], dz[4];
+        double mx[4], my[4], mz[4], dx[4], dy[4], dz[4];
+        bspline4(ux - fx, mx);
+        bspline4(uy - fy, my);
         bspline4(uz - fz, mz);
+        bspline4_d(ux - fx, dx);
+        bspline4_d(uy - fy, dy);
         bspline4_d(uz - fz, dz);
         const int n1 = R.pme_n[1], n2 = R.pme_n[2];
         const int z0 = mesh_index(fz, 0, n2), z1 = mesh_index(fz, 1, n2), z2 = mesh_index(fz, 2, n2),
@@ -521,9 +538,9 @@ __device__ __forceinline__ void pme_grad_warp(const RepDev& R, int ns, int lane,
             const double v0 = row[z0], v1 = row[z1], v2 = row[z2], v3 = row[z3];
             const double t = mz[0] * v0 + mz[1] * v1 + mz[2] * v2 + mz[3] * v3;
             const double tz = dz[0] * v0 + dz[1] * v1 + dz[2] * v2 + dz[3] * v3;
-            const double wx = bspline4_at(ux - fx, a), wy = bspline4_at(uy - fy, b);
-            px += bspline4_d_at(ux - fx, a) * wy * t;
-            py += wx * bspline4_d_at(uy - fy, b) * t;
+            const double wx = sel4(mx, a), wy = sel4(my, b);
+            px += sel4(dx, a) * wy * t;
+            py += wx * sel4(dy, b) * t;
             pz += wx * wy * tz;
         }
     }
