@@ -1231,7 +1231,7 @@ __global__ void __launch_bounds__(kWarpsE * 32)
         long long npair = 0;
         const int nwin = R.span[0] * R.span[1] * R.span[2];
         energy_cells(R, B, ns, centres[3 * p], centres[3 * p + 1], centres[3 * p + 2], self ? self[p] : -1,
-                     z * nwin / nslab, (z + 1) * nwin / nslab, lane, acc, ng, npair);
+                     z, nwin, lane, acc, ng, npair, nullptr, 0, nslab);  // interleaved, as in energy_item
         if (R.pme && z == 0) acc += pme_pose_warp(R, ns, lane, B.site_abs, self ? self[p] : -1);
         acc = warp_sum(acc);
         if (lane == 0) {

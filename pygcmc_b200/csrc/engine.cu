@@ -201,6 +201,15 @@ struct gcmc_ctx {
     long long spin_cap = kPersistSpinCap;
     int gridF = 0;       // k_energy_fb CTAs
     std::vector<int> br_off;  // branch b holds replicas [br_off[b], br_off[b+1])
+    // scratch of the explicit-pose entry points, kept between calls (grown on demand, at
+    // most kScratchMax each; larger calls allocate their own) and freed with the context:
+    // device memory, and page-locked host memory for gcmc_energy_poses' transfers.  Calls on
+    // a context run one after the other on the GPU (order_before / order_after), so they can
+    // share it; the mutex covers the host side.
+    std::mutex scratch_mutex;
+    void* d_scratch = nullptr;
+    void* h_scratch = nullptr;
+    size_t d_scratch_bytes = 0, h_scratch_bytes = 0;
     // ordering of calls that launch on a caller's stream against the context's
     // stream (created once, so such calls allocate nothing): ev_ctx marks the
     // context's work so far, ev_call the caller's launches
@@ -1326,6 +1335,8 @@ int destroy_impl(gcmc_ctx* ctx) {
     if (ctx->d_reps) cudaFree(ctx->d_reps);
     if (ctx->d_reps_b) cudaFree(ctx->d_reps_b);
     if (ctx->d_sync) cudaFree(ctx->d_sync);
+    if (ctx->d_scratch) cudaFree(ctx->d_scratch);
+    if (ctx->h_scratch) cudaFreeHost(ctx->h_scratch);
     if (ctx->ev_ctx) cudaEventDestroy(ctx->ev_ctx);
     if (ctx->ev_call) cudaEventDestroy(ctx->ev_call);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -1700,6 +1711,49 @@ int order_after(gcmc_ctx* ctx, cudaStream_t s) {
     CK(cudaEventRecord(ctx->ev_call, s));
     CK(cudaStreamWaitEvent(ctx->stream, ctx->ev_call, 0));
     return GCMC_OK;
+}
+
+constexpr size_t kScratchMax = 64u << 20;
+
+// The context's scratch, at least this large (scratch_mutex held).  The device block is
+// stream-ordered on the context's stream, which waits for every call's launches; a
+// caller's stream is ordered after it by order_before.
+int grow_scratch(gcmc_ctx* ctx, size_t dev_bytes, size_t host_bytes) {
+    if (dev_bytes > ctx->d_scratch_bytes) {
+        if (ctx->d_scratch) cudaFreeAsync(ctx->d_scratch, ctx->stream);
+        ctx->d_scratch = nullptr;
+        ctx->d_scratch_bytes = 0;
+        dev_bytes = std::max(dev_bytes, (size_t)1 << 20);
+        CK(cudaMallocAsync(&ctx->d_scratch, dev_bytes, ctx->stream));
+        ctx->d_scratch_bytes = dev_bytes;
+    }
+    if (host_bytes > ctx->h_scratch_bytes) {  // (its users wait for their copies before they return)
+        if (ctx->h_scratch) cudaFreeHost(ctx->h_scratch);
+        ctx->h_scratch = nullptr;
+        ctx->h_scratch_bytes = 0;
+        host_bytes = std::max(host_bytes, (size_t)256 << 10);
+        CK(cudaHostAlloc(&ctx->h_scratch, host_bytes, cudaHostAllocDefault));
+        ctx->h_scratch_bytes = host_bytes;
+    }
+    return GCMC_OK;
+}
+
+// Consecutive pieces of a scratch block, 256-byte aligned.
+struct Carver {
+    size_t at = 0;
+    size_t take(size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) & ~(size_t)255;
+        return o;
+    }
+};
+
+// Work items per explicit pose: as many as give every resident warp of the pose-energy
+// grid an item, at most the context's limit.  (The limit for any number of poses made
+// 122,880 items of 8192 poses, 128 us a launch: each builds its pose and walks for itself;
+// few poses keep it, their latency is one item's.)
+int pose_splits(const gcmc_ctx* ctx, const RepHost& h, int nposes) {
+    return std::max(1, std::min(h.nslab, ctx->gridE * kWarpsE / std::max(1, nposes)));
 }
 
 }  // namespace
@@ -2108,57 +2162,63 @@ int gcmc_energy_poses(gcmc_ctx* ctx, int32_t rep, const float* xyz, const float*
     RepHost& h = ctx->reps[rep];
     for (int s = 0; s < nsites; ++s)
         if (site_type[s] < 0 || site_type[s] >= h.ffX) return GCMC_ERR_ARG;
-    const int nslab = h.nslab;
-    float *dxyz = nullptr, *dq = nullptr, *dc = nullptr;
-    int *dt = nullptr, *dself = nullptr, *dng = nullptr;
-    double* dout = nullptr;
-    int st = GCMC_OK;
-    std::vector<int> selfv(nposes, -1);
-    if (self) std::copy(self, self + nposes, selfv.begin());
-    std::vector<double> part((size_t)nposes * nslab);
-    std::vector<int> ngp((size_t)nposes * nslab);
-    do {
-        if ((st = dalloc(&dxyz, (size_t)nposes * nsites * 3)) || (st = dalloc(&dq, nsites)) ||
-            (st = dalloc(&dt, nsites)) || (st = dalloc(&dc, (size_t)nposes * 3)) || (st = dalloc(&dself, nposes)) ||
-            (st = dalloc(&dout, (size_t)nposes * nslab)) || (st = dalloc(&dng, (size_t)nposes * nslab)))
-            break;
-        cudaStream_t s = ctx->stream;
-        if (cudaMemcpyAsync(dxyz, xyz, sizeof(float) * nposes * nsites * 3, cudaMemcpyHostToDevice, s) ||
-            cudaMemcpyAsync(dq, site_q, sizeof(float) * nsites, cudaMemcpyHostToDevice, s) ||
-            cudaMemcpyAsync(dt, site_type, sizeof(int) * nsites, cudaMemcpyHostToDevice, s) ||
-            cudaMemcpyAsync(dc, centres, sizeof(float) * nposes * 3, cudaMemcpyHostToDevice, s) ||
-            cudaMemcpyAsync(dself, selfv.data(), sizeof(int) * nposes, cudaMemcpyHostToDevice, s)) {
-            st = GCMC_ERR_CUDA;
-            break;
+    const int nslab = pose_splits(ctx, h, nposes);
+    // The poses go through the kept page-locked scratch in blocks: while the GPU evaluates
+    // one, the host copies the next one in.  A block's inputs are one copy, the results of
+    // all blocks of a round one copy back.  (Seven allocations, eight pageable copies and
+    // the sum of the splits on the host took 100 us of a 16-pose call.)
+    constexpr int kBlock = 2048;
+    const size_t per_pose = sizeof(float) * 3 * nsites + sizeof(float) * 3 + (self ? sizeof(int) : 0);
+    const int round = (int)std::min<long long>(
+        nposes, std::max<long long>(kBlock, (long long)((kScratchMax / 4) / (per_pose + sizeof(double) + sizeof(int)))));
+    std::lock_guard<std::mutex> lock(ctx->scratch_mutex);
+    cudaStream_t s = ctx->stream;
+    const size_t head = sizeof(float) * nsites + sizeof(int) * nsites;  // site charges and types, before each block
+    const size_t block_in = (head + per_pose * std::min(kBlock, round) + 255) & ~(size_t)255;
+    const int nblk = (round + kBlock - 1) / kBlock;
+    Carver hc, dc;
+    const size_t h_in = hc.take(block_in * nblk), h_out = hc.take((sizeof(double) + sizeof(int)) * round),
+                 h_err = hc.take(sizeof(int) * ctx->nrep);
+    const size_t d_in = dc.take(block_in * nblk), d_out = dc.take((sizeof(double) + sizeof(int)) * round);
+    const size_t d_part = dc.take(nslab > 1 ? (sizeof(double) + sizeof(int)) * (size_t)kBlock * nslab : 0);
+    int st = grow_scratch(ctx, dc.at, hc.at);
+    if (st != GCMC_OK) return st;
+    char *hb = (char*)ctx->h_scratch, *db = (char*)ctx->d_scratch;
+    if ((st = pme_update(ctx, rep, 1, s)) != GCMC_OK) return st;
+    for (int p0 = 0; p0 < nposes; p0 += round) {
+        const int n = std::min(round, nposes - p0);
+        double* d_e = (double*)(db + d_out);
+        int* d_ng = (int*)(db + d_out + sizeof(double) * n);
+        for (int b = 0; b < n; b += kBlock) {
+            const int m = std::min(kBlock, n - b);
+            const size_t off = block_in * (b / kBlock), nx = sizeof(float) * 3 * nsites * (size_t)m;
+            char* w = hb + h_in + off;
+            std::memcpy(w, site_q, sizeof(float) * nsites);
+            std::memcpy(w + sizeof(float) * nsites, site_type, sizeof(int) * nsites);
+            std::memcpy(w + head, xyz + (size_t)(p0 + b) * nsites * 3, nx);
+            std::memcpy(w + head + nx, centres + (size_t)(p0 + b) * 3, sizeof(float) * 3 * m);
+            if (self) std::memcpy(w + head + nx + sizeof(float) * 3 * m, self + p0 + b, sizeof(int) * m);
+            CK(cudaMemcpyAsync(db + d_in + off, w, head + per_pose * m, cudaMemcpyHostToDevice, s));
+            const char* d = db + d_in + off;
+            double* part = nslab > 1 ? (double*)(db + d_part) : d_e + b;
+            int* ngp = nslab > 1 ? (int*)(db + d_part + sizeof(double) * (size_t)kBlock * nslab) : d_ng + b;
+            k_energy_explicit<<<ctx->gridE, kWarpsE * 32, 0, s>>>(
+                ctx->repdev[rep], (const float*)(d + head), (const float*)d, (const int*)(d + sizeof(float) * nsites),
+                nsites, (const float*)(d + head + nx), self ? (const int*)(d + head + nx + sizeof(float) * 3 * m) : nullptr,
+                m, nslab, part, ngp);
+            if (nslab > 1) k_sum_parts<<<(m + 255) / 256, 256, 0, s>>>(part, ngp, m, nslab, d_e + b, d_ng + b);
         }
-        if ((st = pme_update(ctx, rep, 1, s)) != GCMC_OK) break;
-        k_energy_explicit<<<ctx->gridE, kWarpsE * 32, 0, s>>>(ctx->repdev[rep], dxyz, dq, dt, nsites, dc, dself,
-                                                              nposes, nslab, dout, dng);
-        if (cudaGetLastError() != cudaSuccess ||
-            cudaMemcpyAsync(part.data(), dout, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, s) ||
-            cudaMemcpyAsync(ngp.data(), dng, sizeof(int) * ngp.size(), cudaMemcpyDeviceToHost, s) ||
-            cudaStreamSynchronize(s)) {
-            st = GCMC_ERR_CUDA;
-            break;
-        }
-        for (int p = 0; p < nposes; ++p) {
-            double e = 0.0;
-            int ng = 0;
-            for (int z = 0; z < nslab; ++z) {
-                e += part[(size_t)p * nslab + z];
-                ng += ngp[(size_t)p * nslab + z];
-            }
-            out[p] = e;
-            if (n_groups) n_groups[p] = ng;
-        }
-    } while (0);
-    dfree(dxyz); dfree(dq); dfree(dt); dfree(dc); dfree(dself); dfree(dout); dfree(dng);
-    if (st == GCMC_OK) {
-        int32_t err = 0;
-        gcmc_device_error(ctx, &err);
-        if (err) st = GCMC_ERR_DEVICE;
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(hb + h_out, db + d_out, (sizeof(double) + sizeof(int)) * n, cudaMemcpyDeviceToHost, s));
+        for (int r = 0; r < ctx->nrep; ++r)
+            CK(cudaMemcpyAsync(hb + h_err + sizeof(int) * r, ctx->reps[r].err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        std::memcpy(out + p0, hb + h_out, sizeof(double) * n);
+        if (n_groups) std::memcpy(n_groups + p0, hb + h_out + sizeof(double) * n, sizeof(int) * n);
+        for (int r = 0; r < ctx->nrep; ++r)
+            if (((const int*)(hb + h_err))[r]) return GCMC_ERR_DEVICE;
     }
-    return st;
+    return GCMC_OK;
 }
 
 int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float* d_site_q,
@@ -2174,67 +2234,69 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
     if (h.pme) return GCMC_ERR_ARG;  // gradients are of the plain-cutoff energy
     for (int s = 0; s < nsites; ++s)
         if (site_type[s] < 0 || site_type[s] >= h.ffX) return GCMC_ERR_ARG;
-    const int nslab = h.nslab;
+    const int nslab = pose_splits(ctx, h, nposes);
     const size_t ntab = (size_t)h.ffX * h.ffY;
     const size_t tab_smem = d_gff ? (size_t)nsites * h.ffY * 2 * sizeof(float) : 0;
     if (tab_smem > 160 * 1024) return GCMC_ERR_LIMIT;
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    {
-        const int ost = order_before(ctx, s);
-        if (ost != GCMC_OK) return ost;
-    }
-    RepDev R = ctx->repdev[rep];
-    float2* lj = nullptr;
-    double *epart = nullptr, *glj = nullptr;
-    int* ngpart = nullptr;
-    float4* gpart = nullptr;
+    const bool grads = d_gxyz || d_gq || d_gff;
+    Carver c;
+    const size_t o_lj = c.take(d_ff ? sizeof(float2) * ntab : 0);
+    const size_t o_e = c.take(d_energy ? sizeof(double) * nposes * nslab : 0);
+    const size_t o_ng = c.take(d_energy ? sizeof(int) * nposes * nslab : 0);
+    const size_t o_g = c.take(grads ? sizeof(float4) * nposes * nslab * nsites : 0);
+    const size_t o_glj = c.take(d_gff ? sizeof(double) * ntab * 2 : 0);
+    // scratch: the context's, or for a large call or one that is being captured into a
+    // graph (whose replays are not ordered against other calls) an allocation of its own.
+    // (Five stream-ordered allocations a call, whose pool a synchronising caller empties
+    // each time, cost more than the kernels.)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cap));
+    const bool own = cap != cudaStreamCaptureStatusNone || c.at > kScratchMax;
+    std::unique_lock<std::mutex> lock(ctx->scratch_mutex, std::defer_lock);
+    char* w = nullptr;
     int st = GCMC_OK;
-    auto amalloc = [&](void** p, size_t bytes) {
-        if (st == GCMC_OK && cudaMallocAsync(p, bytes, s) != cudaSuccess) st = GCMC_ERR_CUDA;
-    };
-    if (d_ff) {
-        amalloc((void**)&lj, sizeof(float2) * ntab);
-        if (st == GCMC_OK) {
+    if (!own) {  // held until the call is ordered before the next one that uses the scratch
+        lock.lock();
+        if ((st = grow_scratch(ctx, c.at, 0)) != GCMC_OK) return st;
+        w = (char*)ctx->d_scratch;
+    }
+    if ((st = order_before(ctx, s)) != GCMC_OK) return st;
+    if (own && cudaMallocAsync((void**)&w, c.at, s) != cudaSuccess) st = GCMC_ERR_CUDA;
+    if (st == GCMC_OK) {
+        RepDev R = ctx->repdev[rep];
+        float2* lj = (float2*)(w + o_lj);
+        double* glj = d_gff ? (double*)(w + o_glj) : nullptr;
+        float4* gpart = (float4*)(w + o_g);
+        if (d_ff) {
             k_ff_to_lj<<<(int)((ntab + 255) / 256), 256, 0, s>>>(d_ff, lj, (int)ntab);
             R.lj = lj;
         }
-    }
-    if (d_energy) {
-        amalloc((void**)&epart, sizeof(double) * nposes * nslab);
-        amalloc((void**)&ngpart, sizeof(int) * nposes * nslab);
-        if (st == GCMC_OK) {
+        if (d_energy) {
+            double* epart = nslab > 1 ? (double*)(w + o_e) : d_energy;
             k_energy_explicit<<<ctx->gridE, kWarpsE * 32, 0, s>>>(R, d_xyz, d_site_q, d_site_type, nsites, d_centres,
-                                                                  d_self, nposes, nslab, epart, ngpart);
-            k_sum_parts<<<(nposes + 255) / 256, 256, 0, s>>>(epart, ngpart, nposes, nslab, d_energy, nullptr);
+                                                                  d_self, nposes, nslab, epart, (int*)(w + o_ng));
+            if (nslab > 1)
+                k_sum_parts<<<(nposes + 255) / 256, 256, 0, s>>>(epart, (int*)(w + o_ng), nposes, nslab, d_energy,
+                                                                 nullptr);
         }
-    }
-    if (d_gxyz || d_gq || d_gff) {
-        amalloc((void**)&gpart, sizeof(float4) * nposes * nslab * nsites);
-        if (d_gff) {
-            amalloc((void**)&glj, sizeof(double) * ntab * 2);
-            if (st == GCMC_OK && cudaMemsetAsync(glj, 0, sizeof(double) * ntab * 2, s) != cudaSuccess)
+        if (grads) {
+            if (d_gff && cudaMemsetAsync(glj, 0, sizeof(double) * ntab * 2, s) != cudaSuccess) st = GCMC_ERR_CUDA;
+            if (tab_smem > 0 && cudaFuncSetAttribute(k_energy_grad, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)tab_smem) != cudaSuccess)
                 st = GCMC_ERR_CUDA;
+            if (st == GCMC_OK) {
+                k_energy_grad<<<std::max(1, ctx->sms) * 4, kWarpsG * 32, tab_smem, s>>>(
+                    R, d_xyz, d_site_q, d_site_type, nsites, d_centres, d_self, nposes, nslab, d_gout, gpart, glj);
+                if (d_gxyz || d_gq)
+                    k_sum_grad<<<(nposes * nsites + 255) / 256, 256, 0, s>>>(gpart, nposes, nslab, nsites, d_gxyz,
+                                                                             d_gq);
+                if (d_gff) k_glj_to_gff<<<(int)((ntab + 255) / 256), 256, 0, s>>>(glj, d_ff, d_gff, (int)ntab);
+            }
         }
-        if (st == GCMC_OK && tab_smem > 0 &&
-            cudaFuncSetAttribute(k_energy_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab_smem) !=
-                cudaSuccess)
-            st = GCMC_ERR_CUDA;
-        if (st == GCMC_OK) {
-            int sms = 0;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-            k_energy_grad<<<std::max(1, sms) * 4, kWarpsG * 32, tab_smem, s>>>(
-                R, d_xyz, d_site_q, d_site_type, nsites, d_centres, d_self, nposes, nslab, d_gout, gpart, glj);
-            if (d_gxyz || d_gq)
-                k_sum_grad<<<(nposes * nsites + 255) / 256, 256, 0, s>>>(gpart, nposes, nslab, nsites, d_gxyz, d_gq);
-            if (d_gff) k_glj_to_gff<<<(int)((ntab + 255) / 256), 256, 0, s>>>(glj, d_ff, d_gff, (int)ntab);
-        }
+        if (cudaGetLastError() != cudaSuccess) st = GCMC_ERR_CUDA;
     }
-    if (st == GCMC_OK && cudaGetLastError() != cudaSuccess) st = GCMC_ERR_CUDA;
-    if (lj) cudaFreeAsync(lj, s);
-    if (epart) cudaFreeAsync(epart, s);
-    if (ngpart) cudaFreeAsync(ngpart, s);
-    if (gpart) cudaFreeAsync(gpart, s);
-    if (glj) cudaFreeAsync(glj, s);
+    if (own && w) cudaFreeAsync(w, s);
     if (st == GCMC_OK) st = order_after(ctx, s);
     return st;
 }
@@ -2280,12 +2342,12 @@ int gcmc_energy_poses_noalloc(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, co
         return GCMC_ERR_ARG;
     if (nsites < 1 || nsites > kMaxSites) return GCMC_ERR_LIMIT;
     if (nposes <= 0) return GCMC_OK;
-    const int nslab = ctx->reps[rep].nslab;
-    if ((long long)nposes * nslab > kNoAllocMaxParts) {
+    const int cap = ctx->reps[rep].nslab, nslab = pose_splits(ctx, ctx->reps[rep], nposes);
+    if ((long long)nposes * cap > kNoAllocMaxParts) {
         std::fprintf(stderr,
                      "gcmc_b200: gcmc_energy_poses_noalloc: %d poses x %d splits exceed the %d partials of its "
                      "fixed %zu-byte scratch (at most %d poses per call for this context)\n",
-                     nposes, nslab, kNoAllocMaxParts, kNoAllocScratchBytes, kNoAllocMaxParts / nslab);
+                     nposes, cap, kNoAllocMaxParts, kNoAllocScratchBytes, kNoAllocMaxParts / cap);
         return GCMC_ERR_LIMIT;
     }
     int dev = 0;

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kWarpsG * 32)
         long long npair = 0;
         const int nwin = R.span[0] * R.span[1] * R.span[2];
         walk_cells(R, B, ns, centres[3 * p], centres[3 * p + 1], centres[3 * p + 2], self ? self[p] : -1,
-                   z * nwin / nslab, (z + 1) * nwin / nslab, lane, sink, ng, npair);
+                   z, nwin, lane, sink, ng, npair, nullptr, 0, nslab);
         // sum the atom subsets of each site in a fixed order
         stages[warp].red[lane] = make_float4(sink.gx, sink.gy, sink.gz, sink.gq);
         __syncwarp();
