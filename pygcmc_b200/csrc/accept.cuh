@@ -22,8 +22,12 @@
 
 namespace gcmc {
 
-constexpr int kAcceptThreads = 1024;
+// Half of what an SM could hold: the walk's critical path is one warp's, and with 128
+// registers a thread nothing of it spills (1024 threads: protein step 41.8 us, 40.3 now).
+constexpr int kAcceptThreads = 512;
+static_assert(kAcceptThreads >= kPrepThreads, "bin_entries' entries per thread");
 constexpr int kNbHalf = kMaxPoses * kMaxWords / 2;  // words
+constexpr int kListLen = kMaxPoses * (int)(sizeof(double) / sizeof(unsigned short));  // entries in AcceptSmem::E
 
 struct AcceptSmem {
     double E[kMaxPoses];      // energy entering the acceptance (force-biased: dE - ln(q ratio) / beta)
@@ -43,9 +47,11 @@ struct AcceptSmem {
     uint32_t spec_mask[32][kMaxWords];
     uint32_t spec_us[33][kMaxWords];  // unused words after the round's first c seeds (c = 0..32)
     int spec_seed[32];
-    int spec_cnt[32];
     int spec_chosen[32];  // Gumbel argmax, -1 if no member has a finite energy
     double spec_lnq[32];  // exact ln(W) - ln(cnt) (W = sum over members of exp(-beta E)) when spec_dec = 0
+    unsigned spec_conf[32];  // later clusters of the round that would lose members to its acceptance
+    unsigned spec_hit[32];   //   and those that would lose their seed
+    unsigned spec_todo;      // clusters to evaluate
     int spec_dec[32];     // +1 / -1: accepted / rejected for every K the round can reach; 0: compare with lnq
     double kr[2];         // K range of the round: the lowest K the step can reach, K at the round's start
     int spec_n;
@@ -460,14 +466,37 @@ __device__ __forceinline__ double key_value(unsigned long long k) {  // inverse 
 // lnq in [M - ln cnt, M]; dec is decided from that range (ln cnt bounded above
 // by ln 2 * ceil(log2 cnt), a margin above the rounding of the exact form),
 // and exp / log are evaluated only when ln u falls inside it.
-__device__ __forceinline__ void eval_cluster(const AcceptSmem& S, uint32_t m, int lane, double lnu, double Klo,
-                                             double Khi, int& cnt_out, int& chosen_out, int& dec_out,
-                                             double& lnq_out) {
-    const int cnt = __reduce_add_sync(kFull, (unsigned)__popc(m));
+// Where a word holds more than two members they go through a list (list[cap], shared
+// memory of this warp) from which the lanes take one each: left to the words' lanes, a
+// cluster of 13 among 70 poses kept three lanes busy, their exponentials one after
+// another.
+__device__ __forceinline__ void eval_cluster(const AcceptSmem& S, unsigned short* list, int cap, uint32_t m, int lane,
+                                             double lnu, double Klo, double Khi, int& cnt_out, int& chosen_out,
+                                             int& dec_out, double& lnq_out) {
+    const int mine = __popc(m);
+    const int cnt = __reduce_add_sync(kFull, (unsigned)mine);
+    const bool listed = cnt <= cap && __reduce_max_sync(kFull, (unsigned)mine) > 2;
+    if (listed) {
+        int o = mine;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int v = __shfl_up_sync(kFull, o, off);
+            if (lane >= off) o += v;
+        }
+        o -= mine;
+        for (uint32_t mm = m; mm; mm &= mm - 1u) list[o++] = (unsigned short)(32 * lane + __ffs(mm) - 1);
+        __syncwarp();
+    }
+    // the lane's members in turn: f(pose)
+    auto each = [&](auto f) {
+        if (listed)
+            for (int x = lane; x < cnt; x += 32) f((int)list[x]);
+        else
+            for (uint32_t mm = m; mm; mm &= mm - 1u) f(32 * lane + __ffs(mm) - 1);
+    };
     unsigned long long best = 0ull, amax = 0ull;
     int bi = -1;
-    for (uint32_t mm = m; mm; mm &= mm - 1u) {
-        const int i = 32 * lane + __ffs(mm) - 1;
+    each([&](int i) {
         const unsigned long long kk = S.key[i];
         if (kk > best) { best = kk; bi = i; }
         const double ai = S.a[i];
@@ -475,7 +504,7 @@ __device__ __forceinline__ void eval_cluster(const AcceptSmem& S, uint32_t m, in
             const unsigned long long ak = key_order(ai);
             if (ak > amax) amax = ak;
         }
-    }
+    });
     // Gumbel argmax (keys are distinct integers; ties cannot occur between members)
     const unsigned hi = (unsigned)(best >> 32);
     const unsigned mhi = __reduce_max_sync(kFull, hi);
@@ -500,10 +529,11 @@ __device__ __forceinline__ void eval_cluster(const AcceptSmem& S, uint32_t m, in
             dec = -1;
         } else {
             double w = 0.0;
-            for (uint32_t mm = m; mm; mm &= mm - 1u) w += exp(S.a[32 * lane + __ffs(mm) - 1] - M);
+            each([&](int i) { w += exp(S.a[i] - M); });
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) w += __shfl_xor_sync(kFull, w, off);
-            lnq = (log(w) + M) - log((double)cnt);
+            const double l = log(lane == 0 ? w : (double)cnt);  // both logarithms at once
+            lnq = (__shfl_sync(kFull, l, 0) + M) - __shfl_sync(kFull, l, 1);
             dec = 0;
         }
     }
@@ -715,17 +745,18 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
         // The sequential definition: seed = lowest unused pose, members = unused
         // poses within the cutoff of the seed, decision, then the members (and on
         // acceptance the unused poses within the cutoff of the chosen pose) leave
-        // the unused set.  Each round, warp 0 seeds up to 32 clusters ahead
+        // the unused set.  Each round, warp 0 seeds up to a warp's worth (at most 32) clusters ahead
         // assuming no acceptance; all warps evaluate them in parallel (member
         // count, Gumbel argmax and the decision for the round's range of K, see
         // eval_cluster); warp 0 then commits them in order.  A speculative cluster is exactly
         // the sequential one while its seed and all its members are still unused
         // (removing other poses can neither lower the seed nor change the member
-        // set); at the first cluster that fails this test the round ends and the
-        // next one reseeds from there.  The commit accepts iff
+        // set).  One that lost members is evaluated again with the others like it; at the
+        // first one that lost its seed the next round seeds afresh.  The commit accepts iff
         // ln u < ln(W) - ln(cnt) + K(n), K = ln(cavityFactor) + B - ln(n+1) for
         // insertions and 0 for translate/rotate -- u < min(1, exp(lnp)) in log form.
         const bool ins = (D.move == MV_INSERT);
+        unsigned short* const list = reinterpret_cast<unsigned short*>(S.E);  // E is done with: member lists
         uint32_t u = 0u;  // warp 0: unused-pose word `lane`
         if (warp == 0 && lane < nw) {
             const int rem = k - 32 * lane;
@@ -737,97 +768,120 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
         // K only decreases (one ln(n+1) step per accepted insertion), down to Klo
         const double Klo = ins ? K0 - S.lnn[min(k, F.maxNum - D.n)] : 0.0;
         int nrounds = 0;
-        int depth = 32;  // speculation depth: halves after a round cut short, doubles after a full one
+        int depth = min(32, nwarps);  // speculation depth: halves after a round cut short, doubles after a full one
+        // (warp 0's state of the seeded clusters; lane c: cluster c's scalars)
+        int nbw = 0, j = 0;      // clusters seeded, committed
+        int cut = 0;             // first cluster that lost its seed (nbw: none)
+        unsigned todo = 0u;      // clusters to evaluate
+        unsigned touched = 0u;   // clusters that lost members since they were evaluated
+        int my_chosen = -1, my_dec = -1;
+        double my_lnq = 0.0, my_lnu = 0.0;
+        unsigned my_conf = 0u, my_hit = 0u;
         for (int round = 0; round <= k; ++round) {
             ++nrounds;
-            if (warp == 0) {  // speculative seeding
-                uint32_t us = u;
-                int nb = 0;
-                S.spec_us[0][lane] = us;
-                while (nb < depth) {
-                    // lowest unused pose: minimum over the lanes' lowest set bits
-                    const unsigned low = us ? (unsigned)(32 * lane + __ffs(us) - 1) : 0xffffffffu;
-                    const unsigned sdu = __reduce_min_sync(kFull, low);
-                    if (sdu == 0xffffffffu) break;
-                    const int sd = (int)sdu;
-                    uint32_t m = (lane < nw) ? (us & S.nb[sd * nw + lane]) : 0u;
-                    if (lane == (sd >> 5)) m |= 1u << (sd & 31);
-                    us &= ~m;
-                    S.spec_mask[nb][lane] = m;
-                    S.spec_us[nb + 1][lane] = us;
-                    if (lane == 0) S.spec_seed[nb] = sd;
-                    ++nb;
+            if (warp == 0) {
+                if (j >= cut) {  // speculative seeding
+                    uint32_t us = u;
+                    int nb = 0;
+                    S.spec_us[0][lane] = us;
+                    while (nb < depth) {
+                        // lowest unused pose: minimum over the lanes' lowest set bits
+                        const unsigned low = us ? (unsigned)(32 * lane + __ffs(us) - 1) : 0xffffffffu;
+                        const unsigned sdu = __reduce_min_sync(kFull, low);
+                        if (sdu == 0xffffffffu) break;
+                        const int sd = (int)sdu;
+                        uint32_t m = (lane < nw) ? (us & S.nb[sd * nw + lane]) : 0u;
+                        if (lane == (sd >> 5)) m |= 1u << (sd & 31);
+                        us &= ~m;
+                        S.spec_mask[nb][lane] = m;
+                        S.spec_us[nb + 1][lane] = us;
+                        if (lane == 0) S.spec_seed[nb] = sd;
+                        ++nb;
+                    }
+                    nbw = cut = nb;
+                    j = 0;
+                    touched = 0u;
+                    todo = nb == 32 ? 0xffffffffu : (1u << nb) - 1u;
+                    __syncwarp();
+                    my_lnu = lane < nb ? S.lnu[S.spec_seed[lane]] : 0.0;
+                } else {  // the touched clusters with the members they have left
+                    for (unsigned t = todo; t; t &= t - 1u) S.spec_mask[__ffs(t) - 1][lane] &= u;
                 }
                 if (lane == 0) {
-                    S.spec_n = nb;
+                    S.spec_n = nbw;
+                    S.spec_todo = todo;
                     S.kr[0] = Klo;
                     S.kr[1] = K;
                 }
             }
             __syncthreads();
-            const int nb = S.spec_n;
-            if (nb == 0) break;
-            if (warp < nb) {  // evaluation, one warp per speculative cluster
-                const int sd = S.spec_seed[warp];
+            const unsigned work = S.spec_todo;
+            if (work == 0u) break;
+            if ((work >> warp) & 1u) {  // evaluation, one warp per speculative cluster
+                const int nb = S.spec_n, sd = S.spec_seed[warp], cap = kListLen / __popc(work);
                 int cnt, chosen, dec;
                 double lnq;
-                eval_cluster(S, S.spec_mask[warp][lane], lane, S.lnu[sd], S.kr[0], S.kr[1], cnt, chosen, dec, lnq);
+                eval_cluster(S, list + cap * __popc(work & ((1u << warp) - 1u)), cap, S.spec_mask[warp][lane], lane,
+                             S.lnu[sd], S.kr[0], S.kr[1], cnt, chosen, dec, lnq);
+                // what its acceptance would take: the later clusters that would lose members
+                // (lane = word), and those that would lose their seed (lane = cluster)
+                unsigned conf = 0u, hit = 0u;
+                if (dec >= 0) {
+                    const uint32_t row = lane < nw ? S.nb[chosen * nw + lane] : 0u;
+#pragma unroll 4
+                    for (int t = warp + 1; t < nb; ++t) conf |= ((row & S.spec_mask[t][lane]) ? 1u : 0u) << t;
+                    conf = __reduce_or_sync(kFull, conf);
+                    bool h = false;
+                    if (lane > warp && lane < nb) {
+                        const int s2 = S.spec_seed[lane];
+                        h = (S.nb[chosen * nw + (s2 >> 5)] >> (s2 & 31)) & 1u;
+                    }
+                    hit = __ballot_sync(kFull, h);
+                }
                 if (lane == 0) {
-                    S.spec_cnt[warp] = cnt;
                     S.spec_lnq[warp] = lnq;
                     S.spec_chosen[warp] = chosen;
                     S.spec_dec[warp] = dec;
+                    S.spec_conf[warp] = conf;
+                    S.spec_hit[warp] = hit;
                 }
             }
             __syncthreads();
             if (warp == 0) {  // in-order commit
-                // Lane j holds speculative cluster j's scalars.  The decision of a
+                // Lane c holds speculative cluster c's scalars.  The decision of a
                 // cluster depends only on its own scalars and on K, which changes only
                 // at an acceptance, so the decisions of all clusters after the last
-                // acceptance are made at once and the clusters before the first
-                // accepting one are committed together: u keeps only the unused
-                // words after their seeding (spec_us).  A cluster is exact while none
-                // of its poses has left u, and only an acceptance (the unused poses
-                // within the cutoff of its chosen pose) removes poses of later
-                // clusters.  A removed pose's cluster is the first c whose seeding
-                // took it out of spec_us (binary search over c), and the earliest
-                // such cluster is where the round ends.
-                const int my_seed = lane < nb ? S.spec_seed[lane] : 0;
-                const int my_chosen = lane < nb ? S.spec_chosen[lane] : -1;
-                const int my_dec = lane < nb ? S.spec_dec[lane] : -1;
-                const double my_lnq = lane < nb ? S.spec_lnq[lane] : 0.0;
-                const double my_lnu = lane < nb ? S.lnu[my_seed] : 0.0;
-                int j = 0;
-                int cut = nb + 1;  // first cluster that lost a pose to an acceptance (nb + 1: none)
-                while (j < nb) {
+                // acceptance are made at once.  An acceptance takes poses of later
+                // clusters out of the unused set (the unused ones within the cutoff of
+                // its chosen pose).  A later cluster that keeps its seed keeps its place
+                // and its other members, and the clusters after it theirs: it is
+                // evaluated again, in parallel with the others so touched, when its turn
+                // comes.  One that loses its seed ends the seeded clusters, as the seeds
+                // after it change.
+                if ((todo >> lane) & 1u) {
+                    my_chosen = S.spec_chosen[lane];
+                    my_dec = S.spec_dec[lane];
+                    my_lnq = S.spec_lnq[lane];
+                    my_conf = S.spec_conf[lane];
+                    my_hit = S.spec_hit[lane];
+                }
+                touched &= ~todo;
+                while (j < cut && !((touched >> j) & 1u)) {
+                    const int lim = touched ? min(cut, __ffs(touched) - 1) : cut;  // (touched clusters lie after j)
                     const unsigned am = __ballot_sync(
-                        kFull, lane >= j && lane < nb && my_chosen >= 0 &&
+                        kFull, lane >= j && lane < lim && my_chosen >= 0 &&
                                    (my_dec > 0 || (my_dec == 0 && my_lnu < my_lnq + K)));
-                    const int ja = am ? __ffs(am) - 1 : nb;  // first accepting cluster (nb: none)
-                    const int jstop = min(ja, cut);          // clusters [j, jstop) are rejected
-                    u &= S.spec_us[jstop][lane];
+                    const int jstop = am ? __ffs(am) - 1 : lim;  // clusters [j, jstop) are rejected
                     wnc += jstop - j;
                     j = jstop;
-                    if (j >= nb || j == cut) break;
+                    if (!am) continue;
                     // cluster j accepts its chosen pose
                     const int chosen = __shfl_sync(kFull, my_chosen, j);
+                    const unsigned hit = __shfl_sync(kFull, my_hit, j);
+                    touched |= __shfl_sync(kFull, my_conf, j);
+                    if (hit) cut = min(cut, __ffs(hit) - 1);
                     u &= S.spec_us[j + 1][lane];
-                    const uint32_t row = lane < nw ? S.nb[chosen * nw + lane] : 0u;
-                    const uint32_t lost = u & row;
-                    u &= ~row;
-                    unsigned first = 0xffffffffu;
-                    for (uint32_t mm = lost; mm; mm &= mm - 1u) {
-                        const int b = __ffs(mm) - 1;
-                        if ((S.spec_us[nb][lane] >> b) & 1u) continue;  // in no cluster of this round
-                        int lo = j + 2, hi = nb;  // first t with the bit cleared in spec_us[t]: cluster t - 1
-                        while (lo < hi) {
-                            const int mid = (lo + hi) >> 1;
-                            if ((S.spec_us[mid][lane] >> b) & 1u) lo = mid + 1; else hi = mid;
-                        }
-                        first = min(first, (unsigned)(lo - 1));
-                    }
-                    first = __reduce_min_sync(kFull, first);
-                    if (first != 0xffffffffu) cut = min(cut, (int)first);
+                    if (lane < nw) u &= ~S.nb[chosen * nw + lane];
                     int slot = 0;
                     if (ins) {
                         if (wn < F.maxNum) {
@@ -844,7 +898,11 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
                     ++wnc;
                     ++j;
                 }
-                depth = (j < nb) ? max(1, min(depth, 2 * j) / 2 + 1) : min(32, 2 * depth);
+                u &= S.spec_us[j][lane];  // the committed clusters' members
+                if (j >= cut)
+                    depth = (j < nbw) ? max(1, min(depth, 2 * j) / 2 + 1) : min(min(32, nwarps), 2 * depth);
+                else
+                    todo = touched & (cut == 32 ? 0xffffffffu : (1u << cut) - 1u);  // (none before j)
             }
             // no barrier here: warp 0 seeds the next round next, and the other warps
             // read its results only after the barrier that follows the seeding
@@ -991,7 +1049,8 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
 template <bool Pme>
 __global__ void __launch_bounds__(kAcceptThreads, 1) k_accept(const RepDev* __restrict__ reps, int nrep, int spec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    pdl_wait();  // a speculating graph launches this kernel as a dependent of the pose energies
+    pdl_wait();  // one-replica graphs launch this kernel as a dependent of the pose energies
+    pdl_trigger();
     accept_step<Pme>(reps[blockIdx.x], spec, smem_raw);
 }
 template __global__ void k_accept<false>(const RepDev* __restrict__, int, int);

@@ -1357,7 +1357,7 @@ int setup_persist(gcmc_ctx* ctx, const gcmc_options& opt) {
     if (!coop) return GCMC_OK;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     CK(cudaFuncSetAttribute(k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AcceptSmem)));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist, kAcceptThreads, sizeof(AcceptSmem)));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist, kPersistThreads, sizeof(AcceptSmem)));
     if (per_sm < 1) return GCMC_OK;
     if (!ctx->d_sync) CK(cudaMalloc(&ctx->d_sync, sizeof(GridSync)));
     ctx->grid_persist = sms;
@@ -1957,7 +1957,7 @@ int gcmc_run(gcmc_ctx* ctx, int32_t nsteps) {
         GridSync* gs = ctx->d_sync;
         long long cap = ctx->spin_cap;
         void* args[] = {(void*)&reps, (void*)&nrep, (void*)&nst, (void*)&gs, (void*)&cap};
-        CK(cudaLaunchCooperativeKernel((const void*)k_persist, dim3(ctx->grid_persist), dim3(kAcceptThreads), args,
+        CK(cudaLaunchCooperativeKernel((const void*)k_persist, dim3(ctx->grid_persist), dim3(kPersistThreads), args,
                                        sizeof(AcceptSmem), ctx->stream));
         return GCMC_OK;
     }

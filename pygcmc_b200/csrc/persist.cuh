@@ -3,7 +3,7 @@
 // moveArray (gcmc/cpp/gcmc.cu:77-98), here with every replica advanced per
 // step -- instead of a captured graph of per-step kernel launches.
 //
-// One CTA of kAcceptThreads threads per SM, all co-resident (cooperative
+// One CTA of kPersistThreads threads per SM, all co-resident (cooperative
 // launch).  Per MC step:
 //   1. every CTA's 32 warps take the step's pose-energy items of all replicas
 //      (the per-pose-warp kernel's items, energy_items);
@@ -25,7 +25,8 @@
 
 namespace gcmc {
 
-constexpr int kPersistWarps = kAcceptThreads / 32;
+constexpr int kPersistThreads = 1024;  // (the energy phase wants the warps)
+constexpr int kPersistWarps = kPersistThreads / 32;
 constexpr long long kPersistSpinCap = 1ll << 24;  // polls of about 100 ns: over a second
 
 struct GridSync {
@@ -64,7 +65,7 @@ __device__ __forceinline__ bool grid_barrier(GridSync* g, long long cap, int* er
     return *ok_sh != 0;
 }
 
-__global__ void __launch_bounds__(kAcceptThreads, 1) k_persist(const RepDev* __restrict__ reps, int nrep, int nsteps,
+__global__ void __launch_bounds__(kPersistThreads, 1) k_persist(const RepDev* __restrict__ reps, int nrep, int nsteps,
                                                                GridSync* gs, long long spin_cap) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int pre[257];

@@ -121,6 +121,9 @@ __device__ __forceinline__ int pose_block(const RepDev& R, float x, float y, flo
     return (bz * R.nbk[1] + by) * R.nbk[0] + bx;
 }
 
+// The least threads a CTA that prepares steps has.
+constexpr int kPrepThreads = 512;
+
 // Bin the step's pose entries (e = i * nvar + v) by pose block and cut each
 // block's entries into tiles of at most kTilePoses: R.pbin (entries by block),
 // R.tiles (block, first entry in pbin, count).  Whole CTA; scratch: 2 x
@@ -135,8 +138,8 @@ __device__ int bin_entries(const RepDev& R, const StepDesc& D, int* scratch, int
     int* chunks = scratch + kMaxBlocks;
     for (int b = tid; b < nblk; b += nt) cnt[b] = 0;
     __syncthreads();
-    constexpr int kPer = (2 * kMaxPoses + 1023) / 1024;
-    int myb[kPer > 0 ? kPer : 1], myr[kPer > 0 ? kPer : 1];
+    constexpr int kPer = (2 * kMaxPoses + kPrepThreads - 1) / kPrepThreads;  // entries per thread at most
+    int myb[kPer], myr[kPer];
     const int startRes = D.move == MV_INSERT ? 0 : R.frag[D.ftype].startRes;
 #pragma unroll
     for (int q = 0; q < kPer; ++q) {
