@@ -201,15 +201,15 @@ struct gcmc_ctx {
     long long spin_cap = kPersistSpinCap;
     int gridF = 0;       // k_energy_fb CTAs
     std::vector<int> br_off;  // branch b holds replicas [br_off[b], br_off[b+1])
-    // scratch of the explicit-pose entry points, kept between calls (grown on demand, at
-    // most kScratchMax each; larger calls allocate their own) and freed with the context:
-    // device memory, and page-locked host memory for gcmc_energy_poses' transfers.  Calls on
-    // a context run one after the other on the GPU (order_before / order_after), so they can
-    // share it; the mutex covers the host side.
+    // device scratch of the explicit-pose entry points: a small block made with the context
+    // and, for calls that need more, a larger one kept between calls (grown on demand, at
+    // most kScratchMax; larger calls allocate their own).  Calls on a context run one after
+    // the other on the GPU (order_before / order_after), so they can share it; the mutex
+    // covers the host side.
     std::mutex scratch_mutex;
+    void* d_small = nullptr;
     void* d_scratch = nullptr;
-    void* h_scratch = nullptr;
-    size_t d_scratch_bytes = 0, h_scratch_bytes = 0;
+    size_t d_scratch_bytes = 0;
     // ordering of calls that launch on a caller's stream against the context's
     // stream (created once, so such calls allocate nothing): ev_ctx marks the
     // context's work so far, ev_call the caller's launches
@@ -1000,6 +1000,8 @@ int energy_warps(int device, int evar, int ebps, int spare_sms) {
 }
 
 
+constexpr size_t kScratchMax = 64u << 20, kScratchSmall = 256u << 10;
+
 // The replicas' mesh sizes (empty without Ewald): the captured mesh passes' grids
 // and shared memory are sized for them.
 std::vector<int> pme_meshes(const gcmc_ctx* ctx) {
@@ -1335,8 +1337,8 @@ int destroy_impl(gcmc_ctx* ctx) {
     if (ctx->d_reps) cudaFree(ctx->d_reps);
     if (ctx->d_reps_b) cudaFree(ctx->d_reps_b);
     if (ctx->d_sync) cudaFree(ctx->d_sync);
+    if (ctx->d_small) cudaFree(ctx->d_small);
     if (ctx->d_scratch) cudaFree(ctx->d_scratch);
-    if (ctx->h_scratch) cudaFreeHost(ctx->h_scratch);
     if (ctx->ev_ctx) cudaEventDestroy(ctx->ev_ctx);
     if (ctx->ev_call) cudaEventDestroy(ctx->ev_call);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -1398,6 +1400,11 @@ int create_impl(int nrep, const gcmc_replica_in* ins, const gcmc_options* optp, 
     }
     if (cudaEventCreateWithFlags(&ctx->ev_ctx, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_call, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        destroy_impl(ctx);
+        return GCMC_ERR_CUDA;
+    }
+    if (cudaMalloc(&ctx->d_small, kScratchSmall) != cudaSuccess) {
         cudaGetLastError();
         destroy_impl(ctx);
         return GCMC_ERR_CUDA;
@@ -1713,30 +1720,59 @@ int order_after(gcmc_ctx* ctx, cudaStream_t s) {
     return GCMC_OK;
 }
 
-constexpr size_t kScratchMax = 64u << 20;
 
-// The context's scratch, at least this large (scratch_mutex held).  The device block is
-// stream-ordered on the context's stream, which waits for every call's launches; a
-// caller's stream is ordered after it by order_before.
-int grow_scratch(gcmc_ctx* ctx, size_t dev_bytes, size_t host_bytes) {
-    if (dev_bytes > ctx->d_scratch_bytes) {
+// The context's device scratch, at least this large (scratch_mutex held).  The large
+// block is stream-ordered on the context's stream, which waits for every call's launches;
+// a caller's stream is ordered after it by order_before.
+int device_scratch(gcmc_ctx* ctx, size_t bytes, char** out) {
+    if (bytes <= kScratchSmall) {
+        *out = (char*)ctx->d_small;
+        return GCMC_OK;
+    }
+    if (bytes > ctx->d_scratch_bytes) {
         if (ctx->d_scratch) cudaFreeAsync(ctx->d_scratch, ctx->stream);
         ctx->d_scratch = nullptr;
         ctx->d_scratch_bytes = 0;
-        dev_bytes = std::max(dev_bytes, (size_t)1 << 20);
-        CK(cudaMallocAsync(&ctx->d_scratch, dev_bytes, ctx->stream));
-        ctx->d_scratch_bytes = dev_bytes;
+        bytes = std::max(bytes, (size_t)4 << 20);
+        CK(cudaMallocAsync(&ctx->d_scratch, bytes, ctx->stream));
+        ctx->d_scratch_bytes = bytes;
     }
-    if (host_bytes > ctx->h_scratch_bytes) {  // (its users wait for their copies before they return)
-        if (ctx->h_scratch) cudaFreeHost(ctx->h_scratch);
-        ctx->h_scratch = nullptr;
-        ctx->h_scratch_bytes = 0;
-        host_bytes = std::max(host_bytes, (size_t)256 << 10);
-        CK(cudaHostAlloc(&ctx->h_scratch, host_bytes, cudaHostAllocDefault));
-        ctx->h_scratch_bytes = host_bytes;
-    }
+    *out = (char*)ctx->d_scratch;
     return GCMC_OK;
 }
+
+// Page-locked staging of host-side calls, one block for the process (pinning memory takes
+// milliseconds, which every new context's first call would pay), at most kStagingMax bytes,
+// given back by gcmc_release_cache.  A call that finds it taken by another thread's, or
+// that cannot have it, stages in ordinary memory.
+constexpr size_t kStagingMax = 16u << 20;
+struct Staging {
+    std::mutex m;
+    char* p = nullptr;
+    size_t n = 0;
+} g_staging;
+
+struct StagingLease {
+    std::unique_lock<std::mutex> lock{g_staging.m, std::try_to_lock};
+    std::vector<char> own;
+    char* get(size_t bytes) {  // bytes <= kStagingMax
+        if (lock.owns_lock()) {
+            if (bytes > g_staging.n) {
+                if (g_staging.p) cudaFreeHost(g_staging.p);
+                g_staging.p = nullptr;
+                const size_t want = bytes > (2u << 20) ? kStagingMax : (size_t)2 << 20;
+                g_staging.n = cudaHostAlloc((void**)&g_staging.p, want, cudaHostAllocPortable) == cudaSuccess ? want : 0;
+                if (!g_staging.n) {
+                    g_staging.p = nullptr;
+                    cudaGetLastError();
+                }
+            }
+            if (bytes <= g_staging.n) return g_staging.p;
+        }
+        own.resize(bytes);
+        return own.data();
+    }
+};
 
 // Consecutive pieces of a scratch block, 256-byte aligned.
 struct Carver {
@@ -2170,8 +2206,9 @@ int gcmc_energy_poses(gcmc_ctx* ctx, int32_t rep, const float* xyz, const float*
     constexpr int kBlock = 2048;
     const size_t per_pose = sizeof(float) * 3 * nsites + sizeof(float) * 3 + (self ? sizeof(int) : 0);
     const int round = (int)std::min<long long>(
-        nposes, std::max<long long>(kBlock, (long long)((kScratchMax / 4) / (per_pose + sizeof(double) + sizeof(int)))));
+        nposes, (long long)((kStagingMax / 2) / (per_pose + sizeof(double) + sizeof(int))));
     std::lock_guard<std::mutex> lock(ctx->scratch_mutex);
+    StagingLease staging;
     cudaStream_t s = ctx->stream;
     const size_t head = sizeof(float) * nsites + sizeof(int) * nsites;  // site charges and types, before each block
     const size_t block_in = (head + per_pose * std::min(kBlock, round) + 255) & ~(size_t)255;
@@ -2180,10 +2217,11 @@ int gcmc_energy_poses(gcmc_ctx* ctx, int32_t rep, const float* xyz, const float*
     const size_t h_in = hc.take(block_in * nblk), h_out = hc.take((sizeof(double) + sizeof(int)) * round),
                  h_err = hc.take(sizeof(int) * ctx->nrep);
     const size_t d_in = dc.take(block_in * nblk), d_out = dc.take((sizeof(double) + sizeof(int)) * round);
-    const size_t d_part = dc.take(nslab > 1 ? (sizeof(double) + sizeof(int)) * (size_t)kBlock * nslab : 0);
-    int st = grow_scratch(ctx, dc.at, hc.at);
+    const size_t parts = nslab > 1 ? (size_t)std::min(kBlock, round) * nslab : 0;  // of a block
+    const size_t d_part = dc.take(sizeof(double) * parts), d_ngp = dc.take(sizeof(int) * parts);
+    char *hb = staging.get(hc.at), *db = nullptr;
+    int st = device_scratch(ctx, dc.at, &db);
     if (st != GCMC_OK) return st;
-    char *hb = (char*)ctx->h_scratch, *db = (char*)ctx->d_scratch;
     if ((st = pme_update(ctx, rep, 1, s)) != GCMC_OK) return st;
     for (int p0 = 0; p0 < nposes; p0 += round) {
         const int n = std::min(round, nposes - p0);
@@ -2201,7 +2239,7 @@ int gcmc_energy_poses(gcmc_ctx* ctx, int32_t rep, const float* xyz, const float*
             CK(cudaMemcpyAsync(db + d_in + off, w, head + per_pose * m, cudaMemcpyHostToDevice, s));
             const char* d = db + d_in + off;
             double* part = nslab > 1 ? (double*)(db + d_part) : d_e + b;
-            int* ngp = nslab > 1 ? (int*)(db + d_part + sizeof(double) * (size_t)kBlock * nslab) : d_ng + b;
+            int* ngp = nslab > 1 ? (int*)(db + d_ngp) : d_ng + b;
             k_energy_explicit<<<ctx->gridE, kWarpsE * 32, 0, s>>>(
                 ctx->repdev[rep], (const float*)(d + head), (const float*)d, (const int*)(d + sizeof(float) * nsites),
                 nsites, (const float*)(d + head + nx), self ? (const int*)(d + head + nx + sizeof(float) * 3 * m) : nullptr,
@@ -2258,8 +2296,7 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
     int st = GCMC_OK;
     if (!own) {  // held until the call is ordered before the next one that uses the scratch
         lock.lock();
-        if ((st = grow_scratch(ctx, c.at, 0)) != GCMC_OK) return st;
-        w = (char*)ctx->d_scratch;
+        if ((st = device_scratch(ctx, c.at, &w)) != GCMC_OK) return st;
     }
     if ((st = order_before(ctx, s)) != GCMC_OK) return st;
     if (own && cudaMallocAsync((void**)&w, c.at, s) != cudaSuccess) st = GCMC_ERR_CUDA;
@@ -2324,6 +2361,10 @@ int gcmc_release_cache(void) {
     if (g_batch) destroy_impl(g_batch);
     g_cache = nullptr;
     g_batch = nullptr;
+    std::lock_guard<std::mutex> staging(g_staging.m);
+    if (g_staging.p) cudaFreeHost(g_staging.p);
+    g_staging.p = nullptr;
+    g_staging.n = 0;
     return GCMC_OK;
 }
 
