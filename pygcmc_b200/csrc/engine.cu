@@ -111,7 +111,7 @@ struct RepHost {
     float2* lj = nullptr;
     int* moves = nullptr;
     FragDev* frag = nullptr;
-    int* totalNum = nullptr;
+    int* totalNum = nullptr;  // (in the context's d_tot)
     StepDesc* desc = nullptr;
     float4* pcen = nullptr;
     int* pslot = nullptr;
@@ -120,7 +120,7 @@ struct RepHost {
     gcmc_step_log* log = nullptr;
     double* logE = nullptr;
     unsigned long long* counters = nullptr;
-    int* err = nullptr;
+    int* err = nullptr;       // (in the context's d_err)
     double* energy = nullptr;
     float4* psite = nullptr;
     // per-step scratch of the speculating copy (single-replica contexts)
@@ -201,6 +201,14 @@ struct gcmc_ctx {
     long long spin_cap = kPersistSpinCap;
     int gridF = 0;       // k_energy_fb CTAs
     std::vector<int> br_off;  // branch b holds replicas [br_off[b], br_off[b+1])
+    // set-up of all replicas in few launches and copies: every replica's SetupDev and small
+    // tables in one block, the replicas' error words and fragment counts in one array each
+    char* d_pack = nullptr;
+    size_t d_pack_bytes = 0;
+    int* d_err = nullptr;  // [nrep]
+    int* d_tot = nullptr;  // the replicas' totalNum, one after another
+    size_t d_tot_cap = 0;
+    int ntot = 0;
     // device scratch of the explicit-pose entry points: a small block made with the context
     // and, for calls that need more, a larger one kept between calls (grown on demand, at
     // most kScratchMax; larger calls allocate their own).  Calls on a context run one after
@@ -255,9 +263,9 @@ int ensure(T** p, size_t* cap, size_t n) {
 
 void free_rep(RepHost& h) {
     dfree(h.xyzq); dfree(h.atype); dfree(h.gcen); dfree(h.gspan); dfree(h.cell_count); dfree(h.cell_ent);
-    dfree(h.gcell); dfree(h.grid); dfree(h.lj); dfree(h.moves); dfree(h.frag); dfree(h.totalNum);
+    dfree(h.gcell); dfree(h.grid); dfree(h.lj); dfree(h.moves); dfree(h.frag);
     dfree(h.desc); dfree(h.pcen); dfree(h.pslot); dfree(h.epart); dfree(h.nbr); dfree(h.log);
-    dfree(h.logE); dfree(h.counters); dfree(h.err);
+    dfree(h.logE); dfree(h.counters);
     dfree(h.energy); dfree(h.pgum); dfree(h.psite);
     dfree(h.raw_atoms); dfree(h.raw_groups); dfree(h.raw_grid); dfree(h.raw_bits); dfree(h.bits_blk);
     dfree(h.desc2); dfree(h.pcen2); dfree(h.pslot2); dfree(h.epart2); dfree(h.nbr2); dfree(h.pgum2); dfree(h.plnu2);
@@ -381,32 +389,167 @@ void pme_influence(const int n[3], const float cryst[3], double alpha, double* G
             }
 }
 
-// The caller's arrays (uploaded unchanged) into the engine's layout: atoms ->
-// (x, y, z, charge) + type, residues -> centre + (atomStart, atomNum), cavity
-// grid points -> float4.
-__global__ void k_unpack_atoms(const Atom* __restrict__ in, float4* __restrict__ xyzq, int* __restrict__ atype,
-                               int n) {
-    for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-        const Atom A = in[a];
-        xyzq[a] = make_float4(A.position[0], A.position[1], A.position[2], A.charge);
-        atype[a] = A.type;
+// Page-locked staging of host-side calls, one block for the process (pinning memory takes
+// milliseconds, which every new context's first call would pay), at most kStagingMax bytes,
+// given back by gcmc_release_cache.  A call that finds it taken by another thread's, or
+// that cannot have it, stages in ordinary memory.
+constexpr size_t kStagingMax = 16u << 20;
+struct Staging {
+    std::mutex m;
+    char* p = nullptr;
+    size_t n = 0;
+} g_staging;
+
+struct StagingLease {
+    std::unique_lock<std::mutex> lock{g_staging.m, std::try_to_lock};
+    std::vector<char> own;
+    char* get(size_t bytes) {
+        if (lock.owns_lock() && bytes <= kStagingMax) {
+            if (bytes > g_staging.n) {
+                if (g_staging.p) cudaFreeHost(g_staging.p);
+                g_staging.p = nullptr;
+                const size_t want = bytes > (2u << 20) ? kStagingMax : (size_t)2 << 20;
+                g_staging.n = cudaHostAlloc((void**)&g_staging.p, want, cudaHostAllocPortable) == cudaSuccess ? want : 0;
+                if (!g_staging.n) {
+                    g_staging.p = nullptr;
+                    cudaGetLastError();
+                }
+            }
+            if (bytes <= g_staging.n) return g_staging.p;
+        }
+        own.resize(bytes);
+        return own.data();
+    }
+};
+
+// One replica's set-up on the device: what k_setup clears, copies from the packed block
+// and unpacks, and what a run can change (k_pack_moved).
+struct SetupDev {
+    // cleared (a null or zero-length entry is skipped)
+    int *cell_count, *gcell, *err, *fbcnt, *pme_dirty;
+    unsigned long long* counters;
+    double *epart, *epart2, *energy, *logE, *pme_q, *pme_phi;
+    float *fpart, *logF;
+    float4* fbprop;
+    CellEnt* cell_ent;
+    StepDesc *desc, *desc2;
+    int *valid2, *abort2, *sstep2;
+    unsigned long long* pending2;
+    long long nepart, nfpart, nlogE, nlogF, nmesh, ncell_ent;
+    int ncell, ngroups, pme;
+    // copied from the packed block
+    const float2* lj_in;
+    const FragDev* frag_in;
+    const int *tot_in, *moves_in;
+    float2* lj;
+    FragDev* frag;
+    int *tot, *moves;
+    int nlj, nfrag, nmoves;
+    // unpacked: the caller's arrays as uploaded
+    Atom* raw_atoms;
+    residue* raw_groups;
+    const float* raw_grid;
+    float4 *xyzq, *gcen, *grid;
+    int* atype;
+    int2* gspan;
+    int natoms, ngrid, zero_grid;
+    // a cavity grid that comes as a gcmc_grid_bits record
+    const uint32_t* words;
+    int* blk;
+    long long nwords, nvox;
+    int nblk, npts, n1, n2;
+    double s0, s1, s2, dx;
+    // the fixed atoms; the fragment slots' groups [g0, g1) and atoms [a0, a1)
+    int nfix, g0, g1, a0, a1;
+};
+
+__device__ __forceinline__ void clear_words(void* p, long long bytes, unsigned v, long long t, long long nt) {
+    if (!p) return;
+    for (long long i = t; i < bytes / 16; i += nt) static_cast<uint4*>(p)[i] = make_uint4(v, v, v, v);
+    for (long long i = bytes / 16 * 4 + t; i < bytes / 4; i += nt) static_cast<unsigned*>(p)[i] = v;
+}
+
+// All replicas' set-up in one launch (blockIdx.y: the replica): the per-step and state
+// buffers cleared, the small tables copied, the caller's arrays unpacked into the engine's
+// layout: atoms -> (x, y, z, charge) + type, residues -> centre + (atomStart, atomNum),
+// cavity grid points -> float4.  (As some twenty copies, clears and launches per replica,
+// 64 replicas' set-up was 1500 driver calls, 5.5 ms on 16 host threads.)
+__global__ void k_setup(const SetupDev* __restrict__ setups) {
+    const SetupDev& S = setups[blockIdx.y];
+    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+    clear_words(S.cell_count, 4ll * S.ncell, 0u, t, nt);
+    clear_words(S.gcell, 4ll * max(1, S.ngroups), 0xffffffffu, t, nt);
+    clear_words(S.counters, 16 * sizeof(unsigned long long), 0u, t, nt);
+    clear_words(S.epart, 8 * S.nepart, 0u, t, nt);
+    clear_words(S.epart2, 8 * S.nepart, 0u, t, nt);
+    clear_words(S.fpart, 4 * S.nfpart, 0u, t, nt);
+    clear_words(S.fbprop, sizeof(float4) * kMaxPoses * 2, 0u, t, nt);
+    clear_words(S.fbcnt, sizeof(int) * kMaxPoses, 0u, t, nt);
+    clear_words(S.logE, 8 * S.nlogE, 0u, t, nt);  // entries past a step's pose count read as zeros
+    clear_words(S.logF, 4 * S.nlogF, 0u, t, nt);
+    clear_words(S.pme_q, 8 * S.nmesh, 0u, t, nt);
+    clear_words(S.pme_phi, 8 * S.nmesh, 0u, t, nt);
+    // a speculative evaluation may read a cell while the accept kernel edits it: every
+    // record slot then holds a span of real atoms (or none)
+    clear_words(S.cell_ent, sizeof(CellEnt) * S.ncell_ent, 0u, t, nt);
+    for (long long i = t; i < S.nlj; i += nt) S.lj[i] = S.lj_in[i];
+    for (long long i = t; i < S.nfrag * (long long)(sizeof(FragDev) / 4); i += nt)
+        reinterpret_cast<unsigned*>(S.frag)[i] = reinterpret_cast<const unsigned*>(S.frag_in)[i];
+    for (long long i = t; i < S.nfrag; i += nt) S.tot[i] = S.tot_in[i];
+    for (long long i = t; i < S.nmoves; i += nt) S.moves[i] = S.moves_in[i];
+    for (long long i = t; i < S.natoms; i += nt) {
+        const Atom A = S.raw_atoms[i];
+        S.xyzq[i] = make_float4(A.position[0], A.position[1], A.position[2], A.charge);
+        S.atype[i] = A.type;
+    }
+    for (long long i = t; i < S.ngroups; i += nt) {
+        const residue R = S.raw_groups[i];
+        S.gcen[i] = make_float4(R.position[0], R.position[1], R.position[2], 0.0f);
+        S.gspan[i] = make_int2(R.atomStart, R.atomNum);
+    }
+    for (long long i = t; i < S.ngrid; i += nt)
+        S.grid[i] = make_float4(S.raw_grid[3 * i], S.raw_grid[3 * i + 1], S.raw_grid[3 * i + 2], 0.0f);
+    if (t == 0) {
+        *S.err = 0;
+        *S.energy = 0.0;
+        S.pme_dirty[0] = S.pme;
+        S.pme_dirty[1] = 0;
+        if (S.zero_grid) S.grid[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+        StepDesc d{};
+        d.move = MV_NONE;
+        *S.desc = d;
+        if (S.desc2) {
+            *S.desc2 = d;
+            for (int c = 0; c < 2; ++c) {
+                S.valid2[c] = 0;
+                S.abort2[c] = -1;  // no step voided
+                S.sstep2[c] = 0;
+                S.pending2[c] = 0ull;
+            }
+        }
     }
 }
-__global__ void k_unpack_groups(const residue* __restrict__ in, float4* __restrict__ gcen, int2* __restrict__ gspan,
-                                int n) {
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
-        const residue R = in[g];
-        gcen[g] = make_float4(R.position[0], R.position[1], R.position[2], 0.0f);
-        gspan[g] = make_int2(R.atomStart, R.atomNum);
+
+// The charges of the current state onto the (cleared) meshes, an atom per warp: the
+// fixed atoms and the occupied fragment slots of every replica under Ewald (blockIdx.y).
+__global__ void __launch_bounds__(256) k_pme_spread_all(const RepDev* __restrict__ reps,
+                                                        const SetupDev* __restrict__ setups) {
+    const RepDev& R = reps[blockIdx.y];
+    if (!R.pme) return;
+    const int lane = threadIdx.x & 31, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+              nw = (gridDim.x * blockDim.x) >> 5;
+    for (int t = -1; t < R.ntypes; ++t) {
+        const int a0 = t < 0 ? 0 : R.gspan[R.frag[t].startRes].x;
+        const int n = t < 0 ? setups[blockIdx.y].nfix : R.totalNum[t] * R.frag[t].nsites;
+        for (int a = w; a < n; a += nw) {
+            const float4 p = R.xyzq[a0 + a];
+            if (p.w != 0.0f) pme_spread_warp(R, R.pme_q, p.x, p.y, p.z, (double)p.w, lane);
+        }
     }
-}
-__global__ void k_unpack_grid(const float* __restrict__ in, float4* __restrict__ grid, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        grid[i] = make_float4(in[3 * i], in[3 * i + 1], in[3 * i + 2], 0.0f);
 }
 
 // Cavity grid from a gcmc_grid_bits record: base point k = the k-th marked
-// voxel.  Three launches, one word per thread: marked voxels per block of
+// voxel.  Three launches for all replicas, one word per thread: marked voxels per block of
 // kBitsThreads words (k_bits_count), an exclusive scan of the block counts with
 // the total checked against the expected point count (k_bits_scan), and the
 // points of each word at its offset (k_bits_expand).
@@ -442,8 +585,12 @@ __device__ __forceinline__ int bits_block_scan(int v, int* total) {
     return before + x - v;
 }
 
-__global__ void __launch_bounds__(kBitsThreads) k_bits_count(const uint32_t* __restrict__ words, long long nwords,
-                                                              long long nvox, int* __restrict__ blk) {
+__global__ void __launch_bounds__(kBitsThreads) k_bits_count(const SetupDev* __restrict__ setups) {
+    const SetupDev& S = setups[blockIdx.y];
+    if ((int)blockIdx.x >= S.nblk) return;
+    const uint32_t* words = S.words;
+    const long long nwords = S.nwords, nvox = S.nvox;
+    int* blk = S.blk;
     const long long w = (long long)blockIdx.x * kBitsThreads + threadIdx.x;
     const int c = w < nwords ? __popc(bits_word(words, w, nvox)) : 0;
     int total = 0;
@@ -451,9 +598,12 @@ __global__ void __launch_bounds__(kBitsThreads) k_bits_count(const uint32_t* __r
     if (threadIdx.x == 0) blk[blockIdx.x] = total;
 }
 
-// One CTA: blk[0, nblk) -> exclusive offsets; blk[nblk] = total; error bit when total != expect.
-__global__ void __launch_bounds__(kBitsThreads) k_bits_scan(int* __restrict__ blk, int nblk, int expect,
-                                                             int* __restrict__ err) {
+// One CTA a replica: blk[0, nblk) -> exclusive offsets; blk[nblk] = total; error bit when total != npts.
+__global__ void __launch_bounds__(kBitsThreads) k_bits_scan(const SetupDev* __restrict__ setups) {
+    const SetupDev& S = setups[blockIdx.x];
+    const int nblk = S.nblk, expect = S.npts;
+    int *blk = S.blk, *err = S.err;
+    if (nblk == 0) return;
     long long carry = 0;
     for (int b0 = 0; b0 < nblk; b0 += kBitsThreads) {
         const int b = b0 + threadIdx.x;
@@ -469,10 +619,14 @@ __global__ void __launch_bounds__(kBitsThreads) k_bits_scan(int* __restrict__ bl
     }
 }
 
-__global__ void __launch_bounds__(kBitsThreads) k_bits_expand(const uint32_t* __restrict__ words, long long nwords,
-                                                               long long nvox, const int* __restrict__ blk, int n1,
-                                                               int n2, double s0, double s1, double s2, double dx,
-                                                               float4* __restrict__ grid, int npts) {
+__global__ void __launch_bounds__(kBitsThreads) k_bits_expand(const SetupDev* __restrict__ setups) {
+    const SetupDev& S = setups[blockIdx.y];
+    if ((int)blockIdx.x >= S.nblk) return;
+    const uint32_t* words = S.words;
+    const long long nwords = S.nwords, nvox = S.nvox;
+    const int *blk = S.blk, n1 = S.n1, n2 = S.n2, npts = S.npts;
+    const double s0 = S.s0, s1 = S.s1, s2 = S.s2, dx = S.dx;
+    float4* grid = S.grid;
     const long long w = (long long)blockIdx.x * kBitsThreads + threadIdx.x;
     uint32_t b = w < nwords ? bits_word(words, w, nvox) : 0u;
     int total = 0;
@@ -502,7 +656,17 @@ __global__ void __launch_bounds__(kBitsThreads) k_bits_expand(const uint32_t* __
         ++k;
     }
 }
-int unpack_blocks(int n) { return std::max(1, std::min((n + 255) / 256, 148 * 8)); }
+// CTAs of 256 threads per replica of a set-up launch over nrep replicas.
+int setup_blocks(int nrep) { return std::max(16, 148 * 8 / nrep); }
+
+// Bytes of a replica's tables in the packed block (16-byte pieces): pair table, fragment
+// types, counts, and the move schedule unless it is long (copied on its own then).
+constexpr int kPackMoves = 16384;
+size_t pack16(size_t bytes) { return (bytes + 15) & ~(size_t)15; }
+size_t pack_bytes(const InfoStruct& I) {
+    return pack16(sizeof(float2) * (size_t)I.ffXNum * I.ffYNum) + pack16(sizeof(FragDev) * I.fragTypeNum) +
+           pack16(sizeof(int) * I.fragTypeNum) + (I.mcsteps <= kPackMoves ? pack16(sizeof(int) * I.mcsteps) : 0);
+}
 
 int energy_warps(int device, int evar, int ebps, int spare_sms);
 
@@ -512,7 +676,10 @@ bool spec_eligible(int nrep, const gcmc_replica_in* ins, const gcmc_options& opt
     return nrep == 1 && opt.speculate >= 0 && opt.proposal != 2 && opt.branches <= 1 && !pme;
 }
 
-int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_options& opt) {
+// Host set-up of replica r: sizes, allocations, the copies of the caller's large arrays;
+// its tables go to `hp` (device: `dp`) and the rest of the device work to `sd`.
+int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_options& opt, SetupDev& sd, char* hp,
+              char* dp) {
     const bool trace = trace_on();
     double tp = trace ? now_ms() : 0.0;
     auto stamp = [&](int k) {
@@ -525,6 +692,7 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
     RepHost& h = ctx->reps[r];
     RepDev& d = ctx->repdev[r];
     std::memset(&d, 0, sizeof(d));
+    std::memset(&sd, 0, sizeof(sd));
     h.startRes.clear();
     h.maxNum.clear();
     h.host_end = 0;
@@ -662,15 +830,17 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
     h.cap = d.cap = cap;
 
     // atoms, groups and cavity grid points are uploaded as the caller holds them
-    // and unpacked on the device (k_unpack_*): no host-side copies of the
-    // large arrays
-    std::vector<float2> lj((size_t)h.ffX * h.ffY);
-    for (size_t x = 0; x < lj.size(); ++x) {
+    // and unpacked on the device (k_setup): no host-side copies of the large arrays
+    const size_t nlj = (size_t)h.ffX * h.ffY;
+    float2* const lj = (float2*)hp;
+    for (size_t x = 0; x < nlj; ++x) {
         float sigma = in.ff[2 * x], eps = in.ff[2 * x + 1];
         lj[x] = make_float2(sigma * sigma * 100.0f, 4.0f * eps);  // gcmc_energy.h:128-130
     }
-    std::vector<FragDev> frag(h.ntypes);
-    std::vector<int> tot(h.ntypes);
+    const size_t o_frag = pack16(sizeof(float2) * nlj), o_tot = o_frag + pack16(sizeof(FragDev) * h.ntypes),
+                 o_moves = o_tot + pack16(sizeof(int) * h.ntypes);
+    FragDev* const frag = (FragDev*)(hp + o_frag);
+    int* const tot = (int*)(hp + o_tot);
     const double V = (double)I->cryst[0] * (double)I->cryst[1] * (double)I->cryst[2];
     for (int t = 0; t < h.ntypes; ++t) {
         const AtomArray& f = in.fragmentInfo[t];
@@ -702,10 +872,10 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
     } while (0)
     AL(h.xyzq, h.natoms); AL(h.atype, h.natoms); AL(h.gcen, h.ngroups); AL(h.gspan, h.ngroups);
     AL(h.cell_count, h.ncell); AL(h.cell_ent, (size_t)h.ncell * cap); AL(h.gcell, h.ngroups);
-    AL(h.grid, h.G); AL(h.lj, lj.size()); AL(h.moves, h.mcsteps); AL(h.frag, h.ntypes);
-    AL(h.totalNum, h.ntypes); AL(h.desc, 1); AL(h.pcen, kMaxPoses); AL(h.pslot, kMaxPoses);
+    AL(h.grid, h.G); AL(h.lj, nlj); AL(h.moves, h.mcsteps); AL(h.frag, h.ntypes);
+    AL(h.desc, 1); AL(h.pcen, kMaxPoses); AL(h.pslot, kMaxPoses);
     AL(h.epart, (size_t)kMaxPoses * 2 * h.slab_cap); AL(h.nbr, (size_t)kMaxPoses * kMaxWords);
-    AL(h.counters, 16); AL(h.err, 1);
+    AL(h.counters, 16);
     AL(h.energy, 1); AL(h.fpart, (size_t)kMaxPoses * 2 * h.slab_cap * 6); AL(h.fbprop, (size_t)kMaxPoses * 2);
     AL(h.fbcnt, kMaxPoses); AL(h.pgum, kMaxPoses); AL(h.plnu, kMaxPoses);
     AL(h.psite, (size_t)kMaxPoses * kMaxSites);
@@ -779,7 +949,6 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
         CK(cudaMemcpyAsync(h.wcost, tmp.data(), sizeof(int) * h.ncell, cudaMemcpyHostToDevice, ctx->stream));
     }
     AL(h.pme_dirty, 2);  // (every replica: the first of a launch holds the mesh passes' counter)
-    CK(cudaMemsetAsync(h.pme_dirty, 0, 2 * sizeof(int), ctx->stream));
     d.pme_dirty = h.pme_dirty;
     // smooth PME: mesh and influence function
     h.pme = opt.pme > 0 || (opt.pme == 0 && I->PME != 0);
@@ -814,7 +983,9 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
             h.pme_g_for = h.pme_g;
             h.pme_tw_for = h.pme_tw;
         }
-        CK(cudaMemsetAsync(h.pme_phi, 0, sizeof(double) * nr, ctx->stream));
+        sd.pme_q = h.pme_q;
+        sd.pme_phi = h.pme_phi;
+        sd.nmesh = (long long)nr;
         for (const void* k : {(const void*)k_pme_fwd_planes, (const void*)k_pme_inv_planes, (const void*)k_pme_axis,
                               (const void*)k_pme_rows_r2c, (const void*)k_pme_rows_c2r})
             CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPmeSmemMax));
@@ -839,65 +1010,61 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
 #undef AL
     stamp(2);
     cudaStream_t s = ctx->stream;
-    if (h.natoms > 0) {
+    if (h.natoms > 0)
         CK(cudaMemcpyAsync(h.raw_atoms, in.atomInfo, sizeof(Atom) * h.natoms, cudaMemcpyHostToDevice, s));
-        k_unpack_atoms<<<unpack_blocks(h.natoms), 256, 0, s>>>(h.raw_atoms, h.xyzq, h.atype, h.natoms);
-    }
-    if (h.ngroups > 0) {
+    if (h.ngroups > 0)
         CK(cudaMemcpyAsync(h.raw_groups, in.residueInfo, sizeof(residue) * h.ngroups, cudaMemcpyHostToDevice, s));
-        k_unpack_groups<<<unpack_blocks(h.ngroups), 256, 0, s>>>(h.raw_groups, h.gcen, h.gspan, h.ngroups);
-    }
-    CK(cudaMemsetAsync(h.cell_count, 0, sizeof(int) * h.ncell, s));
-    CK(cudaMemsetAsync(h.gcell, 0xff, sizeof(int) * std::max(1, h.ngroups), s));
-    if (h.G > 0 && !opt.grid_bits) {
+    if (h.G > 0 && !opt.grid_bits)
         CK(cudaMemcpyAsync(h.raw_grid, in.grid, sizeof(float) * 3 * (size_t)h.G, cudaMemcpyHostToDevice, s));
-        k_unpack_grid<<<unpack_blocks(h.G), 256, 0, s>>>(h.raw_grid, h.grid, h.G);
-    } else if (h.G == 0) {
-        CK(cudaMemsetAsync(h.grid, 0, sizeof(float4), s));
-    }
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(h.lj, lj.data(), sizeof(float2) * lj.size(), cudaMemcpyHostToDevice, s));
-    if (h.mcsteps > 0) {
-        CK(cudaMemcpyAsync(h.moves, in.moveArray, sizeof(int) * h.mcsteps, cudaMemcpyHostToDevice, s));
-        h.moves_host.assign(in.moveArray, in.moveArray + h.mcsteps);
-    }
-    CK(cudaMemcpyAsync(h.frag, frag.data(), sizeof(FragDev) * h.ntypes, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(h.totalNum, tot.data(), sizeof(int) * h.ntypes, cudaMemcpyHostToDevice, s));
-    StepDesc d0{};
-    d0.step = 0;
-    d0.move = MV_NONE;
-    CK(cudaMemcpyAsync(h.desc, &d0, sizeof(StepDesc), cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(h.counters, 0, sizeof(unsigned long long) * 16, s));
-    CK(cudaMemsetAsync(h.err, 0, sizeof(int), s));
-    if (h.log_cap > 0) {  // entries past a step's pose count read as zeros
-        CK(cudaMemsetAsync(h.logE, 0, sizeof(double) * (size_t)h.log_cap * h.log_kmax, s));
-        if (d.fb) CK(cudaMemsetAsync(h.logF, 0, sizeof(float) * (size_t)h.log_cap * h.log_kmax * 12, s));
-    }
-    if (nblk > 0) {  // after the error word is cleared: the scan reports a count mismatch there
+    if (nblk > 0)
         CK(cudaMemcpyAsync(h.raw_bits, reinterpret_cast<const char*>(in.grid) + sizeof(gcmc_grid_bits),
                            sizeof(uint32_t) * (size_t)nwords, cudaMemcpyHostToDevice, s));
-        k_bits_count<<<nblk, kBitsThreads, 0, s>>>(h.raw_bits, nwords, nvox, h.bits_blk);
-        k_bits_scan<<<1, kBitsThreads, 0, s>>>(h.bits_blk, nblk, h.G, h.err);
-        k_bits_expand<<<nblk, kBitsThreads, 0, s>>>(h.raw_bits, nwords, nvox, h.bits_blk, gb.n[1], gb.n[2],
-                                                    gb.start[0], gb.start[1], gb.start[2], gb.dx, h.grid, h.G);
-        CK(cudaGetLastError());
+    if (h.mcsteps > 0) {
+        if (h.mcsteps > kPackMoves)
+            CK(cudaMemcpyAsync(h.moves, in.moveArray, sizeof(int) * h.mcsteps, cudaMemcpyHostToDevice, s));
+        else
+            std::memcpy(hp + o_moves, in.moveArray, sizeof(int) * h.mcsteps);
+        h.moves_host.assign(in.moveArray, in.moveArray + h.mcsteps);
     }
-    CK(cudaMemsetAsync(h.epart, 0, sizeof(double) * kMaxPoses * 2 * h.slab_cap, s));
-    CK(cudaMemsetAsync(h.energy, 0, sizeof(double), s));
-    CK(cudaMemsetAsync(h.fpart, 0, sizeof(float) * kMaxPoses * 2 * h.slab_cap * 6, s));
-    CK(cudaMemsetAsync(h.fbprop, 0, sizeof(float4) * kMaxPoses * 2, s));
-    CK(cudaMemsetAsync(h.fbcnt, 0, sizeof(int) * kMaxPoses, s));
+    sd.cell_count = h.cell_count; sd.ncell = h.ncell;
+    sd.gcell = h.gcell; sd.ngroups = h.ngroups;
+    sd.err = h.err; sd.fbcnt = h.fbcnt; sd.pme_dirty = h.pme_dirty; sd.counters = h.counters;
+    sd.epart = h.epart; sd.energy = h.energy; sd.fpart = h.fpart; sd.fbprop = h.fbprop;
+    sd.nepart = (long long)kMaxPoses * 2 * h.slab_cap;
+    sd.nfpart = sd.nepart * 6;
+    if (h.log_cap > 0) {
+        sd.logE = h.logE;
+        sd.nlogE = (long long)h.log_cap * h.log_kmax;
+        if (d.fb) {
+            sd.logF = h.logF;
+            sd.nlogF = (long long)h.log_cap * h.log_kmax * 12;
+        }
+    }
+    sd.desc = h.desc;
     if (ctx->spec) {
-        // a speculative evaluation may read a cell while the accept kernel edits it:
-        // every record slot then holds a span of real atoms (or none)
-        CK(cudaMemsetAsync(h.cell_ent, 0, sizeof(CellEnt) * (size_t)h.ncell * cap, s));
-        CK(cudaMemcpyAsync(h.desc2, &d0, sizeof(StepDesc), cudaMemcpyHostToDevice, s));
-        CK(cudaMemsetAsync(h.epart2, 0, sizeof(double) * kMaxPoses * 2 * h.slab_cap, s));
-        CK(cudaMemsetAsync(h.valid2, 0, sizeof(int) * 2, s));
-        CK(cudaMemsetAsync(h.abort2, 0xff, sizeof(int) * 2, s));  // -1: no step voided
-        CK(cudaMemsetAsync(h.sstep2, 0, sizeof(int) * 2, s));
-        CK(cudaMemsetAsync(h.pending2, 0, sizeof(unsigned long long) * 2, s));
+        sd.epart2 = h.epart2; sd.desc2 = h.desc2; sd.valid2 = h.valid2; sd.abort2 = h.abort2;
+        sd.sstep2 = h.sstep2; sd.pending2 = h.pending2;
+        sd.cell_ent = h.cell_ent; sd.ncell_ent = (long long)h.ncell * cap;
     }
+    sd.pme = h.pme;
+    sd.lj_in = (const float2*)dp; sd.lj = h.lj; sd.nlj = (int)nlj;
+    sd.frag_in = (const FragDev*)(dp + o_frag); sd.frag = h.frag; sd.nfrag = h.ntypes;
+    sd.tot_in = (const int*)(dp + o_tot); sd.tot = h.totalNum;
+    sd.moves_in = (const int*)(dp + o_moves); sd.moves = h.moves;
+    sd.nmoves = h.mcsteps > kPackMoves ? 0 : h.mcsteps;
+    sd.raw_atoms = h.raw_atoms; sd.xyzq = h.xyzq; sd.atype = h.atype; sd.natoms = h.natoms;
+    sd.raw_groups = h.raw_groups; sd.gcen = h.gcen; sd.gspan = h.gspan;
+    sd.raw_grid = h.raw_grid; sd.grid = h.grid;
+    sd.ngrid = opt.grid_bits ? 0 : h.G;
+    sd.zero_grid = h.G == 0;
+    if (nblk > 0) {
+        sd.words = h.raw_bits; sd.blk = h.bits_blk; sd.nwords = nwords; sd.nvox = nvox;
+        sd.nblk = nblk; sd.npts = h.G; sd.n1 = gb.n[1]; sd.n2 = gb.n[2];
+        sd.s0 = gb.start[0]; sd.s1 = gb.start[1]; sd.s2 = gb.start[2]; sd.dx = gb.dx;
+    }
+    sd.nfix = h.nfix_atoms;
+    sd.g0 = in.fragmentInfo[0].startRes; sd.g1 = h.ngroups;
+    sd.a0 = h.frag_atoms.x; sd.a1 = h.frag_atoms.y;
 
     stamp(3);
     d.xyzq = h.xyzq; d.atype = h.atype; d.gcen = h.gcen; d.gspan = h.gspan;
@@ -920,6 +1087,49 @@ int setup_rep(gcmc_ctx* ctx, int r, const gcmc_replica_in& in, const gcmc_option
         d.valid = h.valid2; d.pairs_pending = h.pending2; d.abort = h.abort2; d.spec_step = h.sstep2;
         b.valid = h.valid2 + 1; b.pairs_pending = h.pending2 + 1; b.abort = h.abort2 + 1; b.spec_step = h.sstep2 + 1;
     }
+    return GCMC_OK;
+}
+
+// Set-up of all replicas (on host threads), their tables and device work in one copy and
+// a few launches.  `staging` holds the packed block until the context's stream has been
+// waited for.
+int setup_all(gcmc_ctx* ctx, const gcmc_replica_in* ins, const gcmc_options& opt, StagingLease& staging) {
+    const int nrep = ctx->nrep;
+    const size_t head = pack16(sizeof(SetupDev) * nrep);
+    std::vector<size_t> off(nrep), toff(nrep);
+    size_t bytes = head, ntot = 0;
+    for (int r = 0; r < nrep; ++r) {
+        off[r] = bytes;
+        toff[r] = ntot;
+        bytes += pack_bytes(*ins[r].info);
+        ntot += ins[r].info->fragTypeNum;
+    }
+    int st = ensure(&ctx->d_pack, &ctx->d_pack_bytes, bytes);
+    if (st == GCMC_OK) st = ensure(&ctx->d_tot, &ctx->d_tot_cap, ntot);
+    if (st != GCMC_OK) return st;
+    ctx->ntot = (int)ntot;
+    char* const hp = staging.get(bytes);
+    SetupDev* const sd = (SetupDev*)hp;
+    for (int r = 0; r < nrep; ++r) {
+        ctx->reps[r].err = ctx->d_err + r;
+        ctx->reps[r].totalNum = ctx->d_tot + toff[r];
+    }
+    st = for_each_rep(nrep, ctx->device, [&](int r) {
+        return setup_rep(ctx, r, ins[r], opt, sd[r], hp + off[r], ctx->d_pack + off[r]);
+    });
+    if (st != GCMC_OK) return st;
+    int nblk = 0;
+    for (int r = 0; r < nrep; ++r) nblk = std::max(nblk, sd[r].nblk);
+    CK(cudaMemcpyAsync(ctx->d_pack, hp, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    const SetupDev* d = (const SetupDev*)ctx->d_pack;
+    k_setup<<<dim3((unsigned)setup_blocks(nrep), (unsigned)nrep), 256, 0, ctx->stream>>>(d);
+    if (nblk > 0) {  // after the error words are cleared: the scan reports a count mismatch there
+        const dim3 gb((unsigned)nblk, (unsigned)nrep);
+        k_bits_count<<<gb, kBitsThreads, 0, ctx->stream>>>(d);
+        k_bits_scan<<<nrep, kBitsThreads, 0, ctx->stream>>>(d);
+        k_bits_expand<<<gb, kBitsThreads, 0, ctx->stream>>>(d);
+    }
+    CK(cudaGetLastError());
     return GCMC_OK;
 }
 
@@ -1058,19 +1268,12 @@ int pme_update(gcmc_ctx* ctx, int r0, int cnt, cudaStream_t s) {
 }
 
 // The spread charges of the current state (the fixed atoms and the occupied
-// fragment slots; once per set-up, needs d_reps uploaded), marked dirty.
+// fragment slots; once per set-up, needs d_reps uploaded; k_setup marked them dirty).
 int pme_init_fixed(gcmc_ctx* ctx) {
-    for (int r = 0; r < ctx->nrep; ++r) {
-        RepHost& h = ctx->reps[r];
-        if (!h.pme) continue;
-        const size_t nr = (size_t)h.pme_n[0] * h.pme_n[1] * h.pme_n[2];
-        CK(cudaMemsetAsync(h.pme_q, 0, sizeof(double) * nr, ctx->stream));
-        if (h.nfix_atoms > 0)
-            k_pme_spread_range<<<296, 256, 0, ctx->stream>>>(ctx->d_reps + r, h.pme_q, 0, h.nfix_atoms);
-        k_pme_spread_frag<<<148, 256, 0, ctx->stream>>>(ctx->d_reps + r, h.pme_q);
-        CK(cudaMemsetAsync(h.pme_dirty, 1, sizeof(int), ctx->stream));
-        CK(cudaGetLastError());
-    }
+    if (!ctx->pme_any) return GCMC_OK;
+    const dim3 grid((unsigned)std::max(16, 148 * 16 / ctx->nrep), (unsigned)ctx->nrep);
+    k_pme_spread_all<<<grid, 256, 0, ctx->stream>>>(ctx->d_reps, (const SetupDev*)ctx->d_pack);
+    CK(cudaGetLastError());
     return GCMC_OK;
 }
 
@@ -1338,6 +1541,9 @@ int destroy_impl(gcmc_ctx* ctx) {
     if (ctx->d_reps_b) cudaFree(ctx->d_reps_b);
     if (ctx->d_sync) cudaFree(ctx->d_sync);
     if (ctx->d_small) cudaFree(ctx->d_small);
+    if (ctx->d_pack) cudaFree(ctx->d_pack);
+    if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->d_tot) cudaFree(ctx->d_tot);
     if (ctx->d_scratch) cudaFree(ctx->d_scratch);
     if (ctx->ev_ctx) cudaEventDestroy(ctx->ev_ctx);
     if (ctx->ev_call) cudaEventDestroy(ctx->ev_call);
@@ -1404,7 +1610,8 @@ int create_impl(int nrep, const gcmc_replica_in* ins, const gcmc_options* optp, 
         destroy_impl(ctx);
         return GCMC_ERR_CUDA;
     }
-    if (cudaMalloc(&ctx->d_small, kScratchSmall) != cudaSuccess) {
+    if (cudaMalloc(&ctx->d_small, kScratchSmall) != cudaSuccess ||
+        cudaMalloc(&ctx->d_err, sizeof(int) * nrep) != cudaSuccess) {
         cudaGetLastError();
         destroy_impl(ctx);
         return GCMC_ERR_CUDA;
@@ -1413,7 +1620,8 @@ int create_impl(int nrep, const gcmc_replica_in* ins, const gcmc_options* optp, 
     ctx->repdev.resize(nrep);
     for (int r = 0; r < nrep; ++r) ctx->reps[r].frag_atoms = frag_atoms[r];
     ctx->spec = spec_eligible(nrep, ins, opt);
-    if (st == GCMC_OK) st = for_each_rep(nrep, ctx->device, [&](int r) { return setup_rep(ctx, r, ins[r], opt); });
+    StagingLease staging;
+    st = setup_all(ctx, ins, opt, staging);
     if (st == GCMC_OK) {
         finalize_tiling(ctx);
         find_mixed_moves(ctx);
@@ -1474,7 +1682,8 @@ int refill_impl(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins, const gcmc_
     ctx->spec = spec;
     const bool tiled_before = ctx->tiled, pme_before = ctx->pme_any, dual_before = ctx->dual_any;
     const std::vector<int> mesh_before = pme_meshes(ctx);
-    st = for_each_rep(nrep, ctx->device, [&](int r) { return setup_rep(ctx, r, ins[r], opt); });
+    StagingLease staging;
+    st = setup_all(ctx, ins, opt, staging);
     if (st != GCMC_OK) return st;
     if (trace_on()) g_trace[1] = now_ms();
     finalize_tiling(ctx);
@@ -1529,46 +1738,42 @@ gcmc_ctx* g_batch = nullptr;
 // caller's layout into the upload buffers (which hold the caller's arrays as
 // uploaded, so the fields a run never changes keep the caller's values), and
 // one copy per range lands it in place.
-__global__ void k_pack_moved(const float4* __restrict__ gcen, residue* __restrict__ groups, int g0, int g1,
-                             const float4* __restrict__ xyzq, const int* __restrict__ atype, Atom* __restrict__ atoms,
-                             int a0, int a1) {
-    const int ng = g1 - g0, na = a1 - a0, n = ng > na ? ng : na;
+__global__ void k_pack_moved(const SetupDev* __restrict__ setups) {
+    const SetupDev& S = setups[blockIdx.y];
+    const int ng = S.g1 - S.g0, na = S.a1 - S.a0, n = ng > na ? ng : na;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (i < ng) {
-            const float4 c = gcen[g0 + i];
-            residue& R = groups[g0 + i];
+            const float4 c = S.gcen[S.g0 + i];
+            residue& R = S.raw_groups[S.g0 + i];
             R.position[0] = c.x;
             R.position[1] = c.y;
             R.position[2] = c.z;
         }
         if (i < na) {
-            const float4 p = xyzq[a0 + i];
-            Atom& A = atoms[a0 + i];
+            const float4 p = S.xyzq[S.a0 + i];
+            Atom& A = S.raw_atoms[S.a0 + i];
             A.position[0] = p.x;
             A.position[1] = p.y;
             A.position[2] = p.z;
             A.charge = p.w;
-            A.type = atype[a0 + i];
+            A.type = S.atype[S.a0 + i];
         }
     }
 }
 
-// Every replica's changes into the caller's arrays (one stream sync).
+// Every replica's changes into the caller's arrays (one packing launch, one stream sync).
 int download_moved(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins) {
     cudaStream_t s = ctx->stream;
-    std::vector<std::vector<int>> tot(nrep);
+    k_pack_moved<<<dim3((unsigned)setup_blocks(nrep), (unsigned)nrep), 256, 0, s>>>((const SetupDev*)ctx->d_pack);
+    CK(cudaGetLastError());
+    StagingLease staging;
+    int* const tot = (int*)staging.get(sizeof(int) * std::max(1, ctx->ntot));
+    CK(cudaMemcpyAsync(tot, ctx->d_tot, sizeof(int) * ctx->ntot, cudaMemcpyDeviceToHost, s));
     for (int r = 0; r < nrep; ++r) {
         RepHost& h = ctx->reps[r];
         const gcmc_replica_in& in = ins[r];
-        tot[r].resize(h.ntypes);
-        CK(cudaMemcpyAsync(tot[r].data(), h.totalNum, sizeof(int) * h.ntypes, cudaMemcpyDeviceToHost, s));
         const int g0 = in.fragmentInfo[0].startRes, g1 = h.ngroups;
         const int a0 = h.frag_atoms.x, a1 = h.frag_atoms.y;
-        if (g1 <= g0 && a1 <= a0) continue;
-        const int n = std::max(g1 - g0, a1 - a0);
-        k_pack_moved<<<unpack_blocks(n), 256, 0, s>>>(h.gcen, h.raw_groups, g0, g1, h.xyzq, h.atype, h.raw_atoms,
-                                                      a0, a1);
-        CK(cudaGetLastError());
         if (g1 > g0)
             CK(cudaMemcpyAsync(const_cast<residue*>(in.residueInfo) + g0, h.raw_groups + g0,
                                sizeof(residue) * (g1 - g0), cudaMemcpyDeviceToHost, s));
@@ -1579,7 +1784,8 @@ int download_moved(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins) {
     CK(cudaStreamSynchronize(s));
     for (int r = 0; r < nrep; ++r) {
         AtomArray* frag = const_cast<AtomArray*>(ins[r].fragmentInfo);
-        for (int t = 0; t < ctx->reps[r].ntypes; ++t) frag[t].totalNum = tot[r][t];
+        const int* n = tot + (ctx->reps[r].totalNum - ctx->d_tot);
+        for (int t = 0; t < ctx->reps[r].ntypes; ++t) frag[t].totalNum = n[t];
     }
     return GCMC_OK;
 }
@@ -1740,39 +1946,6 @@ int device_scratch(gcmc_ctx* ctx, size_t bytes, char** out) {
     *out = (char*)ctx->d_scratch;
     return GCMC_OK;
 }
-
-// Page-locked staging of host-side calls, one block for the process (pinning memory takes
-// milliseconds, which every new context's first call would pay), at most kStagingMax bytes,
-// given back by gcmc_release_cache.  A call that finds it taken by another thread's, or
-// that cannot have it, stages in ordinary memory.
-constexpr size_t kStagingMax = 16u << 20;
-struct Staging {
-    std::mutex m;
-    char* p = nullptr;
-    size_t n = 0;
-} g_staging;
-
-struct StagingLease {
-    std::unique_lock<std::mutex> lock{g_staging.m, std::try_to_lock};
-    std::vector<char> own;
-    char* get(size_t bytes) {  // bytes <= kStagingMax
-        if (lock.owns_lock()) {
-            if (bytes > g_staging.n) {
-                if (g_staging.p) cudaFreeHost(g_staging.p);
-                g_staging.p = nullptr;
-                const size_t want = bytes > (2u << 20) ? kStagingMax : (size_t)2 << 20;
-                g_staging.n = cudaHostAlloc((void**)&g_staging.p, want, cudaHostAllocPortable) == cudaSuccess ? want : 0;
-                if (!g_staging.n) {
-                    g_staging.p = nullptr;
-                    cudaGetLastError();
-                }
-            }
-            if (bytes <= g_staging.n) return g_staging.p;
-        }
-        own.resize(bytes);
-        return own.data();
-    }
-};
 
 // Consecutive pieces of a scratch block, 256-byte aligned.
 struct Carver {
@@ -2053,12 +2226,10 @@ int gcmc_run_profiled(gcmc_ctx* ctx, int32_t nsteps, float* ms_energy, float* ms
 
 int gcmc_device_error(gcmc_ctx* ctx, int32_t* err) {
     if (!ctx || !err) return GCMC_ERR_ARG;
+    std::vector<int> e(ctx->nrep);
+    CK(cudaMemcpy(e.data(), ctx->d_err, sizeof(int) * ctx->nrep, cudaMemcpyDeviceToHost));
     int acc = 0;
-    for (auto& h : ctx->reps) {
-        int e = 0;
-        CK(cudaMemcpy(&e, h.err, sizeof(int), cudaMemcpyDeviceToHost));
-        acc |= e;
-    }
+    for (int x : e) acc |= x;
     *err = acc;
     return GCMC_OK;
 }
@@ -2248,8 +2419,7 @@ int gcmc_energy_poses(gcmc_ctx* ctx, int32_t rep, const float* xyz, const float*
         }
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(hb + h_out, db + d_out, (sizeof(double) + sizeof(int)) * n, cudaMemcpyDeviceToHost, s));
-        for (int r = 0; r < ctx->nrep; ++r)
-            CK(cudaMemcpyAsync(hb + h_err + sizeof(int) * r, ctx->reps[r].err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(hb + h_err, ctx->d_err, sizeof(int) * ctx->nrep, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         std::memcpy(out + p0, hb + h_out, sizeof(double) * n);
         if (n_groups) std::memcpy(n_groups + p0, hb + h_out + sizeof(double) * n, sizeof(int) * n);

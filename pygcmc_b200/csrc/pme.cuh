@@ -49,26 +49,6 @@ __device__ __forceinline__ double mesh_u(const RepDev& R, double x, int a) {
     return ((x - (double)R.start[a]) / (double)R.L[a]) * (double)R.pme_n[a];
 }
 
-// spread charge q at (x, y, z) onto Q (atomic FP64 adds)
-__device__ __forceinline__ void pme_spread_one(const RepDev& R, double* Q, double x, double y, double z, double q) {
-    double mx[4], my[4], mz[4];
-    const double ux = mesh_u(R, x, 0), uy = mesh_u(R, y, 1), uz = mesh_u(R, z, 2);
-    const double fx = floor(ux), fy = floor(uy), fz = floor(uz);
-    bspline4(ux - fx, mx);
-    bspline4(uy - fy, my);
-    bspline4(uz - fz, mz);
-    const int n0 = R.pme_n[0], n1 = R.pme_n[1], n2 = R.pme_n[2];
-    for (int a = 0; a < 4; ++a) {
-        const int i0 = wrapm((int)fx - a, n0);
-        for (int b = 0; b < 4; ++b) {
-            const int i1 = wrapm((int)fy - b, n1);
-            const double wab = q * mx[a] * my[b];
-            double* row = Q + ((size_t)i0 * n1 + i1) * n2;
-            for (int c = 0; c < 4; ++c) atomicAdd(row + wrapm((int)fz - c, n2), wab * mz[c]);
-        }
-    }
-}
-
 // derivatives of bspline4's weights with respect to w
 __device__ __forceinline__ void bspline4_d(double w, double d[4]) {
     const double c = 1.0 - w;
@@ -99,29 +79,6 @@ __device__ __forceinline__ double pme_phi_at(const RepDev& R, double x, double y
         }
     }
     return p;
-}
-
-// Atoms [a0, a1) of the replica spread onto Q (the fixed atoms, once).
-__global__ void k_pme_spread_range(const RepDev* __restrict__ rep, double* Q, int a0, int a1) {
-    const RepDev& R = *rep;
-    for (int a = a0 + blockIdx.x * blockDim.x + threadIdx.x; a < a1; a += gridDim.x * blockDim.x) {
-        const float4 p = R.xyzq[a];
-        if (p.w != 0.0f) pme_spread_one(R, Q, p.x, p.y, p.z, p.w);
-    }
-}
-
-// The occupied fragment atoms of every type spread onto Q.
-__global__ void k_pme_spread_frag(const RepDev* __restrict__ rep, double* Q) {
-    const RepDev& R = *rep;
-    for (int t = 0; t < R.ntypes; ++t) {
-        const FragDev& F = R.frag[t];
-        const int n = R.totalNum[t] * F.nsites;
-        const int a0 = R.gspan[F.startRes].x;
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-            const float4 p = R.xyzq[a0 + i];
-            if (p.w != 0.0f) pme_spread_one(R, Q, p.x, p.y, p.z, p.w);
-        }
-    }
 }
 
 // ---- the mesh transforms ----
