@@ -812,10 +812,10 @@ def run_ours_large(args, ws, rank, local):
                      "peak_source": f"nominal FP32: {sms} SMs x 128 lanes x 2 x {sm_max:.0f} MHz",
                      "avg_step_us_pme_and_energy": e_ms / 16 * 1e3, "avg_accept_us": a_ms / 16 * 1e3,
                      "traffic": None},
-        # per chunk: k_set_run_end, k_prepare; per graph step: each replica's six mesh-update
+        # per chunk: k_set_run_end, k_prepare; per graph step and branch: three mesh-update
         # launches (which return at once when no charge moved), then per branch two force-bias
         # pose-energy launches and the accept kernel
-        "gpu_launches": args.steps * (2 + 32 * ((chunk + 31) // 32) * (6 * nrep + 3 * opt.branches)),
+        "gpu_launches": args.steps * (2 + 32 * ((chunk + 31) // 32) * 6 * opt.branches),
         "clocks": clk,
     }
 

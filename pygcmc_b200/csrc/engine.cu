@@ -2,7 +2,7 @@
 //
 // A context owns the device-resident state of nrep independent replicas
 // (structure-of-arrays, float4 atoms and group centres, a cell grid over group
-// centres) and a CUDA graph of `kGraphSteps` MC steps; each step is one
+// centres) and CUDA graphs of `kGraphSteps` MC steps; each step is one
 // k_energy launch (every replica's pose items) and one k_accept launch (one
 // CTA per replica) that also prepares the next step, so the whole step loop
 // runs without host round trips.  A one-replica context speculates instead
@@ -30,8 +30,11 @@ using namespace gcmc;
 
 namespace {
 
-constexpr int kGraphSteps = 32;
-static_assert(kGraphSteps % 2 == 0, "a speculating graph ends on its start parity");
+// Steps of the captured graphs: a run launches the long one as often as it fits and the
+// short one for the rest (a graph's steps past the run's end are empty launches, about 6 us
+// each: with the long one alone a 24-step run paid 8 of them).
+constexpr int kGraphSteps[2] = {32, 8};
+static_assert(kGraphSteps[0] % 2 == 0 && kGraphSteps[1] % 2 == 0, "a speculating graph ends on its start parity");
 constexpr int kMaxRep = 256;
 thread_local int g_last_status = GCMC_OK;
 
@@ -177,14 +180,16 @@ struct gcmc_ctx {
     std::vector<RepHost> reps;
     std::vector<RepDev> repdev;
     RepDev* d_reps = nullptr;
-    cudaGraphExec_t gexec = nullptr;
+    cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // of kGraphSteps[0], [1] steps
     // speculation (one replica, one branch, no PME, no force bias): the next step's pose
     // energies run beside the accept kernel; a second descriptor copy holds every other
     // step's scratch, and the step loop has one graph per parity of its first step
     bool spec = false;
     RepDev repdev_b{};
     RepDev* d_reps_b = nullptr;
-    cudaGraphExec_t gexec_spec[2] = {nullptr, nullptr};
+    // (made when first needed: a run that starts at an odd step is rare)
+    cudaGraphExec_t gexec_spec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [parity][length]
+    bool spec_pdl = true;  // the driver captures programmatic launches
     int per_sm_e = 1;      // pose-energy CTAs per SM
     int gridE = 0;       // pose-energy CTAs for all replicas
     int branches = 1;    // independent chains in the captured step loop
@@ -1358,7 +1363,7 @@ void split_branches(gcmc_ctx* ctx, int nb) {
 // if step j accepts nothing), and on a third S evaluates its pose energies
 // once P and F_e are done, on the SMs that A leaves free, stopping early when
 // A accepts a move.  F_p of step j + 1 waits for A and S.  One graph per
-// parity of the run's first step (kGraphSteps is even).
+// parity of the run's first step (the lengths are even) and length.
 // Launch of `kernel` on s as a programmatic dependent of the kernel before it in
 // s: it may be scheduled once every CTA of that kernel has triggered (pdl_trigger)
 // and waits in pdl_wait for that kernel's results, so its launch latency overlaps
@@ -1381,47 +1386,50 @@ cudaError_t launch_dependent(void (*kernel)(Args...), int grid, int block, size_
 
 // pdl: the step's completion pose-energy launch and accept kernel as programmatic
 // dependents of the kernels before them (F_p -> F_e -> accept).
-int build_spec_graph(gcmc_ctx* ctx, int parity, bool pdl) {
-    cudaStream_t sp = nullptr, ss = nullptr;
-    cudaEvent_t ev[4 * kGraphSteps + 1] = {};
+int build_spec_graph(gcmc_ctx* ctx, int parity, int length, bool pdl) {
+    cudaStream_t main = nullptr, sp = nullptr, ss = nullptr;
+    constexpr int N = kGraphSteps[0];
+    const int steps = kGraphSteps[length];
+    cudaEvent_t ev[4 * N + 1] = {};
     int st = GCMC_OK;
-    if (cudaStreamCreateWithFlags(&sp, cudaStreamNonBlocking) != cudaSuccess ||
+    if (cudaStreamCreateWithFlags(&main, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&sp, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&ss, cudaStreamNonBlocking) != cudaSuccess)
         st = GCMC_ERR_CUDA;
     for (auto& e : ev)
         if (st == GCMC_OK && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) st = GCMC_ERR_CUDA;
     cudaGraph_t graph = nullptr;
-    if (st == GCMC_OK && cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+    if (st == GCMC_OK && cudaStreamBeginCapture(main, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         st = GCMC_ERR_CUDA;
     if (st == GCMC_OK) {
         const int grid_s = std::max(1, ctx->gridE - ctx->per_sm_e);
         cudaEvent_t* evF = ev;                    // F_e of step j done
-        cudaEvent_t* evA = ev + kGraphSteps;      // A of step j done
-        cudaEvent_t* evP = ev + 2 * kGraphSteps;  // P of step j + 1 done
-        cudaEvent_t* evS = ev + 3 * kGraphSteps;  // S of step j + 1 done
-        cudaError_t e = cudaEventRecord(ev[4 * kGraphSteps], ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(sp, ev[4 * kGraphSteps], 0);
-        for (int i = 0; i < kGraphSteps && e == cudaSuccess; ++i) {
+        cudaEvent_t* evA = ev + N;                // A of step j done
+        cudaEvent_t* evP = ev + 2 * N;            // P of step j + 1 done
+        cudaEvent_t* evS = ev + 3 * N;            // S of step j + 1 done
+        cudaError_t e = cudaEventRecord(ev[4 * N], main);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(sp, ev[4 * N], 0);
+        for (int i = 0; i < steps && e == cudaSuccess; ++i) {
             const RepDev* cur = ((parity + i) & 1) ? ctx->d_reps_b : ctx->d_reps;
             const RepDev* nxt = ((parity + i) & 1) ? ctx->d_reps : ctx->d_reps_b;
-            if (i > 0) e = cudaStreamWaitEvent(ctx->stream, evS[i - 1], 0);
-            k_prep_spec<<<1, kAcceptThreads, prep_smem(ctx), ctx->stream>>>(cur, 1);
+            if (i > 0) e = cudaStreamWaitEvent(main, evS[i - 1], 0);
+            k_prep_spec<<<1, kAcceptThreads, prep_smem(ctx), main>>>(cur, 1);
             if (pdl && !ctx->tiled) {
                 if (e == cudaSuccess)
                     e = launch_dependent(energy_kernel(ctx->evar, -1, ctx->pme_any), ctx->gridE, kWarpsE * 32, 0,
-                                         ctx->stream, cur, 1, 2);
+                                         main, cur, 1, 2);
             } else {
-                launch_energy(ctx, cur, 1, 2, ctx->gridE, ctx->stream);
+                launch_energy(ctx, cur, 1, 2, ctx->gridE, main);
             }
-            if (e == cudaSuccess) e = cudaEventRecord(evF[i], ctx->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(evF[i], main);
             if (pdl) {  // (speculating: no Ewald)
                 if (e == cudaSuccess)
-                    e = launch_dependent(k_accept<false>, 1, kAcceptThreads, sizeof(AcceptSmem), ctx->stream, cur, 1,
+                    e = launch_dependent(k_accept<false>, 1, kAcceptThreads, sizeof(AcceptSmem), main, cur, 1,
                                          1);
             } else {
-                k_accept<false><<<1, kAcceptThreads, sizeof(AcceptSmem), ctx->stream>>>(cur, 1, 1);
+                k_accept<false><<<1, kAcceptThreads, sizeof(AcceptSmem), main>>>(cur, 1, 1);
             }
-            if (e == cudaSuccess) e = cudaEventRecord(evA[i], ctx->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(evA[i], main);
             if (i > 0 && e == cudaSuccess) e = cudaStreamWaitEvent(sp, evA[i - 1], 0);
             k_prep_spec<<<1, kAcceptThreads, prep_smem(ctx), sp>>>(nxt, 0);
             if (e == cudaSuccess) e = cudaEventRecord(evP[i], sp);
@@ -1430,17 +1438,18 @@ int build_spec_graph(gcmc_ctx* ctx, int parity, bool pdl) {
             launch_energy(ctx, nxt, 1, 1, grid_s, ss);
             if (e == cudaSuccess) e = cudaEventRecord(evS[i], ss);
         }
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, evS[kGraphSteps - 1], 0);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(main, evS[steps - 1], 0);
         if (e == cudaSuccess) e = cudaGetLastError();
-        cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
+        cudaError_t e2 = cudaStreamEndCapture(main, &graph);
         if (e != cudaSuccess || e2 != cudaSuccess) {
             std::fprintf(stderr, "gcmc_b200: graph capture failed: %s\n",
                          cudaGetErrorString(e != cudaSuccess ? e : e2));
             st = GCMC_ERR_CUDA;
         }
     }
-    if (st == GCMC_OK && cudaGraphInstantiate(&ctx->gexec_spec[parity], graph, 0) != cudaSuccess) st = GCMC_ERR_CUDA;
+    if (st == GCMC_OK && cudaGraphInstantiate(&ctx->gexec_spec[parity][length], graph, 0) != cudaSuccess) st = GCMC_ERR_CUDA;
     if (graph) cudaGraphDestroy(graph);
+    if (main) cudaStreamDestroy(main);
     if (sp) cudaStreamDestroy(sp);
     if (ss) cudaStreamDestroy(ss);
     for (auto& e : ev)
@@ -1449,31 +1458,33 @@ int build_spec_graph(gcmc_ctx* ctx, int parity, bool pdl) {
     return st;
 }
 
-int build_graph(gcmc_ctx* ctx) {
-    if (ctx->gexec) {
-        cudaGraphExecDestroy(ctx->gexec);
-        ctx->gexec = nullptr;
-    }
-    for (auto& g : ctx->gexec_spec)
-        if (g) {
-            cudaGraphExecDestroy(g);
-            g = nullptr;
-        }
-    if (ctx->spec) {
-        int st = build_spec_graph(ctx, 0, true);
-        if (st == GCMC_OK) st = build_spec_graph(ctx, 1, true);
-        if (st != GCMC_OK) {  // a driver that cannot capture programmatic launches: plain launches
-            for (auto& g : ctx->gexec_spec)
-                if (g) {
-                    cudaGraphExecDestroy(g);
-                    g = nullptr;
-                }
+// The speculating graph of this parity and length, captured if it is not there yet.
+int spec_graph(gcmc_ctx* ctx, int parity, int length, cudaGraphExec_t* out) {
+    cudaGraphExec_t& x = ctx->gexec_spec[parity][length];
+    if (!x) {
+        int st = build_spec_graph(ctx, parity, length, ctx->spec_pdl);
+        if (st != GCMC_OK && ctx->spec_pdl) {  // a driver that cannot capture programmatic launches: plain ones
             cudaGetLastError();
-            st = build_spec_graph(ctx, 0, false);
-            if (st == GCMC_OK) st = build_spec_graph(ctx, 1, false);
+            ctx->spec_pdl = false;
+            st = build_spec_graph(ctx, parity, length, false);
         }
-        return st;
+        if (st != GCMC_OK) return st;
     }
+    *out = x;
+    return GCMC_OK;
+}
+
+void destroy_graphs(gcmc_ctx* ctx) {
+    auto drop = [](cudaGraphExec_t& x) {
+        if (x) cudaGraphExecDestroy(x);
+        x = nullptr;
+    };
+    for (auto& x : ctx->gexec) drop(x);
+    for (auto& p : ctx->gexec_spec)
+        for (auto& x : p) drop(x);
+}
+
+int build_plain_graph(gcmc_ctx* ctx, int length) {
     const int nb = ctx->branches;
     std::vector<cudaStream_t> side(nb, nullptr);
     std::vector<cudaEvent_t> ev(nb, nullptr);
@@ -1497,7 +1508,7 @@ int build_graph(gcmc_ctx* ctx) {
             // the branch's atoms left them idle: 358 against 306 us per 64-replica step)
             const int grid = ctx->gridE;
             const int gridf = ctx->gridF;
-            for (int s = 0; s < kGraphSteps && e == cudaSuccess; ++s) {
+            for (int s = 0; s < kGraphSteps[length] && e == cudaSuccess; ++s) {
                 if (pme_update(ctx, r0, cnt, side[b]) != GCMC_OK) e = cudaErrorUnknown;
                 if (ctx->fb) {
                     fb_kernel(ctx)<<<gridf, kWarpsG * 32, 0, side[b]>>>(ctx->d_reps + r0, cnt, 1);
@@ -1520,7 +1531,7 @@ int build_graph(gcmc_ctx* ctx) {
             st = GCMC_ERR_CUDA;
         }
     }
-    if (st == GCMC_OK && cudaGraphInstantiate(&ctx->gexec, graph, 0) != cudaSuccess) st = GCMC_ERR_CUDA;
+    if (st == GCMC_OK && cudaGraphInstantiate(&ctx->gexec[length], graph, 0) != cudaSuccess) st = GCMC_ERR_CUDA;
     if (graph) cudaGraphDestroy(graph);
     for (int b = 1; b < nb; ++b)
         if (side[b]) cudaStreamDestroy(side[b]);
@@ -1530,12 +1541,33 @@ int build_graph(gcmc_ctx* ctx) {
     return st;
 }
 
+// The step loop's graphs, the old ones dropped.
+int build_graph(gcmc_ctx* ctx) {
+    destroy_graphs(ctx);
+    int st = GCMC_OK;
+    for (int length = 0; length < 2 && st == GCMC_OK; ++length) {
+        cudaGraphExec_t x;
+        st = ctx->spec ? spec_graph(ctx, 0, length, &x) : build_plain_graph(ctx, length);
+    }
+    return st;
+}
+
+// Graph launches for `need` steps: fn(0) the long graph, fn(1) the short one.
+template <class F>
+int launch_steps(int need, F fn) {
+    int st = GCMC_OK;
+    for (; need > 0 && st == GCMC_OK;) {
+        const int length = need > kGraphSteps[0] - kGraphSteps[1] ? 0 : 1;
+        st = fn(length);
+        need -= kGraphSteps[length];
+    }
+    return st;
+}
+
 int destroy_impl(gcmc_ctx* ctx) {
     if (!ctx) return GCMC_OK;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
-    for (auto g : ctx->gexec_spec)
-        if (g) cudaGraphExecDestroy(g);
+    destroy_graphs(ctx);
     for (auto& h : ctx->reps) free_rep(h);
     if (ctx->d_reps) cudaFree(ctx->d_reps);
     if (ctx->d_reps_b) cudaFree(ctx->d_reps_b);
@@ -1699,7 +1731,7 @@ int refill_impl(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins, const gcmc_
     const int fb = opt.proposal == 2 ? 1 : 0;
     const int evar = opt.energy_variant == 1 ? 1 : 0;
     const bool persist_before = ctx->persist;
-    const bool had_graph = ctx->gexec || ctx->gexec_spec[0];
+    const bool had_graph = ctx->gexec[0] || ctx->gexec_spec[0][0];
     const bool shape_changed = spec_changed || nb != ctx->branches || opt.energy_blocks_per_sm != ctx->ebps ||
                                fb != ctx->fb || evar != ctx->evar || ctx->tiled != tiled_before ||
                                ctx->pme_any != pme_before || pme_meshes(ctx) != mesh_before ||
@@ -2153,9 +2185,11 @@ int gcmc_run(gcmc_ctx* ctx, int32_t nsteps) {
     if (ctx->spec) {  // step `first` lives in descriptor copy first & 1
         k_spec_start<<<1, 32, 0, ctx->stream>>>((first & 1) ? ctx->d_reps_b : ctx->d_reps, first);
         CK(cudaGetLastError());
-        for (int done = 0; done < need; done += kGraphSteps)
-            CK(cudaGraphLaunch(ctx->gexec_spec[first & 1], ctx->stream));
-        return GCMC_OK;
+        return launch_steps(need, [&](int length) {
+            cudaGraphExec_t x;
+            const int st = spec_graph(ctx, first & 1, length, &x);
+            return st != GCMC_OK ? st : (cudaGraphLaunch(x, ctx->stream) == cudaSuccess ? GCMC_OK : GCMC_ERR_CUDA);
+        });
     }
     k_prepare<<<ctx->nrep, kAcceptThreads, prep_smem(ctx), ctx->stream>>>(ctx->d_reps, ctx->nrep);
     CK(cudaGetLastError());
@@ -2170,8 +2204,9 @@ int gcmc_run(gcmc_ctx* ctx, int32_t nsteps) {
                                        sizeof(AcceptSmem), ctx->stream));
         return GCMC_OK;
     }
-    for (int done = 0; done < need; done += kGraphSteps) CK(cudaGraphLaunch(ctx->gexec, ctx->stream));
-    return GCMC_OK;
+    return launch_steps(need, [&](int length) {
+        return cudaGraphLaunch(ctx->gexec[length], ctx->stream) == cudaSuccess ? GCMC_OK : GCMC_ERR_CUDA;
+    });
 }
 
 int gcmc_run_profiled(gcmc_ctx* ctx, int32_t nsteps, float* ms_energy, float* ms_accept, int32_t* move) {
