@@ -1231,13 +1231,14 @@ std::vector<int> pme_meshes(const gcmc_ctx* ctx) {
 // stream s, where they changed since the last update (the passes of pme.cuh; a
 // CTA that finds every mesh current returns at once).
 int pme_update(gcmc_ctx* ctx, int r0, int cnt, cudaStream_t s) {
-    size_t planes = 0, sm0 = 0, sm1 = 0, sm2 = 0;
+    size_t planes = 0, elems = 0, sm0 = 0, sm1 = 0, sm2 = 0;
     int nplane = 0, nrow = 0, nax0 = 0, nax1 = 0;
     for (int r = r0; r < r0 + cnt; ++r) {
         const RepHost& h = ctx->reps[r];
         if (!h.pme) continue;
         const int n0 = h.pme_n[0], n1 = h.pme_n[1], n2 = h.pme_n[2], M = n2 / 2 + 1;
         planes = std::max(planes, pme_plane_smem(n1, n2));
+        elems = std::max(elems, pme_plane_elems(n1, n2));
         sm0 = std::max(sm0, pme_axis_smem(n0));
         sm1 = std::max(sm1, pme_axis_smem(n1));
         sm2 = std::max(sm2, pme_rows_smem(n2));
@@ -1255,15 +1256,16 @@ int pme_update(gcmc_ctx* ctx, int r0, int cnt, cudaStream_t s) {
         return std::max(1, std::min(items, sms * per_sm));
     };
     const bool whole = planes <= (size_t)kPmeSmemMax;
+    const int pt = pme_plane_threads(elems);
     if (whole) {
-        k_pme_fwd_planes<<<grid(nplane, planes, kPlaneThreads), kPlaneThreads, planes, s>>>(reps, cnt);
+        k_pme_fwd_planes<<<grid(nplane, planes, pt), pt, planes, s>>>(reps, cnt);
     } else {
         k_pme_rows_r2c<<<grid(nrow, sm2, kAxisThreads), kAxisThreads, sm2, s>>>(reps, cnt);
         k_pme_axis<<<grid(nax1, sm1, kAxisThreads), kAxisThreads, sm1, s>>>(reps, cnt, 1, -1, 0);
     }
     k_pme_axis<<<grid(nax0, sm0, kAxisThreads), kAxisThreads, sm0, s>>>(reps, cnt, 0, 0, 1);
     if (whole) {
-        k_pme_inv_planes<<<grid(nplane, planes, kPlaneThreads), kPlaneThreads, planes, s>>>(reps, cnt);
+        k_pme_inv_planes<<<grid(nplane, planes, pt), pt, planes, s>>>(reps, cnt);
     } else {
         k_pme_axis<<<grid(nax1, sm1, kAxisThreads), kAxisThreads, sm1, s>>>(reps, cnt, 1, 1, 0);
         k_pme_rows_c2r<<<grid(nrow, sm2, kAxisThreads), kAxisThreads, sm2, s>>>(reps, cnt);

@@ -100,7 +100,11 @@ __device__ __forceinline__ double pme_phi_at(const RepDev& R, double x, double y
 // 8.1 + 7.6 + 9.3 us, against 68 us for six launches with a sincospi per
 // butterfly, radix 2 and 3 and a complex transform per real row; 4 replicas
 // of a 128 x 128 x 96 mesh 75 + 73 + 78 us, against 4 x 228 us.
-constexpr int kPlaneThreads = 512;
+// Threads of a plane's CTA: one CTA fills an SM's shared memory from about 128 x 64 on, so
+// large planes take more warps (16 replicas of 128 x 128 x 96: 926 -> 893 us a step with
+// 768 threads; a 64 x 64 plane is slower with them).
+constexpr int kPlaneThreads = 768;
+inline int pme_plane_threads(size_t elems) { return elems >= 4096 ? kPlaneThreads : 512; }
 constexpr int kAxisThreads = 256;
 constexpr int kAxisLines = 16;   // columns (256 bytes of each row) per axis item
 constexpr int kRowPairs = 8;     // row pairs per item of the separate row passes
