@@ -342,6 +342,16 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
                      const int32_t* d_self, int32_t nposes, const float* d_ff, const double* d_gout,
                      double* d_energy, double* d_gxyz, double* d_gq, double* d_gff, void* stream);
 
+/* Sites of rigid poses, x[p*nsites*3] = com_p + R(u_p) t_s, and the gradients of a
+ * function of them with respect to com[p*3] and u[p*4] (no counterpart in the
+ * reference).  u: unit quaternions (w, x, y, z); the template t[nsites*3] carries no
+ * gradient.  All arrays are DEVICE pointers, float (f64 = 0) or double (f64 = 1);
+ * launches on `stream` (a cudaStream_t) and returns without waiting. */
+int gcmc_rigid_sites(int32_t f64, const void* d_com, const void* d_unit, const void* d_template, int32_t nposes,
+                     int32_t nsites, void* d_sites, void* stream);
+int gcmc_rigid_sites_grad(int32_t f64, const void* d_unit, const void* d_template, const void* d_gsites,
+                          int32_t nposes, int32_t nsites, void* d_gcom, void* d_gunit, void* stream);
+
 /* Allocation-free variant of gcmc_energy_poses (no counterpart in the reference).
  *
  * For callers that cannot allocate GPU memory at the point where they need

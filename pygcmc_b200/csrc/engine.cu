@@ -190,6 +190,7 @@ struct gcmc_ctx {
     // (made when first needed: a run that starts at an odd step is rare)
     cudaGraphExec_t gexec_spec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [parity][length]
     bool spec_pdl = true;  // the driver captures programmatic launches
+    std::vector<cudaStream_t> side;  // side streams of the captures, made once
     int per_sm_e = 1;      // pose-energy CTAs per SM
     int gridE = 0;       // pose-energy CTAs for all replicas
     int branches = 1;    // independent chains in the captured step loop
@@ -210,7 +211,7 @@ struct gcmc_ctx {
     // tables in one block, the replicas' error words and fragment counts in one array each
     char* d_pack = nullptr;
     size_t d_pack_bytes = 0;
-    int* d_err = nullptr;  // [nrep]
+    int* d_err = nullptr;  // [nrep], behind d_small
     int* d_tot = nullptr;  // the replicas' totalNum, one after another
     size_t d_tot_cap = 0;
     int ntot = 0;
@@ -1388,16 +1389,27 @@ cudaError_t launch_dependent(void (*kernel)(Args...), int grid, int block, size_
 
 // pdl: the step's completion pose-energy launch and accept kernel as programmatic
 // dependents of the kernels before them (F_p -> F_e -> accept).
+// At least n side streams for captures.
+int side_streams(gcmc_ctx* ctx, int n) {
+    while ((int)ctx->side.size() < n) {
+        cudaStream_t s = nullptr;
+        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+            cudaGetLastError();
+            return GCMC_ERR_CUDA;
+        }
+        ctx->side.push_back(s);
+    }
+    return GCMC_OK;
+}
+
 int build_spec_graph(gcmc_ctx* ctx, int parity, int length, bool pdl) {
-    cudaStream_t main = nullptr, sp = nullptr, ss = nullptr;
     constexpr int N = kGraphSteps[0];
     const int steps = kGraphSteps[length];
     cudaEvent_t ev[4 * N + 1] = {};
-    int st = GCMC_OK;
-    if (cudaStreamCreateWithFlags(&main, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&sp, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&ss, cudaStreamNonBlocking) != cudaSuccess)
-        st = GCMC_ERR_CUDA;
+    // captured on side streams: a caller may be capturing the context's own
+    int st = side_streams(ctx, 3);
+    if (st != GCMC_OK) return st;
+    const cudaStream_t main = ctx->side[0], sp = ctx->side[1], ss = ctx->side[2];
     for (auto& e : ev)
         if (st == GCMC_OK && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) st = GCMC_ERR_CUDA;
     cudaGraph_t graph = nullptr;
@@ -1451,9 +1463,6 @@ int build_spec_graph(gcmc_ctx* ctx, int parity, int length, bool pdl) {
     }
     if (st == GCMC_OK && cudaGraphInstantiate(&ctx->gexec_spec[parity][length], graph, 0) != cudaSuccess) st = GCMC_ERR_CUDA;
     if (graph) cudaGraphDestroy(graph);
-    if (main) cudaStreamDestroy(main);
-    if (sp) cudaStreamDestroy(sp);
-    if (ss) cudaStreamDestroy(ss);
     for (auto& e : ev)
         if (e) cudaEventDestroy(e);
     if (st != GCMC_OK) cudaGetLastError();
@@ -1488,11 +1497,10 @@ void destroy_graphs(gcmc_ctx* ctx) {
 
 int build_plain_graph(gcmc_ctx* ctx, int length) {
     const int nb = ctx->branches;
-    std::vector<cudaStream_t> side(nb, nullptr);
     std::vector<cudaEvent_t> ev(nb, nullptr);
-    int st = GCMC_OK;
-    for (int b = 1; b < nb && st == GCMC_OK; ++b)
-        if (cudaStreamCreateWithFlags(&side[b], cudaStreamNonBlocking) != cudaSuccess) st = GCMC_ERR_CUDA;
+    int st = side_streams(ctx, nb);
+    if (st != GCMC_OK) return st;
+    std::vector<cudaStream_t> side(ctx->side.begin(), ctx->side.begin() + nb);
     for (int b = 0; b < nb && st == GCMC_OK; ++b)
         if (cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming) != cudaSuccess) st = GCMC_ERR_CUDA;
     cudaGraph_t graph = nullptr;
@@ -1535,8 +1543,6 @@ int build_plain_graph(gcmc_ctx* ctx, int length) {
     }
     if (st == GCMC_OK && cudaGraphInstantiate(&ctx->gexec[length], graph, 0) != cudaSuccess) st = GCMC_ERR_CUDA;
     if (graph) cudaGraphDestroy(graph);
-    for (int b = 1; b < nb; ++b)
-        if (side[b]) cudaStreamDestroy(side[b]);
     for (int b = 0; b < nb; ++b)
         if (ev[b]) cudaEventDestroy(ev[b]);
     if (st != GCMC_OK) cudaGetLastError();
@@ -1570,13 +1576,13 @@ int destroy_impl(gcmc_ctx* ctx) {
     if (!ctx) return GCMC_OK;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     destroy_graphs(ctx);
+    for (auto s : ctx->side) cudaStreamDestroy(s);
     for (auto& h : ctx->reps) free_rep(h);
     if (ctx->d_reps) cudaFree(ctx->d_reps);
     if (ctx->d_reps_b) cudaFree(ctx->d_reps_b);
     if (ctx->d_sync) cudaFree(ctx->d_sync);
     if (ctx->d_small) cudaFree(ctx->d_small);
     if (ctx->d_pack) cudaFree(ctx->d_pack);
-    if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->d_tot) cudaFree(ctx->d_tot);
     if (ctx->d_scratch) cudaFree(ctx->d_scratch);
     if (ctx->ev_ctx) cudaEventDestroy(ctx->ev_ctx);
@@ -1644,12 +1650,12 @@ int create_impl(int nrep, const gcmc_replica_in* ins, const gcmc_options* optp, 
         destroy_impl(ctx);
         return GCMC_ERR_CUDA;
     }
-    if (cudaMalloc(&ctx->d_small, kScratchSmall) != cudaSuccess ||
-        cudaMalloc(&ctx->d_err, sizeof(int) * nrep) != cudaSuccess) {
+    if (cudaMalloc(&ctx->d_small, kScratchSmall + sizeof(int) * nrep) != cudaSuccess) {
         cudaGetLastError();
         destroy_impl(ctx);
         return GCMC_ERR_CUDA;
     }
+    ctx->d_err = (int*)((char*)ctx->d_small + kScratchSmall);
     ctx->reps.resize(nrep);
     ctx->repdev.resize(nrep);
     for (int r = 0; r < nrep; ++r) ctx->reps[r].frag_atoms = frag_atoms[r];
@@ -2489,7 +2495,7 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
     const size_t o_lj = c.take(d_ff ? sizeof(float2) * ntab : 0);
     const size_t o_e = c.take(d_energy ? sizeof(double) * nposes * nslab : 0);
     const size_t o_ng = c.take(d_energy ? sizeof(int) * nposes * nslab : 0);
-    const size_t o_g = c.take(grads ? sizeof(float4) * nposes * nslab * nsites : 0);
+    const size_t o_g = c.take(grads ? sizeof(double4) * nposes * nslab * nsites : 0);
     const size_t o_glj = c.take(d_gff ? sizeof(double) * ntab * 2 : 0);
     // scratch: the context's, or for a large call or one that is being captured into a
     // graph (whose replays are not ordered against other calls) an allocation of its own.
@@ -2511,7 +2517,7 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
         RepDev R = ctx->repdev[rep];
         float2* lj = (float2*)(w + o_lj);
         double* glj = d_gff ? (double*)(w + o_glj) : nullptr;
-        float4* gpart = (float4*)(w + o_g);
+        double4* gpart = (double4*)(w + o_g);
         if (d_ff) {
             k_ff_to_lj<<<(int)((ntab + 255) / 256), 256, 0, s>>>(d_ff, lj, (int)ntab);
             R.lj = lj;
@@ -2543,6 +2549,40 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
     if (own && w) cudaFreeAsync(w, s);
     if (st == GCMC_OK) st = order_after(ctx, s);
     return st;
+}
+
+int gcmc_rigid_sites(int32_t f64, const void* d_com, const void* d_unit, const void* d_template, int32_t nposes,
+                     int32_t nsites, void* d_sites, void* stream) {
+    if (nposes < 0 || nsites < 1) return GCMC_ERR_ARG;
+    if (nposes == 0) return GCMC_OK;
+    if (!d_com || !d_unit || !d_template || !d_sites) return GCMC_ERR_ARG;
+    const unsigned grid = (unsigned)(((long long)nposes * nsites + 127) / 128);
+    if (f64)
+        k_rigid_sites<double><<<grid, 128, 0, (cudaStream_t)stream>>>(
+            (const double*)d_com, (const double*)d_unit, (const double*)d_template, nposes, nsites, (double*)d_sites);
+    else
+        k_rigid_sites<float><<<grid, 128, 0, (cudaStream_t)stream>>>(
+            (const float*)d_com, (const float*)d_unit, (const float*)d_template, nposes, nsites, (float*)d_sites);
+    CK(cudaGetLastError());
+    return GCMC_OK;
+}
+
+int gcmc_rigid_sites_grad(int32_t f64, const void* d_unit, const void* d_template, const void* d_gsites,
+                          int32_t nposes, int32_t nsites, void* d_gcom, void* d_gunit, void* stream) {
+    if (nposes < 0 || nsites < 1) return GCMC_ERR_ARG;
+    if (nposes == 0) return GCMC_OK;
+    if (!d_unit || !d_template || !d_gsites || !d_gcom || !d_gunit) return GCMC_ERR_ARG;
+    const unsigned grid = (unsigned)((nposes + 63) / 64);
+    if (f64)
+        k_rigid_sites_grad<double><<<grid, 64, 0, (cudaStream_t)stream>>>(
+            (const double*)d_unit, (const double*)d_template, (const double*)d_gsites, nposes, nsites, (double*)d_gcom,
+            (double*)d_gunit);
+    else
+        k_rigid_sites_grad<float><<<grid, 64, 0, (cudaStream_t)stream>>>(
+            (const float*)d_unit, (const float*)d_template, (const float*)d_gsites, nposes, nsites, (float*)d_gcom,
+            (float*)d_gunit);
+    CK(cudaGetLastError());
+    return GCMC_OK;
 }
 
 int gcmc_run_gcmc(const InfoStruct* info, AtomArray* fragmentInfo, residue* residueInfo, Atom* atomInfo,

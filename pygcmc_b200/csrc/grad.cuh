@@ -17,6 +17,8 @@
 // weighted by the caller's dL/dE of the pose, go to a per-block shared array
 // [ns][ffY][2] and from there to global FP64 sums.
 #pragma once
+#include <type_traits>
+
 #include "energy.cuh"
 
 namespace gcmc {
@@ -36,8 +38,11 @@ struct GradSinkT {
     float* gtab;   // block shared [ns][ffY][2] (nullptr: no table gradient)
     float w;       // dL/dE of the current pose
     int ffY;
-    float gx = 0.f, gy = 0.f, gz = 0.f, gq = 0.f;
-    float e = 0.f;  // WithE: this lane's FP32 sum of its pair energies
+    // this lane's sums: FP32 over the whole item for the force-bias kernel (WithE, with the pair
+    // energies in e); FP32 over a staged batch and FP64 over the batches for the gradients
+    using Sum = typename std::conditional<WithE, float, double>::type;
+    Sum gx = 0, gy = 0, gz = 0, gq = 0;
+    float e = 0.f;
 
     template <bool PairImage>
     __device__ __forceinline__ void flush_t(const RepDev& R, WarpBuf& B, int na, int ns, int lane) {
@@ -74,6 +79,8 @@ struct GradSinkT {
             }
             __syncwarp();
             if (active) {
+                float hx = WithE ? (float)gx : 0.f, hy = WithE ? (float)gy : 0.f, hz = WithE ? (float)gz : 0.f;
+                float hq = WithE ? (float)gq : 0.f;
                 for (int f = sub; f < m; f += nsub) {
                     const float4 a = st->a[f];
                     const int ta = st->t[f];
@@ -103,10 +110,10 @@ struct GradSinkT {
                     const float t6 = fmaf(2.0f * s6, s6, -s6);
                     const float G = -fmaf(3.0f * p.y, t6, 0.5f * gel) * ir2;
                     const float m2 = -2.0f * G;
-                    gx = fmaf(m2, dx, gx);  // dU/dx_s = -2 G (atom - site)
-                    gy = fmaf(m2, dy, gy);
-                    gz = fmaf(m2, dz, gz);
-                    gq = fmaf(kCoulomb * a.w, cq, gq);
+                    hx = fmaf(m2, dx, hx);  // dU/dx_s = -2 G (atom - site)
+                    hy = fmaf(m2, dy, hy);
+                    hz = fmaf(m2, dz, hz);
+                    hq = fmaf(kCoulomb * a.w, cq, hq);
                     if (WithE) e = fmaf(p.y, fmaf(s6, s6, -s6), e) + uel;
                     if (gtab) {
                         float* g = gtab + ((size_t)s * ffY + ta) * 2;
@@ -114,6 +121,10 @@ struct GradSinkT {
                         atomicAdd(g + 1, w * fmaf(s6, s6, -s6));
                     }
                 }
+                gx = WithE ? (Sum)hx : gx + (Sum)hx;
+                gy = WithE ? (Sum)hy : gy + (Sum)hy;
+                gz = WithE ? (Sum)hz : gz + (Sum)hz;
+                gq = WithE ? (Sum)hq : gq + (Sum)hq;
             }
             __syncwarp();
         }
@@ -126,13 +137,13 @@ struct GradSinkT {
 using GradSink = GradSinkT<false>;
 
 // item = (pose, slab) as in k_energy_explicit; part[(item * ns + s)] =
-// (dE/dx, dE/dy, dE/dz, dE/dq) of site s from this slab's atoms.
+// (dE/dx, dE/dy, dE/dz, dE/dq) of site s from this slab's atoms (FP64).
 // Dynamic shared memory: ns * ffY * 2 floats when glj != nullptr.
 __global__ void __launch_bounds__(kWarpsG * 32)
     k_energy_grad(const RepDev R, const float* __restrict__ xyz, const float* __restrict__ q,
                   const int* __restrict__ type, int ns, const float* __restrict__ centres,
                   const int* __restrict__ self, int nposes, int nslab, const double* __restrict__ gout,
-                  float4* __restrict__ part, double* __restrict__ glj) {
+                  double4* __restrict__ part, double* __restrict__ glj) {
     extern __shared__ float gtab[];
     __shared__ WarpBuf bufs[kWarpsG];
     __shared__ GradStage stages[kWarpsG];
@@ -163,17 +174,15 @@ __global__ void __launch_bounds__(kWarpsG * 32)
         walk_cells(R, B, ns, centres[3 * p], centres[3 * p + 1], centres[3 * p + 2], self ? self[p] : -1,
                    z, nwin, lane, sink, ng, npair, nullptr, 0, nslab);
         // sum the atom subsets of each site in a fixed order
-        stages[warp].red[lane] = make_float4(sink.gx, sink.gy, sink.gz, sink.gq);
-        __syncwarp();
-        if (lane < ns) {
-            const int nsub = 32 / ns;
-            float4 acc = stages[warp].red[lane];
-            for (int k = 1; k < nsub; ++k) {
-                const float4 v = stages[warp].red[k * ns + lane];
-                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-            }
-            part[(size_t)it * ns + lane] = acc;
+        double4 acc = make_double4(sink.gx, sink.gy, sink.gz, sink.gq);
+        for (int k = 1; k < 32 / ns; ++k) {
+            const int from = (k * ns + lane) & 31;
+            acc.x += __shfl_sync(kFull, sink.gx, from);
+            acc.y += __shfl_sync(kFull, sink.gy, from);
+            acc.z += __shfl_sync(kFull, sink.gz, from);
+            acc.w += __shfl_sync(kFull, sink.gq, from);
         }
+        if (lane < ns) part[(size_t)it * ns + lane] = acc;
         __syncwarp();
     }
     __syncthreads();
@@ -381,14 +390,14 @@ template __global__ void k_energy_fb<false>(const RepDev* __restrict__, int, int
 template __global__ void k_energy_fb<true>(const RepDev* __restrict__, int, int);
 
 // gxyz[p][s][3], gq[p][s] = the slabs' partial sums in slab order (FP64).
-__global__ void k_sum_grad(const float4* __restrict__ part, int nposes, int nslab, int ns,
+__global__ void k_sum_grad(const double4* __restrict__ part, int nposes, int nslab, int ns,
                            double* __restrict__ gxyz, double* __restrict__ gq) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;  // p * ns + s
     if (i >= nposes * ns) return;
     const int p = i / ns, s = i - p * ns;
     double x = 0.0, y = 0.0, zz = 0.0, w = 0.0;
     for (int z = 0; z < nslab; ++z) {
-        const float4 v = part[((size_t)p * nslab + z) * ns + s];
+        const double4 v = part[((size_t)p * nslab + z) * ns + s];
         x += v.x; y += v.y; zz += v.z; w += v.w;
     }
     if (gxyz) {
@@ -416,6 +425,79 @@ __global__ void k_glj_to_gff(const double* __restrict__ glj, const float* __rest
     if (i >= n) return;
     gff[2 * i] += glj[2 * i] * 200.0 * (double)ff[2 * i];
     gff[2 * i + 1] += glj[2 * i + 1] * 4.0;
+}
+
+// ---------------------------------------------------------------------------
+// Sites of rigid poses, x_{p,s} = com_p + R(u_p) t_s (u unit quaternions w, x, y,
+// z; t the centred template), and their gradients.  One launch each way in place
+// of some 30 elementwise launches forward and 70 backward, which cost the
+// differentiable energy of 61 poses more than its pose-energy kernels.
+// Every operation is rounded on its own, in the order of the tensor expression
+// (grad.py), and the rotation is the fused multiply-add chain over j = 0, 1, 2 of a
+// matrix product, so single precision gives the same sites bit for bit.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float r_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float r_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float r_sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float r_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double r_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double r_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double r_sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double r_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// A thread per site.
+template <typename T>
+__global__ void k_rigid_sites(const T* __restrict__ com, const T* __restrict__ u, const T* __restrict__ tpl,
+                              int nposes, int ns, T* __restrict__ out) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= (long long)nposes * ns) return;
+    const long long p = i / ns;
+    const int s = (int)(i - p * ns);
+    const T w = u[4 * p], x = u[4 * p + 1], y = u[4 * p + 2], z = u[4 * p + 3];
+    const T one = T(1), two = T(2);
+    const T R[9] = {r_sub(one, r_mul(two, r_add(r_mul(y, y), r_mul(z, z)))),
+                    r_mul(two, r_sub(r_mul(x, y), r_mul(w, z))),
+                    r_mul(two, r_add(r_mul(x, z), r_mul(w, y))),
+                    r_mul(two, r_add(r_mul(x, y), r_mul(w, z))),
+                    r_sub(one, r_mul(two, r_add(r_mul(x, x), r_mul(z, z)))),
+                    r_mul(two, r_sub(r_mul(y, z), r_mul(w, x))),
+                    r_mul(two, r_sub(r_mul(x, z), r_mul(w, y))),
+                    r_mul(two, r_add(r_mul(y, z), r_mul(w, x))),
+                    r_sub(one, r_mul(two, r_add(r_mul(x, x), r_mul(y, y))))};
+    const T t0 = tpl[3 * s], t1 = tpl[3 * s + 1], t2 = tpl[3 * s + 2];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        out[3 * i + c] =
+            r_add(com[3 * p + c], r_fma(R[3 * c + 2], t2, r_fma(R[3 * c + 1], t1, r_mul(R[3 * c], t0))));
+}
+
+// gcom_p = sum_s g_{p,s} and gu_p from the rotation's derivatives; a thread per pose,
+// sums in FP64.
+template <typename T>
+__global__ void k_rigid_sites_grad(const T* __restrict__ u, const T* __restrict__ tpl, const T* __restrict__ g,
+                                   int nposes, int ns, T* __restrict__ gcom, T* __restrict__ gu) {
+    const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (p >= nposes) return;
+    double c[3] = {0.0, 0.0, 0.0}, G[9] = {};
+    for (int s = 0; s < ns; ++s) {
+        const T* gs = g + (p * ns + s) * 3;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double v = (double)gs[i];
+            c[i] += v;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) G[3 * i + j] += v * (double)tpl[3 * s + j];
+        }
+    }
+    for (int i = 0; i < 3; ++i) gcom[3 * p + i] = (T)c[i];
+    const double w = u[4 * p], x = u[4 * p + 1], y = u[4 * p + 2], z = u[4 * p + 3];
+    gu[4 * p] = (T)(2.0 * (-z * G[1] + y * G[2] + z * G[3] - x * G[5] - y * G[6] + x * G[7]));
+    gu[4 * p + 1] =
+        (T)(2.0 * (y * G[1] + z * G[2] + y * G[3] - 2.0 * x * G[4] - w * G[5] + z * G[6] + w * G[7] - 2.0 * x * G[8]));
+    gu[4 * p + 2] =
+        (T)(2.0 * (-2.0 * y * G[0] + x * G[1] + w * G[2] + x * G[3] + z * G[5] - w * G[6] + z * G[7] - 2.0 * y * G[8]));
+    gu[4 * p + 3] =
+        (T)(2.0 * (-2.0 * z * G[0] - w * G[1] + x * G[2] + w * G[3] - 2.0 * z * G[4] + y * G[5] + x * G[6] + y * G[7]));
 }
 
 }  // namespace gcmc

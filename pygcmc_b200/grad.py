@@ -94,13 +94,76 @@ def pose_energy(engine, rep, xyz, q, ff, site_type, centres=None, self_res=None)
 def quat_to_matrix(q):
     """Rotation matrices [..., 3, 3] of quaternions q [..., 4] = (w, x, y, z),
     normalised first (so gradients are tangent to the unit sphere)."""
-    q = q / q.norm(dim=-1, keepdim=True)
+    return _unit_matrix(q / q.norm(dim=-1, keepdim=True))
+
+
+def _unit_matrix(q):
     w, x, y, z = q.unbind(-1)
     return torch.stack([
         torch.stack([1 - 2 * (y * y + z * z), 2 * (x * y - z * w), 2 * (x * z + y * w)], -1),
         torch.stack([2 * (x * y + z * w), 1 - 2 * (x * x + z * z), 2 * (y * z - x * w)], -1),
         torch.stack([2 * (x * z - y * w), 2 * (y * z + x * w), 1 - 2 * (x * x + y * y)], -1),
     ], -2)
+
+
+def _unit_sites(com, unit, tpl):
+    """Sites of unit quaternions as a tensor expression."""
+    return com[:, None, :] + torch.einsum("pij,sj->psi", _unit_matrix(unit), tpl)
+
+
+def _plain_cuda(com, quat, tpl):
+    """Whether :class:`RigidSites` may take these inputs: dense tensors of one floating type on
+    the current GPU, no broadcasting, no gradient of the template, and nothing that has to see the
+    tensor operations themselves (tracing or compiling, function transforms, forward-mode
+    differentiation, dispatch modes, autocast).  Fewer than 8 poses or one site keep the expression:
+    the library's product of such narrow matrices adds its three terms in another order, and the
+    single-precision sites would differ in the last bit (equal for all of 8 to 8192 poses tried)."""
+    return (type(com) in _TENSORS and type(quat) in _TENSORS and type(tpl) is torch.Tensor
+            and com.is_cuda and com.dtype in (torch.float32, torch.float64)
+            and quat.dtype == com.dtype and quat.device == com.device == tpl.device
+            and com.dim() == 2 and quat.dim() == 2 and com.shape == (quat.shape[0], 3) and quat.shape[1] == 4
+            and com.shape[0] >= 8 and tpl.shape[0] >= 2
+            and not tpl.requires_grad
+            and com.device.index == torch.cuda.current_device()
+            and not (torch.is_autocast_enabled() or torch.jit.is_tracing() or torch.compiler.is_compiling())
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and torch.autograd.forward_ad._current_level < 0
+            and torch.utils._python_dispatch._get_current_dispatch_mode() is None)
+
+
+_TENSORS = (torch.Tensor, torch.nn.Parameter)
+
+
+class RigidSites(torch.autograd.Function):
+    """x [P, ns, 3] = com + R(unit) t of unit quaternions [P, 4]: one kernel each way instead of the
+    tensor expression's hundred launches (whose operations it repeats, rounding by rounding).
+    Differentiated twice, its backward is the tensor expression's."""
+
+    @staticmethod
+    def forward(ctx, com, unit, tpl):
+        com_c, unit_c, tpl = com.contiguous(), unit.contiguous(), tpl.contiguous()
+        P, ns = unit.shape[0], tpl.shape[0]
+        out = torch.empty((P, ns, 3), dtype=com.dtype, device=com.device)
+        check(lib().gcmc_rigid_sites(int(com.dtype == torch.float64), _p(com_c), _p(unit_c), _p(tpl), P, ns, _p(out),
+                                     _stream()), "gcmc_rigid_sites")
+        ctx.save_for_backward(com, unit, tpl)
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        com, unit, tpl = ctx.saved_tensors
+        if torch.is_grad_enabled():  # create_graph: a differentiable backward
+            with torch.enable_grad():
+                c = com if com.requires_grad else com.detach().requires_grad_()
+                u = unit if unit.requires_grad else unit.detach().requires_grad_()
+                return (*torch.autograd.grad(_unit_sites(c, u, tpl), (c, u), g, create_graph=True), None)
+        g = g.contiguous()
+        unit_c = unit.contiguous()
+        P, ns = g.shape[0], g.shape[1]
+        gcom, gunit = torch.empty_like(com, memory_format=torch.contiguous_format), torch.empty_like(unit_c)
+        check(lib().gcmc_rigid_sites_grad(int(g.dtype == torch.float64), _p(unit_c), _p(tpl), _p(g), P, ns, _p(gcom),
+                                          _p(gunit), _stream()), "gcmc_rigid_sites_grad")
+        return gcom, gunit, None
 
 
 def lj_table(eps_kcal, rmin_half, n_rows: int):
@@ -128,8 +191,10 @@ class RigidFragment:
         self.site_type = t
 
     def sites(self, com, quat):
-        R = quat_to_matrix(quat)
-        return com[:, None, :] + torch.einsum("pij,sj->psi", R, self.template.to(com.dtype))
+        tpl = self.template.to(com.dtype)
+        if _plain_cuda(com, quat, tpl):
+            return RigidSites.apply(com, quat / quat.norm(dim=-1, keepdim=True), tpl)
+        return com[:, None, :] + torch.einsum("pij,sj->psi", quat_to_matrix(quat), tpl)
 
     def energy(self, com, quat, ff, charges=None):
         q = self.charges if charges is None else charges

@@ -1,0 +1,88 @@
+"""The fused rigid-site kernels against the tensor expression they stand for (needs a B200).
+
+Forward: every operation is rounded alike and a matrix product's three terms are a fused
+multiply-add chain, so the sites agree to the last bit or, should the library's product order its
+terms differently, to a rounding of the largest term: 4 eps (|com| + |t|).  Backward: sums of ns
+products, FP64 inside: ns eps of the sum of |terms| plus the expression's own rounding, 64 eps of
+that sum in all.  Inputs that the fused path does not take, and second derivatives, follow the
+expression.
+"""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(P, ns, dtype, seed=0):
+    g = torch.Generator().manual_seed(seed + 31 * P + ns)
+    com = 60 * torch.rand((P, 3), generator=g, dtype=torch.float64)
+    quat = torch.randn((P, 4), generator=g, dtype=torch.float64)
+    tpl = 2 * torch.randn((ns, 3), generator=g, dtype=torch.float64)
+    w = torch.randn((P, ns, 3), generator=g, dtype=torch.float64)
+    return [t.to("cuda", dtype) for t in (com, quat, tpl, w)]
+
+
+class Frag:
+    def __init__(self, tpl):
+        self.template = tpl
+
+
+def fused(com, quat, tpl):
+    from pygcmc_b200.grad import RigidFragment
+    return RigidFragment.sites(Frag(tpl), com, quat)
+
+
+def expression(com, quat, tpl):
+    from pygcmc_b200.grad import quat_to_matrix
+    return com[:, None, :] + torch.einsum("pij,sj->psi", quat_to_matrix(quat), tpl)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("P,ns", [(1, 1), (7, 3), (8, 2), (61, 3), (63, 20), (64, 4), (65, 12), (1000, 7), (4096, 5)])
+def test_sites_and_gradients(P, ns, dtype):
+    com, quat, tpl, w = inputs(P, ns, dtype)
+    eps = torch.finfo(dtype).eps
+    c, q = com.clone().requires_grad_(), quat.clone().requires_grad_()
+    x = fused(c, q, tpl)
+    assert (type(x.grad_fn).__name__ == "RigidSitesBackward") == (P >= 8 and ns >= 2)
+    ref = expression(com, quat, tpl)
+    bound = 4 * eps * (com.abs().amax() + tpl.abs().amax())
+    assert (x - ref).abs().max() <= bound
+    (x * w).sum().backward()
+    c2, q2 = (t.double().clone().requires_grad_() for t in (com, quat))
+    (expression(c2, q2, tpl.double()) * w.double()).sum().backward()
+    l1c = w.double().abs().sum(1)
+    l1q = (w.double().abs().sum(2) @ tpl.double().abs().sum(1, keepdim=True)) * 8 / quat.double().norm(dim=1)[:, None]
+    assert ((c.grad.double() - c2.grad).abs() <= 64 * eps * l1c).all()
+    assert ((q.grad.double() - q2.grad).abs() <= 64 * eps * l1q).all()
+
+
+def test_forms_outside_the_fused_path():
+    com, quat, tpl, w = inputs(33, 6, torch.float64)
+    ref = expression(com, quat, tpl)
+    # strided inputs (fused), one quaternion for all poses, mixed types, a differentiable template, the CPU
+    buf = torch.zeros((33, 8), device="cuda", dtype=torch.float64)
+    buf[:, ::2] = quat
+    assert torch.allclose(fused(com.t().contiguous().t(), buf[:, ::2], tpl), ref, rtol=0, atol=1e-13)
+    assert torch.allclose(fused(com, quat[:1], tpl), expression(com, quat[:1], tpl), rtol=0, atol=1e-13)
+    t = tpl.clone().requires_grad_()
+    fused(com, quat, t).sum().backward()
+    assert t.grad is not None
+    assert torch.allclose(fused(com.cpu(), quat.cpu(), tpl.cpu()).cuda(), ref, rtol=0, atol=1e-13)
+    assert fused(com[:0], quat[:0], tpl).shape == (0, 6, 3)
+    # function transforms and forward mode
+    one = torch.func.vmap(lambda c, q: expression(c[None], q[None], tpl)[0])(com, quat)
+    assert torch.allclose(torch.func.vmap(lambda c, q: fused(c[None], q[None], tpl)[0])(com, quat), one, rtol=0,
+                          atol=1e-13)
+    _, jv = torch.func.jvp(lambda q: fused(com, q, tpl), (quat,), (quat + 1,))
+    _, jr = torch.func.jvp(lambda q: expression(com, q, tpl), (quat,), (quat + 1,))
+    assert torch.allclose(jv, jr, rtol=1e-12, atol=1e-12)
+    # second derivatives
+    q = quat.clone().requires_grad_()
+    for f in (fused, expression):
+        (g,) = torch.autograd.grad((f(com, q, tpl) * w).sum(), q, create_graph=True)
+        (h,) = torch.autograd.grad((g * g).sum(), q)
+        if f is fused:
+            first = h
+    assert torch.allclose(first, h, rtol=1e-10, atol=1e-10)
