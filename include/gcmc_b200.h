@@ -352,6 +352,17 @@ int gcmc_rigid_sites(int32_t f64, const void* d_com, const void* d_unit, const v
 int gcmc_rigid_sites_grad(int32_t f64, const void* d_unit, const void* d_template, const void* d_gsites,
                           int32_t nposes, int32_t nsites, void* d_gcom, void* d_gunit, void* stream);
 
+/* The pair table (sigma [nm], eps [kJ/mol]) [rows * n * 2] of per-type CHARMM
+ * parameters eps[n] [kcal/mol] and rmin/2 rmin[n] [A], the first `rows` types being
+ * the table's rows (Lorentz-Berthelot combining, gcmc/python/simulation.py:64-72),
+ * and the gradients of a function of it with respect to both (no counterpart in the
+ * reference).  DEVICE pointers, float (f64 = 0) or double (f64 = 1); launches on
+ * `stream` and returns without waiting.  1 <= rows <= n <= 32768. */
+int gcmc_lj_pairs(int32_t f64, const void* d_eps, const void* d_rmin, int32_t n, int32_t rows, void* d_out,
+                  void* stream);
+int gcmc_lj_pairs_grad(int32_t f64, const void* d_eps, const void* d_gout, int32_t n, int32_t rows, void* d_geps,
+                       void* d_grmin, void* stream);
+
 /* Allocation-free variant of gcmc_energy_poses (no counterpart in the reference).
  *
  * For callers that cannot allocate GPU memory at the point where they need

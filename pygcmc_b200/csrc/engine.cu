@@ -2083,6 +2083,12 @@ int device_scratch(gcmc_ctx* ctx, size_t bytes, char** out) {
     return GCMC_OK;
 }
 
+// The numbers of the pair table's expression, rounded as it rounds them.
+template <typename T>
+LjScale<T> lj_scale() {
+    return {T(1) / (T)std::pow(2.0, 1.0 / 6.0), T(1) / T(10), (T)kKcalToKJ};
+}
+
 // Consecutive pieces of a scratch block, 256-byte aligned.
 struct Carver {
     size_t at = 0;
@@ -2645,6 +2651,34 @@ int gcmc_rigid_sites_grad(int32_t f64, const void* d_unit, const void* d_templat
         k_rigid_sites_grad<float><<<grid, 64, 0, (cudaStream_t)stream>>>(
             (const float*)d_unit, (const float*)d_template, (const float*)d_gsites, nposes, nsites, (float*)d_gcom,
             (float*)d_gunit);
+    CK(cudaGetLastError());
+    return GCMC_OK;
+}
+
+int gcmc_lj_pairs(int32_t f64, const void* d_eps, const void* d_rmin, int32_t n, int32_t rows, void* d_out,
+                  void* stream) {
+    if (!d_eps || !d_rmin || !d_out || rows < 1 || rows > n || n > 32768) return GCMC_ERR_ARG;
+    const unsigned grid = (unsigned)((rows * (long long)n + 127) / 128);
+    if (f64)
+        k_lj_pairs<double><<<grid, 128, 0, (cudaStream_t)stream>>>((const double*)d_eps, (const double*)d_rmin, n, rows,
+                                                                   lj_scale<double>(), (double*)d_out);
+    else
+        k_lj_pairs<float><<<grid, 128, 0, (cudaStream_t)stream>>>((const float*)d_eps, (const float*)d_rmin, n, rows,
+                                                                  lj_scale<float>(), (float*)d_out);
+    CK(cudaGetLastError());
+    return GCMC_OK;
+}
+
+int gcmc_lj_pairs_grad(int32_t f64, const void* d_eps, const void* d_gout, int32_t n, int32_t rows, void* d_geps,
+                       void* d_grmin, void* stream) {
+    if (!d_eps || !d_gout || !d_geps || !d_grmin || rows < 1 || rows > n || n > 32768) return GCMC_ERR_ARG;
+    const unsigned grid = (unsigned)((n + 3) / 4);
+    if (f64)
+        k_lj_pairs_grad<double><<<grid, 128, 0, (cudaStream_t)stream>>>(
+            (const double*)d_eps, (const double*)d_gout, n, rows, lj_scale<double>(), (double*)d_geps, (double*)d_grmin);
+    else
+        k_lj_pairs_grad<float><<<grid, 128, 0, (cudaStream_t)stream>>>(
+            (const float*)d_eps, (const float*)d_gout, n, rows, lj_scale<float>(), (float*)d_geps, (float*)d_grmin);
     CK(cudaGetLastError());
     return GCMC_OK;
 }

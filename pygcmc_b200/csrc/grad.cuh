@@ -500,4 +500,56 @@ __global__ void k_rigid_sites_grad(const T* __restrict__ u, const T* __restrict_
         (T)(2.0 * (-2.0 * z * G[0] - w * G[1] + x * G[2] + w * G[3] - 2.0 * z * G[4] + y * G[5] + x * G[6] + y * G[7]));
 }
 
+// ---------------------------------------------------------------------------
+// The pair table of per-type CHARMM parameters, (sigma, eps) per (row, column):
+//   sigma_i = 2 rmin_i / 2^(1/6) / 10,  e_i = c eps_i,
+//   out[i][j] = ((sigma_i + sigma_j) / 2, sqrt(e_i e_j)),
+// and its gradients; a launch each way in place of some 35 (bound by the host's launches:
+// the gradients of 4096 poses with a 23 x 24 table 950 -> 635 us a pass).  As with the rigid
+// sites every operation is rounded on its own in the tensor expression's order
+// (a division by a number is a product with its rounded reciprocal there).
+// ---------------------------------------------------------------------------
+template <typename T>
+struct LjScale {
+    T inv_root, inv_ten, c;
+    __device__ __forceinline__ T sigma(T rmin) const { return r_mul(r_mul(r_mul(T(2), rmin), inv_root), inv_ten); }
+};
+__device__ __forceinline__ float r_sqrt(float a) { return __fsqrt_rn(a); }
+__device__ __forceinline__ double r_sqrt(double a) { return __dsqrt_rn(a); }
+
+template <typename T>
+__global__ void k_lj_pairs(const T* __restrict__ eps, const T* __restrict__ rmin, int n, int rows, LjScale<T> k,
+                           T* __restrict__ out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= rows * n) return;
+    const int i = t / n, j = t - i * n;
+    out[2 * t] = r_mul(r_add(k.sigma(rmin[i]), k.sigma(rmin[j])), T(0.5));
+    out[2 * t + 1] = r_sqrt(r_mul(r_mul(k.c, eps[i]), r_mul(k.c, eps[j])));
+}
+
+// A warp per type: the table's row (if it has one) and column, sums in FP64.
+template <typename T>
+__global__ void k_lj_pairs_grad(const T* __restrict__ eps, const T* __restrict__ g, int n, int rows, LjScale<T> k,
+                                T* __restrict__ geps, T* __restrict__ grmin) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const double ei = (double)k.c * (double)eps[i];
+    double ds = 0.0, de = 0.0;
+    auto add = [&](int a, int b, int other) {  // entry (a, b), whose other type is `other`
+        const T* v = g + 2 * ((size_t)a * n + b);
+        const double eo = (double)k.c * (double)eps[other];
+        ds += 0.5 * (double)v[0];
+        de += (double)v[1] / (2.0 * sqrt(ei * eo)) * eo;
+    };
+    if (i < rows)
+        for (int j = lane; j < n; j += 32) add(i, j, j);
+    for (int r = lane; r < rows; r += 32) add(r, i, r);
+    ds = warp_sum(ds);
+    de = warp_sum(de);
+    if (lane == 0) {
+        grmin[i] = (T)(2.0 * (double)k.inv_root * (double)k.inv_ten * ds);
+        geps[i] = (T)((double)k.c * de);
+    }
+}
+
 }  // namespace gcmc

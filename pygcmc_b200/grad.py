@@ -118,13 +118,17 @@ def _plain_cuda(com, quat, tpl):
     differentiation, dispatch modes, autocast).  Fewer than 8 poses or one site keep the expression:
     the library's product of such narrow matrices adds its three terms in another order, and the
     single-precision sites would differ in the last bit (equal for all of 8 to 8192 poses tried)."""
-    return (type(com) in _TENSORS and type(quat) in _TENSORS and type(tpl) is torch.Tensor
-            and com.is_cuda and com.dtype in (torch.float32, torch.float64)
-            and quat.dtype == com.dtype and quat.device == com.device == tpl.device
+    return (_plain(com, quat) and type(tpl) is torch.Tensor and tpl.device == com.device
             and com.dim() == 2 and quat.dim() == 2 and com.shape == (quat.shape[0], 3) and quat.shape[1] == 4
             and com.shape[0] >= 8 and tpl.shape[0] >= 2
-            and not tpl.requires_grad
-            and com.device.index == torch.cuda.current_device()
+            and not tpl.requires_grad)
+
+
+def _plain(a, b):
+    """Two dense tensors of one floating type on the current GPU, and nothing that has to see the
+    tensor operations on them."""
+    return (type(a) in _TENSORS and type(b) in _TENSORS and a.is_cuda and a.dtype in (torch.float32, torch.float64)
+            and b.dtype == a.dtype and b.device == a.device and a.device.index == torch.cuda.current_device()
             and not (torch.is_autocast_enabled() or torch.jit.is_tracing() or torch.compiler.is_compiling())
             and torch._C._functorch.peek_interpreter_stack() is None
             and torch.autograd.forward_ad._current_level < 0
@@ -153,10 +157,9 @@ class RigidSites(torch.autograd.Function):
     def backward(ctx, g):
         com, unit, tpl = ctx.saved_tensors
         if torch.is_grad_enabled():  # create_graph: a differentiable backward
-            with torch.enable_grad():
-                c = com if com.requires_grad else com.detach().requires_grad_()
-                u = unit if unit.requires_grad else unit.detach().requires_grad_()
-                return (*torch.autograd.grad(_unit_sites(c, u, tpl), (c, u), g, create_graph=True), None)
+            c = com if com.requires_grad else com.detach().requires_grad_()
+            u = unit if unit.requires_grad else unit.detach().requires_grad_()
+            return (*torch.autograd.grad(_unit_sites(c, u, tpl), (c, u), g, create_graph=True), None)
         g = g.contiguous()
         unit_c = unit.contiguous()
         P, ns = g.shape[0], g.shape[1]
@@ -171,11 +174,48 @@ def lj_table(eps_kcal, rmin_half, n_rows: int):
     CHARMM eps [kcal/mol] and rmin/2 [A] (n types, the first n_rows being the
     fragment site types): sigma = 2 rmin/2 / 2^(1/6) / 10, eps_kJ = 4.184 eps,
     Lorentz-Berthelot combining (gcmc/python/simulation.py:64-72)."""
+    if _plain(eps_kcal, rmin_half) and eps_kcal.dim() == 1 and eps_kcal.shape == rmin_half.shape \
+            and 1 <= n_rows <= eps_kcal.shape[0] <= 32768:
+        return LJPairs.apply(eps_kcal, rmin_half, int(n_rows))
+    return _lj_expression(eps_kcal, rmin_half, n_rows)
+
+
+def _lj_expression(eps_kcal, rmin_half, n_rows):
     sigma = 2.0 * rmin_half / 2.0 ** (1.0 / 6.0) / 10.0
     e = V.KCAL_TO_KJ * eps_kcal
     s2 = (sigma[:n_rows, None] + sigma[None, :]) / 2
     e2 = torch.sqrt(e[:n_rows, None] * e[None, :])
     return torch.stack([s2, e2], -1).reshape(-1)
+
+
+class LJPairs(torch.autograd.Function):
+    """The table of :func:`lj_table` by one kernel each way (the tensor expression's operations,
+    rounding by rounding: equal for every table of 1 to 59 types tried, both precisions), in place
+    of some 35 launches: 950 -> 635 us a pass of 4096 poses with gradients; differentiated twice, its backward is the expression's."""
+
+    @staticmethod
+    def forward(ctx, eps, rmin, rows):
+        e, r = eps.contiguous(), rmin.contiguous()
+        n = e.shape[0]
+        out = torch.empty(rows * n * 2, dtype=e.dtype, device=e.device)
+        check(lib().gcmc_lj_pairs(int(e.dtype == torch.float64), _p(e), _p(r), n, rows, _p(out), _stream()),
+              "gcmc_lj_pairs")
+        ctx.save_for_backward(eps, rmin)
+        ctx.rows = rows
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        eps, rmin = ctx.saved_tensors
+        if torch.is_grad_enabled():  # create_graph: a differentiable backward
+            e = eps if eps.requires_grad else eps.detach().requires_grad_()
+            r = rmin if rmin.requires_grad else rmin.detach().requires_grad_()
+            return (*torch.autograd.grad(_lj_expression(e, r, ctx.rows), (e, r), g, create_graph=True), None)
+        e, g = eps.contiguous(), g.contiguous()
+        geps, grmin = torch.empty_like(e), torch.empty_like(e)
+        check(lib().gcmc_lj_pairs_grad(int(e.dtype == torch.float64), _p(e), _p(g), e.shape[0], ctx.rows, _p(geps),
+                                       _p(grmin), _stream()), "gcmc_lj_pairs_grad")
+        return geps, grmin, None
 
 
 class RigidFragment:

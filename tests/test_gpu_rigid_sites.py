@@ -1,4 +1,4 @@
-"""The fused rigid-site kernels against the tensor expression they stand for (needs a B200).
+"""The fused rigid-site and pair-table kernels against the tensor expressions they stand for (needs a B200).
 
 Forward: every operation is rounded alike and a matrix product's three terms are a fused
 multiply-add chain, so the sites agree to the last bit or, should the library's product order its
@@ -86,3 +86,38 @@ def test_forms_outside_the_fused_path():
         if f is fused:
             first = h
     assert torch.allclose(first, h, rtol=1e-10, atol=1e-10)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n,rows", [(1, 1), (2, 1), (24, 23), (31, 31), (33, 32), (70, 40)])
+def test_pair_table(n, rows, dtype):
+    """Values: the same roundings, so equal to the last bit or at most one of them (4 eps); gradients:
+    sums of at most n + rows terms, 64 eps of the sum of |terms|."""
+    from pygcmc_b200.grad import _lj_expression, lj_table
+    g = torch.Generator().manual_seed(n)
+    eps = (0.02 + 0.18 * torch.rand(n, generator=g, dtype=torch.float64)).to("cuda", dtype)
+    rmin = (1.0 + 1.2 * torch.rand(n, generator=g, dtype=torch.float64)).to("cuda", dtype)
+    w = torch.randn(rows * n * 2, generator=g, dtype=torch.float64).to("cuda", dtype)
+    e, r = eps.clone().requires_grad_(), rmin.clone().requires_grad_()
+    out = lj_table(e, r, rows)
+    assert type(out.grad_fn).__name__ == "LJPairsBackward"
+    u = torch.finfo(dtype).eps
+    ref = _lj_expression(eps, rmin, rows)
+    assert ((out - ref).abs() <= 4 * u * ref.abs()).all()
+    (out * w).sum().backward()
+    want = []
+    for weights in (w.double(), w.double().abs()):  # the gradients, and the sums of |terms|
+        e2, r2 = (t.detach().double().clone().requires_grad_() for t in (eps, rmin))
+        (_lj_expression(e2, r2, rows) * weights).sum().backward()
+        want.append((e2.grad, r2.grad))
+    for got, exact, scale in zip((e.grad, r.grad), *want):
+        assert ((got.double() - exact).abs() <= 64 * u * scale).all()
+    # another type of the parameters, and second derivatives, follow the expression
+    assert torch.allclose(lj_table(eps.double(), rmin.float(), rows).double(), ref.double(), rtol=1e-6)
+    e3 = eps.clone().requires_grad_()
+    hs = []
+    for f in (lj_table, _lj_expression):
+        (d,) = torch.autograd.grad((f(e3, rmin, rows) * w).sum(), e3, create_graph=True)
+        (h,) = torch.autograd.grad((d * d).sum(), e3)
+        hs.append(h)
+    assert torch.allclose(*hs, rtol=1e-3 if dtype == torch.float32 else 1e-10)
