@@ -343,14 +343,22 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
                      double* d_energy, double* d_gxyz, double* d_gq, double* d_gff, void* stream);
 
 /* Sites of rigid poses, x[p*nsites*3] = com_p + R(u_p) t_s, and the gradients of a
- * function of them with respect to com[p*3] and u[p*4] (no counterpart in the
- * reference).  u: unit quaternions (w, x, y, z); the template t[nsites*3] carries no
- * gradient.  All arrays are DEVICE pointers, float (f64 = 0) or double (f64 = 1);
+ * function of them with respect to com[p*3] and the quaternions before their
+ * normalisation, q[p*4] = norm[p] u[p*4] (no counterpart in the reference).  u: unit
+ * quaternions (w, x, y, z); the template t[nsites*3] carries no gradient.  All arrays are DEVICE pointers, float (f64 = 0) or double (f64 = 1);
  * launches on `stream` (a cudaStream_t) and returns without waiting. */
 int gcmc_rigid_sites(int32_t f64, const void* d_com, const void* d_unit, const void* d_template, int32_t nposes,
                      int32_t nsites, void* d_sites, void* stream);
-int gcmc_rigid_sites_grad(int32_t f64, const void* d_unit, const void* d_template, const void* d_gsites,
-                          int32_t nposes, int32_t nsites, void* d_gcom, void* d_gunit, void* stream);
+int gcmc_rigid_sites_grad(int32_t f64, const void* d_unit, const void* d_norm, const void* d_template,
+                          const void* d_gsites, int32_t nposes, int32_t nsites, void* d_gcom, void* d_gquat,
+                          void* stream);
+
+/* The chain rule behind gcmc_energy_grad's outputs for a function with dL/dE[p] =
+ * d_weight[p]: d_ox[p*nsites*3] = d_gxyz * weight, d_oq[nsites] = sum over poses of
+ * d_gq * weight, d_off[nff] = d_gff as float (no counterpart in the reference).  A null
+ * output is left out.  DEVICE pointers; launches on `stream` and returns without waiting. */
+int gcmc_pose_chain(const double* d_weight, const double* d_gxyz, const double* d_gq, const double* d_gff,
+                    int32_t nposes, int32_t nsites, int32_t nff, float* d_ox, float* d_oq, float* d_off, void* stream);
 
 /* The pair table (sigma [nm], eps [kJ/mol]) [rows * n * 2] of per-type CHARMM
  * parameters eps[n] [kcal/mol] and rmin/2 rmin[n] [A], the first `rows` types being

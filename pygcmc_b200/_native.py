@@ -83,7 +83,8 @@ def lib():
         "gcmc_energy_total": (c_int, [c_void, c_int, P(ctypes.c_double)]),
         "gcmc_energy_grad": (c_int, [c_void, c_int] + [c_void] * 4 + [c_int, c_void, c_void, c_int] + [c_void] * 7),
         "gcmc_rigid_sites": (c_int, [c_int, c_void, c_void, c_void, c_int, c_int, c_void, c_void]),
-        "gcmc_rigid_sites_grad": (c_int, [c_int, c_void, c_void, c_void, c_int, c_int, c_void, c_void, c_void]),
+        "gcmc_rigid_sites_grad": (c_int, [c_int, c_void, c_void, c_void, c_void, c_int, c_int, c_void, c_void, c_void]),
+        "gcmc_pose_chain": (c_int, [c_void, c_void, c_void, c_void, c_int, c_int, c_int, c_void, c_void, c_void, c_void]),
         "gcmc_lj_pairs": (c_int, [c_int, c_void, c_void, c_int, c_int, c_void, c_void]),
         "gcmc_lj_pairs_grad": (c_int, [c_int, c_void, c_void, c_int, c_int, c_void, c_void, c_void]),
         "gcmc_run_batch": (c_int, [c_int, c_void, P(Options)]),
@@ -149,6 +150,6 @@ EXPORTS = ["runGCMC_cuda", "gcmc_run_gcmc", "gcmc_run_batch", "gcmc_energy_grad"
            "gcmc_energy_total", "gcmc_autotune", "gcmc_release_cache", "gcmc_last_status", "gcmc_status_string", "gcmc_default_options",
            "gcmc_create", "gcmc_run", "gcmc_run_profiled", "gcmc_sync", "gcmc_download", "gcmc_get_logs", "gcmc_counters",
            "gcmc_device_error", "gcmc_phase_cycles", "gcmc_stream", "gcmc_destroy", "gcmc_energy_poses",
-           "gcmc_energy_poses_noalloc", "gcmc_rigid_sites", "gcmc_rigid_sites_grad", "gcmc_lj_pairs",
-           "gcmc_lj_pairs_grad", "gcmc_synth_place", "gcmc_synth_chain_sphere",
+           "gcmc_energy_poses_noalloc", "gcmc_rigid_sites", "gcmc_rigid_sites_grad", "gcmc_pose_chain",
+           "gcmc_lj_pairs", "gcmc_lj_pairs_grad", "gcmc_synth_place", "gcmc_synth_chain_sphere",
            "gcmc_synth_chain_slab"]

@@ -2637,20 +2637,35 @@ int gcmc_rigid_sites(int32_t f64, const void* d_com, const void* d_unit, const v
     return GCMC_OK;
 }
 
-int gcmc_rigid_sites_grad(int32_t f64, const void* d_unit, const void* d_template, const void* d_gsites,
-                          int32_t nposes, int32_t nsites, void* d_gcom, void* d_gunit, void* stream) {
+int gcmc_rigid_sites_grad(int32_t f64, const void* d_unit, const void* d_norm, const void* d_template,
+                          const void* d_gsites, int32_t nposes, int32_t nsites, void* d_gcom, void* d_gquat,
+                          void* stream) {
     if (nposes < 0 || nsites < 1) return GCMC_ERR_ARG;
     if (nposes == 0) return GCMC_OK;
-    if (!d_unit || !d_template || !d_gsites || !d_gcom || !d_gunit) return GCMC_ERR_ARG;
+    if (!d_unit || !d_norm || !d_template || !d_gsites || !d_gcom || !d_gquat) return GCMC_ERR_ARG;
     const unsigned grid = (unsigned)((nposes + 63) / 64);
     if (f64)
         k_rigid_sites_grad<double><<<grid, 64, 0, (cudaStream_t)stream>>>(
-            (const double*)d_unit, (const double*)d_template, (const double*)d_gsites, nposes, nsites, (double*)d_gcom,
-            (double*)d_gunit);
+            (const double*)d_unit, (const double*)d_norm, (const double*)d_template, (const double*)d_gsites, nposes, nsites, (double*)d_gcom,
+            (double*)d_gquat);
     else
         k_rigid_sites_grad<float><<<grid, 64, 0, (cudaStream_t)stream>>>(
-            (const float*)d_unit, (const float*)d_template, (const float*)d_gsites, nposes, nsites, (float*)d_gcom,
-            (float*)d_gunit);
+            (const float*)d_unit, (const float*)d_norm, (const float*)d_template, (const float*)d_gsites, nposes, nsites, (float*)d_gcom,
+            (float*)d_gquat);
+    CK(cudaGetLastError());
+    return GCMC_OK;
+}
+
+int gcmc_pose_chain(const double* d_weight, const double* d_gxyz, const double* d_gq, const double* d_gff,
+                    int32_t nposes, int32_t nsites, int32_t nff, float* d_ox, float* d_oq, float* d_off, void* stream) {
+    if (nposes < 0 || nsites < 1 || nff < 0) return GCMC_ERR_ARG;
+    const long long n3 = 3LL * nposes * nsites, nx = d_ox ? (n3 + kChainThreads - 1) / kChainThreads : 0;
+    const int nq = d_oq ? nsites : 0, nf = d_off ? (nff + kChainThreads - 1) / kChainThreads : 0;
+    if ((nposes && (!d_weight || (d_ox && !d_gxyz) || (d_oq && !d_gq))) || (nf && !d_gff)) return GCMC_ERR_ARG;
+    if (nx + nq + nf == 0) return GCMC_OK;
+    if (nx + nq + nf > INT32_MAX) return GCMC_ERR_ARG;
+    k_pose_chain<<<(unsigned)(nx + nq + nf), kChainThreads, 0, (cudaStream_t)stream>>>(
+        ChainArgs{d_weight, d_gxyz, d_gq, d_gff, d_ox, d_oq, d_off, n3, nposes, nsites, nff, (int)nx, nq});
     CK(cudaGetLastError());
     return GCMC_OK;
 }

@@ -36,6 +36,12 @@ def _stream():
     return ctypes.c_void_p(h if h else 1)
 
 
+# Up to this many poses the gradients' chain rule is one kernel (k_pose_chain), whose sum over the
+# poses is one block per site.  8 sites, us by the kernel and by the six tensor operations: 64 poses
+# 26 and 60, 16384 22 and 61, 65536 33 and 45; beyond, the operations' split reduction is the faster.
+CHAIN_POSES = 65536
+
+
 class PoseEnergy(torch.autograd.Function):
     """E[p] (float64) of poses ``xyz`` [P, ns, 3] float32 with charges ``q`` [ns]
     float32 and pair table ``ff`` [ffX*ffY*2] float32 (all CUDA); ``centres``
@@ -71,6 +77,12 @@ class PoseEnergy(torch.autograd.Function):
                                          ctx.site_type.ctypes.data_as(ctypes.c_void_p), ns, _p(centres),
                                          _p(ctx.self_res), P, _p(ff), _p(gE), None, _p(gxyz), _p(gq), _p(gff),
                                          _stream()), "gcmc_energy_grad")
+        if P <= CHAIN_POSES:
+            gx, gqs, gf = (torch.empty(shape, dtype=torch.float32, device=xyz.device) if need else None
+                           for need, shape in ((need_x, (P, ns, 3)), (need_q, (ns,)), (need_ff, ff.shape)))
+            check(lib().gcmc_pose_chain(_p(gE), _p(gxyz), _p(gq), _p(gff), P, ns, ff.shape[0], _p(gx), _p(gqs),
+                                        _p(gf), _stream()), "gcmc_pose_chain")
+            return gx, gqs, gf, None, None, None, None, None, None
         gx = (gxyz * gE[:, None, None]).to(xyz.dtype) if need_x else None
         gqs = (gq * gE[:, None]).sum(0).to(q.dtype) if need_q else None
         gf = gff.to(ff.dtype) if need_ff else None
@@ -106,9 +118,8 @@ def _unit_matrix(q):
     ], -2)
 
 
-def _unit_sites(com, unit, tpl):
-    """Sites of unit quaternions as a tensor expression."""
-    return com[:, None, :] + torch.einsum("pij,sj->psi", _unit_matrix(unit), tpl)
+def _sites_expression(com, quat, tpl):
+    return com[:, None, :] + torch.einsum("pij,sj->psi", quat_to_matrix(quat), tpl)
 
 
 def _plain_cuda(com, quat, tpl):
@@ -139,34 +150,34 @@ _TENSORS = (torch.Tensor, torch.nn.Parameter)
 
 
 class RigidSites(torch.autograd.Function):
-    """x [P, ns, 3] = com + R(unit) t of unit quaternions [P, 4]: one kernel each way instead of the
+    """x [P, ns, 3] = com + R(quat / |quat|) t: one kernel each way instead of the
     tensor expression's hundred launches (whose operations it repeats, rounding by rounding).
     Differentiated twice, its backward is the tensor expression's."""
 
     @staticmethod
-    def forward(ctx, com, unit, tpl):
-        com_c, unit_c, tpl = com.contiguous(), unit.contiguous(), tpl.contiguous()
+    def forward(ctx, com, quat, tpl):
+        norm = quat.norm(dim=-1, keepdim=True)
+        com_c, unit, tpl = com.contiguous(), (quat / norm).contiguous(), tpl.contiguous()
         P, ns = unit.shape[0], tpl.shape[0]
         out = torch.empty((P, ns, 3), dtype=com.dtype, device=com.device)
-        check(lib().gcmc_rigid_sites(int(com.dtype == torch.float64), _p(com_c), _p(unit_c), _p(tpl), P, ns, _p(out),
+        check(lib().gcmc_rigid_sites(int(com.dtype == torch.float64), _p(com_c), _p(unit), _p(tpl), P, ns, _p(out),
                                      _stream()), "gcmc_rigid_sites")
-        ctx.save_for_backward(com, unit, tpl)
+        ctx.save_for_backward(quat, tpl, unit, norm)  # (no gradient needs com, which may change)
         return out
 
     @staticmethod
     def backward(ctx, g):
-        com, unit, tpl = ctx.saved_tensors
+        quat, tpl, unit, norm = ctx.saved_tensors
         if torch.is_grad_enabled():  # create_graph: a differentiable backward
-            c = com if com.requires_grad else com.detach().requires_grad_()
-            u = unit if unit.requires_grad else unit.detach().requires_grad_()
-            return (*torch.autograd.grad(_unit_sites(c, u, tpl), (c, u), g, create_graph=True), None)
+            c = torch.zeros_like(quat[:, :3], requires_grad=True)
+            q = quat if quat.requires_grad else quat.detach().requires_grad_()
+            return (*torch.autograd.grad(_sites_expression(c, q, tpl), (c, q), g, create_graph=True), None)
         g = g.contiguous()
-        unit_c = unit.contiguous()
         P, ns = g.shape[0], g.shape[1]
-        gcom, gunit = torch.empty_like(com, memory_format=torch.contiguous_format), torch.empty_like(unit_c)
-        check(lib().gcmc_rigid_sites_grad(int(g.dtype == torch.float64), _p(unit_c), _p(tpl), _p(g), P, ns, _p(gcom),
-                                          _p(gunit), _stream()), "gcmc_rigid_sites_grad")
-        return gcom, gunit, None
+        gcom, gquat = unit.new_empty((P, 3)), torch.empty_like(unit)
+        check(lib().gcmc_rigid_sites_grad(int(g.dtype == torch.float64), _p(unit), _p(norm), _p(tpl), _p(g), P, ns,
+                                          _p(gcom), _p(gquat), _stream()), "gcmc_rigid_sites_grad")
+        return gcom, gquat, None
 
 
 def lj_table(eps_kcal, rmin_half, n_rows: int):
@@ -176,7 +187,8 @@ def lj_table(eps_kcal, rmin_half, n_rows: int):
     Lorentz-Berthelot combining (gcmc/python/simulation.py:64-72)."""
     if _plain(eps_kcal, rmin_half) and eps_kcal.dim() == 1 and eps_kcal.shape == rmin_half.shape \
             and 1 <= n_rows <= eps_kcal.shape[0] <= 32768:
-        return LJPairs.apply(eps_kcal, rmin_half, int(n_rows))
+        # (a copy to save: the caller may change eps between the passes, as with the expression)
+        return LJPairs.apply(eps_kcal.clone(), rmin_half, int(n_rows))
     return _lj_expression(eps_kcal, rmin_half, n_rows)
 
 
@@ -200,16 +212,16 @@ class LJPairs(torch.autograd.Function):
         out = torch.empty(rows * n * 2, dtype=e.dtype, device=e.device)
         check(lib().gcmc_lj_pairs(int(e.dtype == torch.float64), _p(e), _p(r), n, rows, _p(out), _stream()),
               "gcmc_lj_pairs")
-        ctx.save_for_backward(eps, rmin)
+        ctx.save_for_backward(eps)  # (the table is linear in rmin)
         ctx.rows = rows
         return out
 
     @staticmethod
     def backward(ctx, g):
-        eps, rmin = ctx.saved_tensors
+        (eps,) = ctx.saved_tensors
         if torch.is_grad_enabled():  # create_graph: a differentiable backward
             e = eps if eps.requires_grad else eps.detach().requires_grad_()
-            r = rmin if rmin.requires_grad else rmin.detach().requires_grad_()
+            r = torch.zeros_like(eps, requires_grad=True)
             return (*torch.autograd.grad(_lj_expression(e, r, ctx.rows), (e, r), g, create_graph=True), None)
         e, g = eps.contiguous(), g.contiguous()
         geps, grmin = torch.empty_like(e), torch.empty_like(e)
@@ -233,8 +245,8 @@ class RigidFragment:
     def sites(self, com, quat):
         tpl = self.template.to(com.dtype)
         if _plain_cuda(com, quat, tpl):
-            return RigidSites.apply(com, quat / quat.norm(dim=-1, keepdim=True), tpl)
-        return com[:, None, :] + torch.einsum("pij,sj->psi", quat_to_matrix(quat), tpl)
+            return RigidSites.apply(com, quat, tpl)
+        return _sites_expression(com, quat, tpl)
 
     def energy(self, com, quat, ff, charges=None):
         q = self.charges if charges is None else charges

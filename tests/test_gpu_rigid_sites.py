@@ -121,3 +121,46 @@ def test_pair_table(n, rows, dtype):
         (h,) = torch.autograd.grad((d * d).sum(), e3)
         hs.append(h)
     assert torch.allclose(*hs, rtol=1e-3 if dtype == torch.float32 else 1e-10)
+
+
+@pytest.mark.parametrize("P,ns,nff", [(1, 1, 2), (0, 3, 0), (85, 3, 7), (86, 1, 256), (255, 20, 257), (4097, 5, 1104)])
+def test_chain_rule_of_pose_gradients(P, ns, nff):
+    """Products and conversions are single roundings (equal); the sum over the poses in FP64 and one
+    rounding to FP32: 2^-24 of the sum and P 2^-53 of the sum of |terms|."""
+    import ctypes
+    from pygcmc_b200._native import check, lib
+    g = torch.Generator().manual_seed(P + ns)
+    w, gx, gq, gff = (torch.randn(s, generator=g, dtype=torch.float64).cuda() for s in ((P,), (P, ns, 3), (P, ns), (nff,)))
+    out = [torch.full(s, 7.0, device="cuda") for s in ((P, ns, 3), (ns,), (nff,))]
+
+    def p(t):
+        return ctypes.c_void_p(t.data_ptr())
+    stream = ctypes.c_void_p(1)
+    check(lib().gcmc_pose_chain(p(w), p(gx), p(gq), p(gff), P, ns, nff, *map(p, out), stream), "gcmc_pose_chain")
+    want = (gq * w[:, None]).sum(0)
+    assert torch.equal(out[0], (gx * w[:, None, None]).float())
+    assert torch.equal(out[2], gff.float())
+    assert ((out[1].double() - want).abs() <= 2.0 ** -23 * want.abs() + P * 2.0 ** -52 * (gq * w[:, None]).abs().sum(0)).all()
+    kept = out[1].clone()  # the charges' sum alone, again: the same bits
+    out[1].zero_()
+    check(lib().gcmc_pose_chain(p(w), None, p(gq), None, P, ns, 0, None, p(out[1]), None, stream), "gcmc_pose_chain")
+    assert torch.equal(out[1], kept)
+
+
+def test_inputs_may_change_before_the_backward():
+    """Centres and the table's parameters are not needed by any gradient as they stand: in-place updates
+    between the two passes are allowed, as with the expressions."""
+    from pygcmc_b200.grad import _lj_expression, lj_table
+    com, quat, tpl, w = inputs(40, 5, torch.float64)
+    eps, rmin = com[:, 0].abs() + 0.1, quat[:, 0].abs() + 1
+    got = []
+    for sites, table in ((fused, lj_table), (expression, _lj_expression)):
+        c, q, e, r = (t.clone().requires_grad_() for t in (com, quat, eps, rmin))
+        out = (sites(c, q, tpl) * w).sum() + (table(e, r, 7) ** 2).sum()
+        with torch.no_grad():
+            for t in (c, e, r):
+                t += 1
+        out.backward()
+        got.append((c.grad, q.grad, e.grad, r.grad))
+    for a, b in zip(*got):
+        assert torch.allclose(a, b, rtol=1e-11, atol=1e-11)
