@@ -132,7 +132,7 @@ def _plain_cuda(com, quat, tpl):
     return (_plain(com, quat) and type(tpl) is torch.Tensor and tpl.device == com.device
             and com.dim() == 2 and quat.dim() == 2 and com.shape == (quat.shape[0], 3) and quat.shape[1] == 4
             and com.shape[0] >= 8 and tpl.shape[0] >= 2
-            and not tpl.requires_grad)
+            and not (tpl.requires_grad or tpl.is_neg()))
 
 
 def _plain(a, b):
@@ -140,6 +140,7 @@ def _plain(a, b):
     tensor operations on them."""
     return (type(a) in _TENSORS and type(b) in _TENSORS and a.is_cuda and a.dtype in (torch.float32, torch.float64)
             and b.dtype == a.dtype and b.device == a.device and a.device.index == torch.cuda.current_device()
+            and not (a.is_neg() or b.is_neg())
             and not (torch.is_autocast_enabled() or torch.jit.is_tracing() or torch.compiler.is_compiling())
             and torch._C._functorch.peek_interpreter_stack() is None
             and torch.autograd.forward_ad._current_level < 0
@@ -147,6 +148,18 @@ def _plain(a, b):
 
 
 _TENSORS = (torch.Tensor, torch.nn.Parameter)
+
+
+def _expression_backward(g):
+    """Whether a backward pass has to be the tensor expression's: it is to be differentiated
+    (create_graph), or runs for a batch of gradients at once (is_grads_batched, vmap)."""
+    return torch.is_grad_enabled() or not torch._C._has_storage(g)
+
+
+def _grad_of(expression, inputs, g):
+    again = torch.is_grad_enabled()
+    with torch.enable_grad():
+        return torch.autograd.grad(expression(), inputs, g, create_graph=again)
 
 
 class RigidSites(torch.autograd.Function):
@@ -168,11 +181,11 @@ class RigidSites(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         quat, tpl, unit, norm = ctx.saved_tensors
-        if torch.is_grad_enabled():  # create_graph: a differentiable backward
+        if _expression_backward(g):
             c = torch.zeros_like(quat[:, :3], requires_grad=True)
             q = quat if quat.requires_grad else quat.detach().requires_grad_()
-            return (*torch.autograd.grad(_sites_expression(c, q, tpl), (c, q), g, create_graph=True), None)
-        g = g.contiguous()
+            return (*_grad_of(lambda: _sites_expression(c, q, tpl), (c, q), g), None)
+        g = g.resolve_neg().contiguous()
         P, ns = g.shape[0], g.shape[1]
         gcom, gquat = unit.new_empty((P, 3)), torch.empty_like(unit)
         check(lib().gcmc_rigid_sites_grad(int(g.dtype == torch.float64), _p(unit), _p(norm), _p(tpl), _p(g), P, ns,
@@ -185,8 +198,8 @@ def lj_table(eps_kcal, rmin_half, n_rows: int):
     CHARMM eps [kcal/mol] and rmin/2 [A] (n types, the first n_rows being the
     fragment site types): sigma = 2 rmin/2 / 2^(1/6) / 10, eps_kJ = 4.184 eps,
     Lorentz-Berthelot combining (gcmc/python/simulation.py:64-72)."""
-    if _plain(eps_kcal, rmin_half) and eps_kcal.dim() == 1 and eps_kcal.shape == rmin_half.shape \
-            and 1 <= n_rows <= eps_kcal.shape[0] <= 32768:
+    if isinstance(n_rows, (int, np.integer)) and _plain(eps_kcal, rmin_half) and eps_kcal.dim() == 1 \
+            and eps_kcal.shape == rmin_half.shape and 1 <= n_rows <= eps_kcal.shape[0] <= 32768:
         # (a copy to save: the caller may change eps between the passes, as with the expression)
         return LJPairs.apply(eps_kcal.clone(), rmin_half, int(n_rows))
     return _lj_expression(eps_kcal, rmin_half, n_rows)
@@ -219,11 +232,11 @@ class LJPairs(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (eps,) = ctx.saved_tensors
-        if torch.is_grad_enabled():  # create_graph: a differentiable backward
+        if _expression_backward(g):
             e = eps if eps.requires_grad else eps.detach().requires_grad_()
             r = torch.zeros_like(eps, requires_grad=True)
-            return (*torch.autograd.grad(_lj_expression(e, r, ctx.rows), (e, r), g, create_graph=True), None)
-        e, g = eps.contiguous(), g.contiguous()
+            return (*_grad_of(lambda: _lj_expression(e, r, ctx.rows), (e, r), g), None)
+        e, g = eps.contiguous(), g.resolve_neg().contiguous()
         geps, grmin = torch.empty_like(e), torch.empty_like(e)
         check(lib().gcmc_lj_pairs_grad(int(e.dtype == torch.float64), _p(e), _p(g), e.shape[0], ctx.rows, _p(geps),
                                        _p(grmin), _stream()), "gcmc_lj_pairs_grad")

@@ -71,6 +71,14 @@ def test_forms_outside_the_fused_path():
     assert t.grad is not None
     assert torch.allclose(fused(com.cpu(), quat.cpu(), tpl.cpu()).cuda(), ref, rtol=0, atol=1e-13)
     assert fused(com[:0], quat[:0], tpl).shape == (0, 6, 3)
+    assert torch.allclose(fused(torch._neg_view(-com), quat, tpl), ref, rtol=0, atol=1e-13)
+    # the table: the rows given as None (all of them) or as a float (refused)
+    from pygcmc_b200.grad import _lj_expression, lj_table
+    e, r = quat[:, 0].abs(), quat[:, 1].abs()
+    assert torch.equal(lj_table(e, r, None), _lj_expression(e, r, None))
+    assert torch.equal(lj_table(torch._neg_view(-e), r, 5), _lj_expression(e, r, 5))
+    with pytest.raises(TypeError):
+        lj_table(e, r, 5.0)
     # function transforms and forward mode
     one = torch.func.vmap(lambda c, q: expression(c[None], q[None], tpl)[0])(com, quat)
     assert torch.allclose(torch.func.vmap(lambda c, q: fused(c[None], q[None], tpl)[0])(com, quat), one, rtol=0,
@@ -162,5 +170,21 @@ def test_inputs_may_change_before_the_backward():
                 t += 1
         out.backward()
         got.append((c.grad, q.grad, e.grad, r.grad))
+    for a, b in zip(*got):
+        assert torch.allclose(a, b, rtol=1e-11, atol=1e-11)
+
+
+def test_batched_gradients():
+    """Several output gradients at once (is_grads_batched) give what the expressions give."""
+    from pygcmc_b200.grad import _lj_expression, lj_table
+    com, quat, tpl, w = inputs(12, 4, torch.float64)
+    eps, rmin = com[:, 0].abs() + 0.1, quat[:, 0].abs() + 1
+    got = []
+    for sites, table in ((fused, lj_table), (expression, _lj_expression)):
+        c, q, e, r = (t.clone().requires_grad_() for t in (com, quat, eps, rmin))
+        x, y = sites(c, q, tpl), table(e, r, 7)
+        many = torch.stack([w, 2 * w, w.flip(0)])
+        got.append(torch.autograd.grad(x, (c, q), many, is_grads_batched=True)
+                   + torch.autograd.grad(y, (e, r), many.reshape(3, -1)[:, :1].expand(3, y.numel()), is_grads_batched=True))
     for a, b in zip(*got):
         assert torch.allclose(a, b, rtol=1e-11, atol=1e-11)
