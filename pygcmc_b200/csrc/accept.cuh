@@ -1017,7 +1017,6 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
             *R.energy = et;
         }
         R.counters[0] += 1ull;
-        if (S.misc[0] == 0) R.counters[14] += 1ull;  // steps that accepted nothing
         R.counters[1] += (unsigned long long)(k * D.nvar);
         if (logging) {
             gcmc_step_log L;

@@ -1839,93 +1839,6 @@ int download_moved(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins) {
     return GCMC_OK;
 }
 
-// Advance every replica by nsteps steps (asynchronous).  spec: by the speculating graphs
-// (a speculating context's only; its steps may also run one after another, in the first
-// descriptor copy).
-int run_steps(gcmc_ctx* ctx, int nsteps, bool spec) {
-    if (nsteps <= 0) return GCMC_OK;
-    const int first = ctx->reps[0].host_end;
-    int need = 0;
-    for (auto& h : ctx->reps) {
-        long long e = std::min<long long>((long long)h.host_end + nsteps, h.mcsteps);
-        need = std::max(need, (int)(e - h.host_end));
-        h.host_end = (int)e;
-    }
-    if (need == 0) return GCMC_OK;
-    k_set_run_end<<<(ctx->nrep + 127) / 128, 128, 0, ctx->stream>>>(ctx->d_reps, ctx->nrep, nsteps);
-    if (spec) {  // step `first` lives in descriptor copy first & 1
-        k_spec_start<<<1, 32, 0, ctx->stream>>>((first & 1) ? ctx->d_reps_b : ctx->d_reps, first);
-        CK(cudaGetLastError());
-        return launch_steps(need, [&](int length) {
-            cudaGraphExec_t x;
-            const int st = spec_graph(ctx, first & 1, length, &x);
-            return st != GCMC_OK ? st : (cudaGraphLaunch(x, ctx->stream) == cudaSuccess ? GCMC_OK : GCMC_ERR_CUDA);
-        });
-    }
-    if (ctx->spec) {
-        for (int length = 0; length < 2; ++length)
-            if (!ctx->gexec[length]) {
-                const int st = build_plain_graph(ctx, length);
-                if (st != GCMC_OK) return st;
-            }
-        k_prepare_at<<<1, kAcceptThreads, prep_smem(ctx), ctx->stream>>>(ctx->d_reps, first);
-    } else {
-        k_prepare<<<ctx->nrep, kAcceptThreads, prep_smem(ctx), ctx->stream>>>(ctx->d_reps, ctx->nrep);
-    }
-    CK(cudaGetLastError());
-    if (ctx->persist) {  // the whole step range in one cooperative launch
-        CK(cudaMemsetAsync(ctx->d_sync, 0, sizeof(GridSync), ctx->stream));
-        const RepDev* reps = ctx->d_reps;
-        int nrep = ctx->nrep, nst = need;
-        GridSync* gs = ctx->d_sync;
-        long long cap = ctx->spin_cap;
-        void* args[] = {(void*)&reps, (void*)&nrep, (void*)&nst, (void*)&gs, (void*)&cap};
-        CK(cudaLaunchCooperativeKernel((const void*)k_persist, dim3(ctx->grid_persist), dim3(kPersistThreads), args,
-                                       sizeof(AcceptSmem), ctx->stream));
-        return GCMC_OK;
-    }
-    return launch_steps(need, [&](int length) {
-        return cudaGraphLaunch(ctx->gexec[length], ctx->stream) == cudaSuccess ? GCMC_OK : GCMC_ERR_CUDA;
-    });
-}
-
-// A run whose caller waits for it (the drop-in's), in a speculating context: in chunks of
-// kGraphSteps[0] steps, each speculating or not by what the last finished one did.  The
-// two loops give the same chain.  A step's speculation is lost when the step before it
-// accepts a move, and then costs about 7 us (its launches, and the wait for it to drain);
-// when it stands it saves the pose energies' time beside the accept kernel.  Measured,
-// speculating against not, us per step: 2000-atom protein, most steps accepting, 41 / 33;
-// 800 waters 52 / 49; 6000-atom protein at the start, a third of the steps accepting
-// nothing, 40 / 37, half of them 30.7 / 30.3, two thirds 29 / 34.  So from 11 in 20 on; the
-// first chunks, of which nothing is known, do not.
-int run_adaptive(gcmc_ctx* ctx, int nsteps) {
-    StagingLease staging;
-    unsigned long long* const stat = (unsigned long long*)staging.get(2 * 16 * sizeof(unsigned long long));
-    const cudaEvent_t done[2] = {ctx->ev_ctx, ctx->ev_call};
-    staging.pending = ctx->stream;
-    unsigned long long steps = 0, quiet = 0;
-    bool spec = false;
-    for (int i = 0, left = nsteps; left > 0; ++i) {
-        if (i >= 2) {  // (one chunk stays queued while the host waits)
-            CK(cudaEventSynchronize(done[i & 1]));
-            const unsigned long long *c = stat + 16 * (i & 1), ds = c[0] - steps, dq = c[14] - quiet;
-            steps = c[0];
-            quiet = c[14];
-            if (ds > 0) spec = 20 * dq >= 11 * ds;
-        }
-        const int n = std::min(left, kGraphSteps[0]);
-        const int st = run_steps(ctx, n, spec);
-        if (st != GCMC_OK) return st;
-        left -= n;
-        CK(cudaMemcpyAsync(stat + 16 * (i & 1), ctx->reps[0].counters, 16 * sizeof(unsigned long long),
-                           cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaEventRecord(done[i & 1], ctx->stream));
-    }
-    CK(cudaStreamSynchronize(ctx->stream));  // (the staging is leased until here)
-    staging.pending = nullptr;
-    return GCMC_OK;
-}
-
 // Refill *slot (or create it) for these inputs, run every replica's mcsteps
 // steps and download the results in place.  Called under g_cache_mutex.
 int cached_run(gcmc_ctx** slot, int nrep, const gcmc_replica_in* ins, const gcmc_options* opt) {
@@ -1964,7 +1877,7 @@ int cached_run(gcmc_ctx** slot, int nrep, const gcmc_replica_in* ins, const gcmc
     const double t1 = trace ? now_ms() : 0.0;
     int most = 0;
     for (int r = 0; r < nrep; ++r) most = std::max(most, (int)ins[r].info->mcsteps);
-    st = (*slot)->spec ? run_adaptive(*slot, most) : gcmc_run(*slot, most);
+    st = gcmc_run(*slot, most);
     if (st == GCMC_OK) st = gcmc_sync(*slot);
     const double t2 = trace ? now_ms() : 0.0;
     if (st == GCMC_OK) st = download_moved(*slot, nrep, ins);
@@ -2282,7 +2195,41 @@ void* gcmc_stream(gcmc_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
 int gcmc_run(gcmc_ctx* ctx, int32_t nsteps) {
     if (!ctx) return GCMC_ERR_ARG;
-    return run_steps(ctx, nsteps, ctx->spec);
+    if (nsteps <= 0) return GCMC_OK;
+    const int first = ctx->reps[0].host_end;
+    int need = 0;
+    for (auto& h : ctx->reps) {
+        long long e = std::min<long long>((long long)h.host_end + nsteps, h.mcsteps);
+        need = std::max(need, (int)(e - h.host_end));
+        h.host_end = (int)e;
+    }
+    if (need == 0) return GCMC_OK;
+    k_set_run_end<<<(ctx->nrep + 127) / 128, 128, 0, ctx->stream>>>(ctx->d_reps, ctx->nrep, nsteps);
+    if (ctx->spec) {  // step `first` lives in descriptor copy first & 1
+        k_spec_start<<<1, 32, 0, ctx->stream>>>((first & 1) ? ctx->d_reps_b : ctx->d_reps, first);
+        CK(cudaGetLastError());
+        return launch_steps(need, [&](int length) {
+            cudaGraphExec_t x;
+            const int st = spec_graph(ctx, first & 1, length, &x);
+            return st != GCMC_OK ? st : (cudaGraphLaunch(x, ctx->stream) == cudaSuccess ? GCMC_OK : GCMC_ERR_CUDA);
+        });
+    }
+    k_prepare<<<ctx->nrep, kAcceptThreads, prep_smem(ctx), ctx->stream>>>(ctx->d_reps, ctx->nrep);
+    CK(cudaGetLastError());
+    if (ctx->persist) {  // the whole step range in one cooperative launch
+        CK(cudaMemsetAsync(ctx->d_sync, 0, sizeof(GridSync), ctx->stream));
+        const RepDev* reps = ctx->d_reps;
+        int nrep = ctx->nrep, nst = need;
+        GridSync* gs = ctx->d_sync;
+        long long cap = ctx->spin_cap;
+        void* args[] = {(void*)&reps, (void*)&nrep, (void*)&nst, (void*)&gs, (void*)&cap};
+        CK(cudaLaunchCooperativeKernel((const void*)k_persist, dim3(ctx->grid_persist), dim3(kPersistThreads), args,
+                                       sizeof(AcceptSmem), ctx->stream));
+        return GCMC_OK;
+    }
+    return launch_steps(need, [&](int length) {
+        return cudaGraphLaunch(ctx->gexec[length], ctx->stream) == cudaSuccess ? GCMC_OK : GCMC_ERR_CUDA;
+    });
 }
 
 int gcmc_run_profiled(gcmc_ctx* ctx, int32_t nsteps, float* ms_energy, float* ms_accept, int32_t* move) {
