@@ -24,6 +24,12 @@ from . import values as V
 from ._native import check, lib
 
 
+def _dense(t):
+    """t with its elements in order in memory and no negation left to a view's bit: what a raw
+    pointer stands for."""
+    return t.resolve_neg().contiguous()
+
+
 def _p(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
 
@@ -49,10 +55,7 @@ class PoseEnergy(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, xyz, q, ff, centres, engine, rep, site_type, site_type_dev, self_res):
-        xyz = xyz.contiguous()
-        q = q.contiguous()
-        ff = ff.contiguous()
-        centres = centres.contiguous()
+        xyz, q, ff, centres = (_dense(t) for t in (xyz, q, ff, centres))
         P, ns = xyz.shape[0], xyz.shape[1]
         E = torch.empty(P, dtype=torch.float64, device=xyz.device)
         check(lib().gcmc_energy_grad(engine.handle, rep, _p(xyz), _p(q), _p(site_type_dev),
@@ -67,7 +70,7 @@ class PoseEnergy(torch.autograd.Function):
     def backward(ctx, gE):
         xyz, q, ff, centres = ctx.saved_tensors
         P, ns = xyz.shape[0], xyz.shape[1]
-        gE = gE.detach().to(torch.float64).contiguous()
+        gE = _dense(gE.detach().to(torch.float64))
         need_x, need_q, need_ff = ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.needs_input_grad[2]
         gxyz = torch.empty((P, ns, 3), dtype=torch.float64, device=xyz.device) if need_x else None
         gq = torch.empty((P, ns), dtype=torch.float64, device=xyz.device) if need_q else None
@@ -185,7 +188,7 @@ class RigidSites(torch.autograd.Function):
             c = torch.zeros_like(quat[:, :3], requires_grad=True)
             q = quat if quat.requires_grad else quat.detach().requires_grad_()
             return (*_grad_of(lambda: _sites_expression(c, q, tpl), (c, q), g), None)
-        g = g.resolve_neg().contiguous()
+        g = _dense(g)
         P, ns = g.shape[0], g.shape[1]
         gcom, gquat = unit.new_empty((P, 3)), torch.empty_like(unit)
         check(lib().gcmc_rigid_sites_grad(int(g.dtype == torch.float64), _p(unit), _p(norm), _p(tpl), _p(g), P, ns,
@@ -236,7 +239,7 @@ class LJPairs(torch.autograd.Function):
             e = eps if eps.requires_grad else eps.detach().requires_grad_()
             r = torch.zeros_like(eps, requires_grad=True)
             return (*_grad_of(lambda: _lj_expression(e, r, ctx.rows), (e, r), g), None)
-        e, g = eps.contiguous(), g.resolve_neg().contiguous()
+        e, g = eps.contiguous(), _dense(g)
         geps, grmin = torch.empty_like(e), torch.empty_like(e)
         check(lib().gcmc_lj_pairs_grad(int(e.dtype == torch.float64), _p(e), _p(g), e.shape[0], ctx.rows, _p(geps),
                                        _p(grmin), _stream()), "gcmc_lj_pairs_grad")
