@@ -41,3 +41,40 @@ def test_negated_views(protein_small, n):
         assert (a - b).norm() <= 0.01 * a.norm()
         E2 = pose_energy(eng, 0, *(torch._neg_view(-v) for v in (xyz, q, ff)), t, centres=torch._neg_view(-cen))
         assert np.array_equal(E.detach().cpu().numpy(), E2.cpu().numpy(), equal_nan=True)
+
+
+@pytest.mark.parametrize("ns", [20, 11, 3])
+def test_error_does_not_grow_with_the_poses(oracle_lib, protein_small, ns):
+    """A call of thousands of poses gives each one work item, a call of sixteen gives each many; the rounding
+    error of the charges' gradients against FP64 may not depend on that.  Root mean square over some
+    thousand sums of |terms|-normalised errors, whose own scatter is a few percent: 1.25 allowed (FP32 over a
+    whole staged batch: 1.8 with 20 sites)."""
+    import ctypes
+    from pygcmc_b200._native import check, lib
+    from pygcmc_b200.engine import Engine
+    s, n, few = protein_small, 4096, 16
+    g = np.random.default_rng(ns)
+    com, _ = PZ.random_poses(s, n, seed=ns)
+    cen = com.astype(np.float32)
+    xyz = (cen[:, None, :] + g.normal(size=(1, ns, 3))).astype(np.float32)
+    q = g.uniform(-0.5, 0.5, ns).astype(np.float32)
+    t = np.zeros(ns, np.int32)
+
+    def charge_gradients(eng, x, c):
+        d = [torch.tensor(a, device="cuda") for a in (x, q, t, c)]
+        out = torch.empty(x.shape[:2], dtype=torch.float64, device="cuda")
+        p = [ctypes.c_void_p(a.data_ptr()) for a in d]
+        check(lib().gcmc_energy_grad(eng.handle, 0, p[0], p[1], p[2], t.ctypes.data_as(ctypes.c_void_p), ns, p[3], None,
+                                     len(x), None, None, None, None, ctypes.c_void_p(out.data_ptr()), None,
+                                     ctypes.c_void_p(1)), "gcmc_energy_grad")
+        return out.cpu().numpy()
+    m = 320
+    with Engine(s.copy()) as eng:
+        many = charge_gradients(eng, xyz, cen)[:m]
+        alone = np.concatenate([charge_gradients(eng, xyz[i:i + few], cen[i:i + few]) for i in range(0, m, few)])
+    ref = oracle_lib.grad_batch(s, xyz[:m].astype(np.float64), q.astype(np.float64), t, cen[:m])
+    l1 = ref["gq_l1"]
+    ok = l1 > 0
+    err = [np.sqrt(np.mean(((v - ref["gq"])[ok] / l1[ok]) ** 2)) for v in (many, alone)]
+    print(ns, err)
+    assert err[0] <= 1.25 * err[1]
