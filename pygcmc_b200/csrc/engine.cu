@@ -410,9 +410,13 @@ struct StagingLease {
     std::unique_lock<std::mutex> lock{g_staging.m, std::try_to_lock};
     std::vector<char> own;
     cudaStream_t pending = nullptr;  // copies of the memory may be in flight on this stream
-    ~StagingLease() {  // (a call that fails half-way: its copies end before the next lease)
-        if (pending) cudaStreamSynchronize(pending);
+    // Waits for them (a call that fails half-way: its copies end before the next lease); an
+    // owner that destroys the stream first has to call this before.
+    void finish() {
+        if (pending && cudaStreamSynchronize(pending) != cudaSuccess) cudaGetLastError();
+        pending = nullptr;
     }
+    ~StagingLease() { finish(); }
     char* get(size_t bytes) {
         if (lock.owns_lock() && bytes <= kStagingMax) {
             if (bytes > g_staging.n) {
@@ -1699,6 +1703,7 @@ int create_impl(int nrep, const gcmc_replica_in* ins, const gcmc_options* optp, 
         if (err) st = (err & ERR_GRID_BITS) ? GCMC_ERR_ARG : GCMC_ERR_DEVICE;
     }
     if (st != GCMC_OK) {
+        staging.finish();  // before the stream goes
         cudaGetLastError();
         destroy_impl(ctx);
         return st;
