@@ -1981,9 +1981,17 @@ int order_after(gcmc_ctx* ctx, cudaStream_t s) {
 }
 
 
+int is_capturing(cudaStream_t s, bool* yes) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &c));
+    *yes = c != cudaStreamCaptureStatusNone;
+    return GCMC_OK;
+}
+
 // The context's device scratch, at least this large (scratch_mutex held).  The large
 // block is stream-ordered on the context's stream, which waits for every call's launches;
-// a caller's stream is ordered after it by order_before.
+// a caller's stream is ordered after it by order_before.  Not while that stream is being
+// captured: the block would belong to the graph, not to the context.
 int device_scratch(gcmc_ctx* ctx, size_t bytes, char** out) {
     if (bytes <= kScratchSmall) {
         *out = (char*)ctx->d_small;
@@ -2432,6 +2440,10 @@ int gcmc_energy_poses(gcmc_ctx* ctx, int32_t rep, const float* xyz, const float*
     RepHost& h = ctx->reps[rep];
     for (int s = 0; s < nsites; ++s)
         if (site_type[s] < 0 || site_type[s] >= h.ffX) return GCMC_ERR_ARG;
+    bool captured = false;
+    int st = is_capturing(ctx->stream, &captured);
+    if (st != GCMC_OK) return st;
+    if (captured) return GCMC_ERR_CUDA;  // (the call waits for its results)
     const int nslab = pose_splits(ctx, h, nposes);
     // The poses go through the kept page-locked scratch in blocks: while the GPU evaluates
     // one, the host copies the next one in.  A block's inputs are one copy, the results of
@@ -2454,7 +2466,7 @@ int gcmc_energy_poses(gcmc_ctx* ctx, int32_t rep, const float* xyz, const float*
     const size_t parts = nslab > 1 ? (size_t)std::min(kBlock, round) * nslab : 0;  // of a block
     const size_t d_part = dc.take(sizeof(double) * parts), d_ngp = dc.take(sizeof(int) * parts);
     char *hb = staging.get(hc.at), *db = nullptr;
-    int st = device_scratch(ctx, dc.at, &db);
+    st = device_scratch(ctx, dc.at, &db);
     if (st != GCMC_OK) return st;
     if ((st = pme_update(ctx, rep, 1, s)) != GCMC_OK) return st;
     staging.pending = s;
@@ -2520,15 +2532,17 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
     const size_t o_g = c.take(grads ? sizeof(double4) * nposes * nslab * nsites : 0);
     const size_t o_glj = c.take(d_gff ? sizeof(double) * ntab * 2 : 0);
     // scratch: the context's, or for a large call or one that is being captured into a
-    // graph (whose replays are not ordered against other calls) an allocation of its own.
+    // graph (whose replays are not ordered against other calls; a stream joins the context's
+    // capture in order_before) an allocation of its own.
     // (Five stream-ordered allocations a call, whose pool a synchronising caller empties
     // each time, cost more than the kernels.)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(s, &cap));
-    const bool own = cap != cudaStreamCaptureStatusNone || c.at > kScratchMax;
+    bool captured = false, joins = false;
+    int st = is_capturing(s, &captured);
+    if (st == GCMC_OK) st = is_capturing(ctx->stream, &joins);
+    if (st != GCMC_OK) return st;
+    const bool own = captured || joins || c.at > kScratchMax;
     std::unique_lock<std::mutex> lock(ctx->scratch_mutex, std::defer_lock);
     char* w = nullptr;
-    int st = GCMC_OK;
     if (!own) {  // held until the call is ordered before the next one that uses the scratch
         lock.lock();
         if ((st = device_scratch(ctx, c.at, &w)) != GCMC_OK) return st;
