@@ -2583,8 +2583,9 @@ int gcmc_energy_grad(gcmc_ctx* ctx, int32_t rep, const float* d_xyz, const float
         if (cudaGetLastError() != cudaSuccess) st = GCMC_ERR_CUDA;
     }
     if (own && w) cudaFreeAsync(w, s);
-    if (st == GCMC_OK) st = order_after(ctx, s);
-    return st;
+    // (after a failure too: what was launched before it still uses the scratch)
+    const int ost = order_after(ctx, s);
+    return st != GCMC_OK ? st : ost;
 }
 
 int gcmc_rigid_sites(int32_t f64, const void* d_com, const void* d_unit, const void* d_template, int32_t nposes,

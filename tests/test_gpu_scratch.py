@@ -75,3 +75,34 @@ def test_gradients_on_a_stream_that_joins_a_capture(protein_small):
         want, _ = e.energy_poses(xyz, q, t, cen)
         assert np.array_equal(out[1].cpu().numpy(), want, equal_nan=True)
         assert not out[0].any()  # captured, and never launched
+
+
+def test_failed_gradients_keep_their_place(protein_small):
+    """A gradient call that fails after its first launches (here on the error of a call before it) still has the
+    context's stream wait for them, as they use the scratch that the next call takes."""
+    import torch
+    from pygcmc_b200._native import lib
+    from pygcmc_b200.engine import Engine
+    stream, side = torch.cuda.Stream(), torch.cuda.Stream()
+    xyz, q, t, cen = _poses(protein_small, 64)
+    d = [torch.tensor(a, device="cuda") for a in (xyz, q, t, cen)]
+    out = torch.empty(64, dtype=torch.float64, device="cuda")
+    done = torch.cuda.Event()
+    with Engine(protein_small.copy(), stream=stream.cuda_stream) as e:
+        want, _ = e.energy_poses(xyz, q, t, cen)
+        torch.cuda.synchronize()
+        with _capture(stream.cuda_stream):
+            assert lib().gcmc_sync(e.handle) == 1
+        p = [ctypes.c_void_p(a.data_ptr()) for a in d]
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(1_000_000_000)  # about half a second
+            st = lib().gcmc_energy_grad(e.handle, 0, p[0], p[1], p[2], t.ctypes.data_as(ctypes.c_void_p), xyz.shape[1],
+                                        p[3], None, 64, None, None, ctypes.c_void_p(out.data_ptr()), None, None, None,
+                                        ctypes.c_void_p(side.cuda_stream))
+            done.record()
+        assert st == 1
+        assert not done.query()
+        got, _ = e.energy_poses(xyz, q, t, cen)
+        assert done.query()
+        assert np.array_equal(got, want, equal_nan=True)
+        torch.cuda.synchronize()
