@@ -178,16 +178,18 @@ class RigidSites(torch.autograd.Function):
         out = torch.empty((P, ns, 3), dtype=com.dtype, device=com.device)
         check(lib().gcmc_rigid_sites(int(com.dtype == torch.float64), _p(com_c), _p(unit), _p(tpl), P, ns, _p(out),
                                      _stream()), "gcmc_rigid_sites")
-        ctx.save_for_backward(quat, tpl, unit, norm)  # (no gradient needs com, which may change)
+        # (no gradient needs com, and the centres' needs none of the others: those may change)
+        ctx.save_for_backward(*((quat, tpl, unit, norm) if ctx.needs_input_grad[1] else ()))
         return out
 
     @staticmethod
     def backward(ctx, g):
+        if not ctx.needs_input_grad[1]:
+            return g.sum(1), None, None
         quat, tpl, unit, norm = ctx.saved_tensors
         if _expression_backward(g):
             c = torch.zeros_like(quat[:, :3], requires_grad=True)
-            q = quat if quat.requires_grad else quat.detach().requires_grad_()
-            return (*_grad_of(lambda: _sites_expression(c, q, tpl), (c, q), g), None)
+            return (*_grad_of(lambda: _sites_expression(c, quat, tpl), (c, quat), g), None)
         g = _dense(g)
         P, ns = g.shape[0], g.shape[1]
         gcom, gquat = unit.new_empty((P, 3)), torch.empty_like(unit)
