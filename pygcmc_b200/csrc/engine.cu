@@ -34,7 +34,7 @@ namespace {
 // short one for the rest (a graph's steps past the run's end are empty launches, about 6 us
 // each: with the long one alone a 24-step run paid 8 of them).
 constexpr int kGraphSteps[2] = {32, 8};
-static_assert(kGraphSteps[0] % 2 == 0 && kGraphSteps[1] % 2 == 0, "a speculating graph ends on its start parity");
+static_assert(kGraphSteps[0] % 2 == 0 && kGraphSteps[1] % 2 == 0, "a speculating graph ends on the copy it began with");
 constexpr int kMaxRep = 256;
 thread_local int g_last_status = GCMC_OK;
 
@@ -183,12 +183,10 @@ struct gcmc_ctx {
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // of kGraphSteps[0], [1] steps
     // speculation (one replica, one branch, no PME, no force bias): the next step's pose
     // energies run beside the accept kernel; a second descriptor copy holds every other
-    // step's scratch, and the step loop has one graph per parity of its first step
+    // step's scratch, a run's first step in the first copy
     bool spec = false;
     RepDev repdev_b{};
     RepDev* d_reps_b = nullptr;
-    // (made when first needed: a run that starts at an odd step is rare)
-    cudaGraphExec_t gexec_spec[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [parity][length]
     bool spec_pdl = true;  // the driver captures programmatic launches
     std::vector<cudaStream_t> side;  // side streams of the captures, made once
     int per_sm_e = 1;      // pose-energy CTAs per SM
@@ -1368,14 +1366,15 @@ void split_branches(gcmc_ctx* ctx, int nb) {
 // to the context's stream, so one branch's accept kernel (a CTA per replica)
 // overlaps another's pose energies; each branch gets a share of the
 // pose-energy grid in proportion to its atoms.
-// Speculating (one replica): step j (descriptor copy j & 1) is, on the
+// Speculating (one replica): step j of a run (descriptor copy j & 1) is, on the
 // context's stream, F_p (prepare it again unless its speculation stands), F_e
 // (its pose energies unless they stand) and A (accept).  On a second stream P
 // prepares step j + 1 in the other copy as soon as A of step j - 1 is done (as
 // if step j accepts nothing), and on a third S evaluates its pose energies
 // once P and F_e are done, on the SMs that A leaves free, stopping early when
-// A accepts a move.  F_p of step j + 1 waits for A and S.  One graph per
-// parity of the run's first step (the lengths are even) and length.
+// A accepts a move.  F_p of step j + 1 waits for A and S.  One graph per length;
+// the lengths are even, so that each graph of a run starts at the first copy.
+
 // Launch of `kernel` on s as a programmatic dependent of the kernel before it in
 // s: it may be scheduled once every CTA of that kernel has triggered (pdl_trigger)
 // and waits in pdl_wait for that kernel's results, so its launch latency overlaps
@@ -1396,8 +1395,6 @@ cudaError_t launch_dependent(void (*kernel)(Args...), int grid, int block, size_
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// pdl: the step's completion pose-energy launch and accept kernel as programmatic
-// dependents of the kernels before them (F_p -> F_e -> accept).
 // At least n side streams for captures.
 int side_streams(gcmc_ctx* ctx, int n) {
     while ((int)ctx->side.size() < n) {
@@ -1411,7 +1408,9 @@ int side_streams(gcmc_ctx* ctx, int n) {
     return GCMC_OK;
 }
 
-int build_spec_graph(gcmc_ctx* ctx, int parity, int length, bool pdl) {
+// pdl: the step's completion pose-energy launch and accept kernel as programmatic
+// dependents of the kernels before them (F_p -> F_e -> accept).
+int build_spec_graph(gcmc_ctx* ctx, int length, bool pdl) {
     constexpr int N = kGraphSteps[0];
     const int steps = kGraphSteps[length];
     cudaEvent_t ev[4 * N + 1] = {};
@@ -1433,8 +1432,8 @@ int build_spec_graph(gcmc_ctx* ctx, int parity, int length, bool pdl) {
         cudaError_t e = cudaEventRecord(ev[4 * N], main);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(sp, ev[4 * N], 0);
         for (int i = 0; i < steps && e == cudaSuccess; ++i) {
-            const RepDev* cur = ((parity + i) & 1) ? ctx->d_reps_b : ctx->d_reps;
-            const RepDev* nxt = ((parity + i) & 1) ? ctx->d_reps : ctx->d_reps_b;
+            const RepDev* cur = (i & 1) ? ctx->d_reps_b : ctx->d_reps;
+            const RepDev* nxt = (i & 1) ? ctx->d_reps : ctx->d_reps_b;
             if (i > 0) e = cudaStreamWaitEvent(main, evS[i - 1], 0);
             k_prep_spec<<<1, kAcceptThreads, prep_smem(ctx), main>>>(cur, 1);
             if (pdl && !ctx->tiled) {
@@ -1470,28 +1469,12 @@ int build_spec_graph(gcmc_ctx* ctx, int parity, int length, bool pdl) {
             st = GCMC_ERR_CUDA;
         }
     }
-    if (st == GCMC_OK && cudaGraphInstantiate(&ctx->gexec_spec[parity][length], graph, 0) != cudaSuccess) st = GCMC_ERR_CUDA;
+    if (st == GCMC_OK && cudaGraphInstantiate(&ctx->gexec[length], graph, 0) != cudaSuccess) st = GCMC_ERR_CUDA;
     if (graph) cudaGraphDestroy(graph);
     for (auto& e : ev)
         if (e) cudaEventDestroy(e);
     if (st != GCMC_OK) cudaGetLastError();
     return st;
-}
-
-// The speculating graph of this parity and length, captured if it is not there yet.
-int spec_graph(gcmc_ctx* ctx, int parity, int length, cudaGraphExec_t* out) {
-    cudaGraphExec_t& x = ctx->gexec_spec[parity][length];
-    if (!x) {
-        int st = build_spec_graph(ctx, parity, length, ctx->spec_pdl);
-        if (st != GCMC_OK && ctx->spec_pdl) {  // a driver that cannot capture programmatic launches: plain ones
-            cudaGetLastError();
-            ctx->spec_pdl = false;
-            st = build_spec_graph(ctx, parity, length, false);
-        }
-        if (st != GCMC_OK) return st;
-    }
-    *out = x;
-    return GCMC_OK;
 }
 
 void destroy_graphs(gcmc_ctx* ctx) {
@@ -1500,8 +1483,6 @@ void destroy_graphs(gcmc_ctx* ctx) {
         x = nullptr;
     };
     for (auto& x : ctx->gexec) drop(x);
-    for (auto& p : ctx->gexec_spec)
-        for (auto& x : p) drop(x);
 }
 
 int build_plain_graph(gcmc_ctx* ctx, int length) {
@@ -1563,8 +1544,11 @@ int build_graph(gcmc_ctx* ctx) {
     destroy_graphs(ctx);
     int st = GCMC_OK;
     for (int length = 0; length < 2 && st == GCMC_OK; ++length) {
-        cudaGraphExec_t x;
-        st = ctx->spec ? spec_graph(ctx, 0, length, &x) : build_plain_graph(ctx, length);
+        st = ctx->spec ? build_spec_graph(ctx, length, ctx->spec_pdl) : build_plain_graph(ctx, length);
+        if (st != GCMC_OK && ctx->spec && ctx->spec_pdl) {  // a driver that cannot capture programmatic launches
+            ctx->spec_pdl = false;
+            st = build_spec_graph(ctx, length, false);
+        }
     }
     return st;
 }
@@ -1750,7 +1734,7 @@ int refill_impl(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins, const gcmc_
     const int fb = opt.proposal == 2 ? 1 : 0;
     const int evar = opt.energy_variant == 1 ? 1 : 0;
     const bool persist_before = ctx->persist;
-    const bool had_graph = ctx->gexec[0] || ctx->gexec_spec[0][0];
+    const bool had_graph = ctx->gexec[0] != nullptr;
     const bool shape_changed = spec_changed || nb != ctx->branches || opt.energy_blocks_per_sm != ctx->ebps ||
                                fb != ctx->fb || evar != ctx->evar || ctx->tiled != tiled_before ||
                                ctx->pme_any != pme_before || pme_meshes(ctx) != mesh_before ||
@@ -2218,16 +2202,10 @@ int gcmc_run(gcmc_ctx* ctx, int32_t nsteps) {
     }
     if (need == 0) return GCMC_OK;
     k_set_run_end<<<(ctx->nrep + 127) / 128, 128, 0, ctx->stream>>>(ctx->d_reps, ctx->nrep, nsteps);
-    if (ctx->spec) {  // step `first` lives in descriptor copy first & 1
-        k_spec_start<<<1, 32, 0, ctx->stream>>>((first & 1) ? ctx->d_reps_b : ctx->d_reps, first);
-        CK(cudaGetLastError());
-        return launch_steps(need, [&](int length) {
-            cudaGraphExec_t x;
-            const int st = spec_graph(ctx, first & 1, length, &x);
-            return st != GCMC_OK ? st : (cudaGraphLaunch(x, ctx->stream) == cudaSuccess ? GCMC_OK : GCMC_ERR_CUDA);
-        });
-    }
-    k_prepare<<<ctx->nrep, kAcceptThreads, prep_smem(ctx), ctx->stream>>>(ctx->d_reps, ctx->nrep);
+    if (ctx->spec)  // (a run's first step is in the first descriptor copy)
+        k_spec_start<<<1, 32, 0, ctx->stream>>>(ctx->d_reps, first);
+    else
+        k_prepare<<<ctx->nrep, kAcceptThreads, prep_smem(ctx), ctx->stream>>>(ctx->d_reps, ctx->nrep);
     CK(cudaGetLastError());
     if (ctx->persist) {  // the whole step range in one cooperative launch
         CK(cudaMemsetAsync(ctx->d_sync, 0, sizeof(GridSync), ctx->stream));
