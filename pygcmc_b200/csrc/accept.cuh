@@ -745,7 +745,7 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
         // The sequential definition: seed = lowest unused pose, members = unused
         // poses within the cutoff of the seed, decision, then the members (and on
         // acceptance the unused poses within the cutoff of the chosen pose) leave
-        // the unused set.  Each round, warp 0 seeds up to a warp's worth (at most 32) clusters ahead
+        // the unused set.  Each round, warp 0 seeds up to a cluster per warp (at most 32) ahead
         // assuming no acceptance; all warps evaluate them in parallel (member
         // count, Gumbel argmax and the decision for the round's range of K, see
         // eval_cluster); warp 0 then commits them in order.  A speculative cluster is exactly
@@ -1049,8 +1049,7 @@ __device__ __forceinline__ void accept_step(const RepDev& R, int spec, unsigned 
 template <bool Pme>
 __global__ void __launch_bounds__(kAcceptThreads, 1) k_accept(const RepDev* __restrict__ reps, int nrep, int spec) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    pdl_wait();  // one-replica graphs launch this kernel as a dependent of the pose energies
-    pdl_trigger();
+    pdl_wait();  // a speculating graph launches this kernel as a dependent of the pose energies
     accept_step<Pme>(reps[blockIdx.x], spec, smem_raw);
 }
 template __global__ void k_accept<false>(const RepDev* __restrict__, int, int);
