@@ -138,16 +138,35 @@ def _plain_cuda(com, quat, tpl):
             and not (tpl.requires_grad or tpl.is_neg()))
 
 
+def _torch_hooks():
+    """torch's functions that say whether something has to see the tensor operations themselves, or
+    None where this torch lacks one of them: the tensor expressions then serve every call."""
+    try:
+        torch.autograd.forward_ad._current_level
+        return (torch._C._functorch.peek_interpreter_stack,
+                torch.utils._python_dispatch._get_current_dispatch_mode, torch.compiler.is_compiling,
+                torch._C._has_storage)
+    except AttributeError:
+        return None
+
+
+_HOOKS = _torch_hooks()
+
+
+def _watched():
+    if _HOOKS is None:
+        return True
+    transforms, dispatch_mode, compiling, _ = _HOOKS
+    return (torch.is_autocast_enabled() or torch.jit.is_tracing() or compiling() or transforms() is not None
+            or torch.autograd.forward_ad._current_level >= 0 or dispatch_mode() is not None)
+
+
 def _plain(a, b):
     """Two dense tensors of one floating type on the current GPU, and nothing that has to see the
     tensor operations on them."""
     return (type(a) in _TENSORS and type(b) in _TENSORS and a.is_cuda and a.dtype in (torch.float32, torch.float64)
             and b.dtype == a.dtype and b.device == a.device and a.device.index == torch.cuda.current_device()
-            and not (a.is_neg() or b.is_neg())
-            and not (torch.is_autocast_enabled() or torch.jit.is_tracing() or torch.compiler.is_compiling())
-            and torch._C._functorch.peek_interpreter_stack() is None
-            and torch.autograd.forward_ad._current_level < 0
-            and torch.utils._python_dispatch._get_current_dispatch_mode() is None)
+            and not (a.is_neg() or b.is_neg() or _watched()))
 
 
 _TENSORS = (torch.Tensor, torch.nn.Parameter)
@@ -156,7 +175,7 @@ _TENSORS = (torch.Tensor, torch.nn.Parameter)
 def _expression_backward(g):
     """Whether a backward pass has to be the tensor expression's: it is to be differentiated
     (create_graph), or runs for a batch of gradients at once (is_grads_batched, vmap)."""
-    return torch.is_grad_enabled() or not torch._C._has_storage(g)
+    return torch.is_grad_enabled() or not _HOOKS[3](g)
 
 
 def _grad_of(expression, inputs, g):
