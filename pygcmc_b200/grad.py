@@ -157,16 +157,17 @@ def _watched():
     if _HOOKS is None:
         return True
     transforms, dispatch_mode, compiling, _ = _HOOKS
-    return (torch.is_autocast_enabled() or torch.jit.is_tracing() or compiling() or transforms() is not None
+    # (a compiler must not meet anything but the first question)
+    return (compiling() or torch.is_autocast_enabled() or torch.jit.is_tracing() or transforms() is not None
             or torch.autograd.forward_ad._current_level >= 0 or dispatch_mode() is not None)
 
 
 def _plain(a, b):
     """Two dense tensors of one floating type on the current GPU, and nothing that has to see the
     tensor operations on them."""
-    return (type(a) in _TENSORS and type(b) in _TENSORS and a.is_cuda and a.dtype in (torch.float32, torch.float64)
-            and b.dtype == a.dtype and b.device == a.device and a.device.index == torch.cuda.current_device()
-            and not (a.is_neg() or b.is_neg() or _watched()))
+    return (not _watched() and type(a) in _TENSORS and type(b) in _TENSORS and a.is_cuda
+            and a.dtype in (torch.float32, torch.float64) and b.dtype == a.dtype and b.device == a.device and a.device.index == torch.cuda.current_device()
+            and not (a.is_neg() or b.is_neg()))
 
 
 _TENSORS = (torch.Tensor, torch.nn.Parameter)

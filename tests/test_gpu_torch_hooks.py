@@ -37,3 +37,24 @@ def test_missing_names_mean_the_expression(monkeypatch, holder, name):
     assert fused == (holder is None), node
     for a, b in zip(got, want[1]):
         assert torch.allclose(a, b, rtol=1e-11, atol=1e-11)
+
+
+@pytest.mark.parametrize("backend", ["eager", "aot_eager"])
+def test_compiled_whole(backend):
+    """Under a compiler that allows no break in the graph the sites and the pair table are the expressions, with
+    their gradients."""
+    import pygcmc_b200.grad as grad
+    g = torch.Generator().manual_seed(6)
+    com, quat, tpl = (torch.randn(s, generator=g, dtype=torch.float64).cuda() for s in ((16, 3), (16, 4), (5, 3)))
+    par = [0.1 + torch.rand(9, generator=g, dtype=torch.float64).cuda() for _ in range(2)]
+    frag = type("Frag", (), {"template": tpl})
+    for f, ref, inputs in (
+            (lambda c, q: grad.RigidFragment.sites(frag, c, q), lambda c, q: grad._sites_expression(c, q, tpl), (com, quat)),
+            (lambda e, r: grad.lj_table(e, r, 4), lambda e, r: grad._lj_expression(e, r, 4), par)):
+        got = []
+        for fn in (torch.compile(f, backend=backend, fullgraph=True), ref):
+            leaves = [v.clone().requires_grad_() for v in inputs]
+            out = fn(*leaves)
+            got.append([out, *torch.autograd.grad((out * out).sum(), leaves)])
+        for a, b in zip(*got):
+            assert torch.allclose(a, b, rtol=1e-11, atol=1e-11)
