@@ -1734,7 +1734,6 @@ int refill_impl(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins, const gcmc_
     const int fb = opt.proposal == 2 ? 1 : 0;
     const int evar = opt.energy_variant == 1 ? 1 : 0;
     const bool persist_before = ctx->persist;
-    const bool had_graph = ctx->gexec[0] != nullptr;
     const bool shape_changed = spec_changed || nb != ctx->branches || opt.energy_blocks_per_sm != ctx->ebps ||
                                fb != ctx->fb || evar != ctx->evar || ctx->tiled != tiled_before ||
                                ctx->pme_any != pme_before || pme_meshes(ctx) != mesh_before ||
@@ -1748,7 +1747,8 @@ int refill_impl(gcmc_ctx* ctx, int nrep, const gcmc_replica_in* ins, const gcmc_
         st = set_energy_grid(ctx, opt.energy_blocks_per_sm);
         if (st != GCMC_OK) return st;
         split_branches(ctx, nb);
-        if (!ctx->persist && (shape_changed || !had_graph)) {
+        if (shape_changed) destroy_graphs(ctx);  // (a persistent loop has none, and leaves none of another shape)
+        if (!ctx->persist && !ctx->gexec[0]) {
             st = build_graph(ctx);
             if (st != GCMC_OK) return st;
         }

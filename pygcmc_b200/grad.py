@@ -166,7 +166,8 @@ def _plain(a, b):
     """Two dense tensors of one floating type on the current GPU, and nothing that has to see the
     tensor operations on them."""
     return (not _watched() and type(a) in _TENSORS and type(b) in _TENSORS and a.is_cuda
-            and a.dtype in (torch.float32, torch.float64) and b.dtype == a.dtype and b.device == a.device and a.device.index == torch.cuda.current_device()
+            and a.dtype in (torch.float32, torch.float64) and b.dtype == a.dtype and b.device == a.device
+            and a.device.index == torch.cuda.current_device()
             and not (a.is_neg() or b.is_neg()))
 
 

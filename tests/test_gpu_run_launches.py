@@ -35,3 +35,38 @@ def test_runs_capture_nothing(protein_small, kernel):
     assert np.array_equal(whole.fragmentInfo["totalNum"], parts.fragmentInfo["totalNum"])
     assert np.array_equal(whole.atomInfo["position"], parts.atomInfo["position"])
     assert np.array_equal(whole.residueInfo["position"], parts.residueInfo["position"])
+
+
+def test_no_graph_of_another_shape(protein_small):
+    """A kept batch context whose calls go from a graph of one kernel to the persistent loop of another and from
+    there to a graph of that kernel: each call gives the chains of a fresh context."""
+    from pygcmc_b200._native import default_options, lib
+    from pygcmc_b200.engine import Engine
+    from pygcmc_b200.gpu import runGCMC_batch
+    n = 48
+
+    def replicas():
+        out = []
+        for r in range(2):
+            s = protein_small.copy()
+            s.SimInfo = s.SimInfo.copy()
+            s.SimInfo[0]["mcsteps"] = n
+            s.SimInfo[0]["seed"] = 17 + r
+            s.moveArray = np.ascontiguousarray(s.moveArray[:n])
+            out.append(s)
+        return out
+    assert lib().gcmc_release_cache() == 0
+    for kernel, persistent in ((1, 0), (0, 1), (0, 0), (1, 0), (0, 1), (1, 0)):
+        opts = default_options(energy_kernel=kernel, persistent=persistent)
+        got = replicas()
+        runGCMC_batch(got, opts)
+        with Engine(replicas(), opts) as e:
+            e.run(n)
+            e.sync()
+            for r, s in enumerate(got):
+                want = e.download(r)
+                assert np.array_equal(s.fragmentInfo["totalNum"], want.fragmentInfo["totalNum"])
+                for f in want.fragmentInfo:
+                    a, b = int(f["startRes"]), int(f["startRes"]) + int(f["totalNum"])
+                    assert np.array_equal(s.residueInfo["position"][a:b], want.residueInfo["position"][a:b])
+    assert lib().gcmc_release_cache() == 0
