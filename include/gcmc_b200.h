@@ -221,7 +221,10 @@ int gcmc_run_gcmc(const InfoStruct* info, AtomArray* fragmentInfo, residue* resi
                   Atom* atomInfo, const float* grid, const float* ff, const int* moveArray,
                   const gcmc_options* opt);
 /* Free the device contexts kept between runGCMC_cuda / gcmc_run_gcmc /
- * gcmc_run_batch calls. */
+ * gcmc_run_batch calls, the page-locked staging block that all contexts share
+ * (16 MiB at most), and the scratch that the contexts in use keep for large
+ * gcmc_energy_poses / gcmc_energy_grad calls (64 MiB at most each; it is back
+ * with the driver once the context's stream has been waited for). */
 int gcmc_release_cache(void);
 
 /* Batched drop-in (no counterpart in the reference, which runs one system per

@@ -1565,8 +1565,17 @@ int launch_steps(int need, F fn) {
     return st;
 }
 
+// The contexts in use, whose scratch gcmc_release_cache gives back (the list is never
+// destroyed: a context may be, after the process's static objects).
+std::mutex g_live_mutex;
+std::vector<gcmc_ctx*>& g_live = *new std::vector<gcmc_ctx*>;
+
 int destroy_impl(gcmc_ctx* ctx) {
     if (!ctx) return GCMC_OK;
+    {
+        std::lock_guard<std::mutex> lock(g_live_mutex);
+        g_live.erase(std::remove(g_live.begin(), g_live.end(), ctx), g_live.end());
+    }
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     destroy_graphs(ctx);
     for (auto s : ctx->side) cudaStreamDestroy(s);
@@ -1691,6 +1700,10 @@ int create_impl(int nrep, const gcmc_replica_in* ins, const gcmc_options* optp, 
         cudaGetLastError();
         destroy_impl(ctx);
         return st;
+    }
+    {
+        std::lock_guard<std::mutex> lock(g_live_mutex);
+        g_live.push_back(ctx);
     }
     *out = ctx;
     return GCMC_OK;
@@ -1991,6 +2004,16 @@ int device_scratch(gcmc_ctx* ctx, size_t bytes, char** out) {
     }
     *out = (char*)ctx->d_scratch;
     return GCMC_OK;
+}
+
+// The large block goes back, behind the calls that use it; the next call that needs one allocates.
+void release_scratch(gcmc_ctx* ctx) {
+    std::lock_guard<std::mutex> lock(ctx->scratch_mutex);
+    bool captured = true;
+    if (!ctx->d_scratch || is_capturing(ctx->stream, &captured) != GCMC_OK || captured) return;
+    if (cudaFreeAsync(ctx->d_scratch, ctx->stream) != cudaSuccess) cudaGetLastError();
+    ctx->d_scratch = nullptr;
+    ctx->d_scratch_bytes = 0;
 }
 
 // The numbers of the pair table's expression, rounded as it rounds them.
@@ -2670,6 +2693,8 @@ int gcmc_release_cache(void) {
     if (g_staging.p) cudaFreeHost(g_staging.p);
     g_staging.p = nullptr;
     g_staging.n = 0;
+    std::lock_guard<std::mutex> live(g_live_mutex);
+    for (gcmc_ctx* ctx : g_live) release_scratch(ctx);
     return GCMC_OK;
 }
 

@@ -106,3 +106,42 @@ def test_failed_gradients_keep_their_place(protein_small):
         assert done.query()
         assert np.array_equal(got, want, equal_nan=True)
         torch.cuda.synchronize()
+
+
+def test_scratch_is_given_back(protein_small):
+    """gcmc_release_cache frees the large scratch of a context in use, and the context works on; with other
+    contexts made and closed before it."""
+    import torch
+    from pygcmc_b200._native import lib
+    from pygcmc_b200.engine import Engine
+    n = 120000
+    xyz, q, t, cen = (torch.tensor(a, device="cuda") if i != 2 else a for i, a in enumerate(_poses(protein_small, n)))
+    tt = torch.tensor(t, device="cuda")
+    out = torch.empty((3,) + xyz.shape, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+
+    def call(e, row):
+        p = [ctypes.c_void_p(a.data_ptr()) for a in (xyz, q, tt, cen)]
+        assert lib().gcmc_energy_grad(e.handle, 0, p[0], p[1], p[2], t.ctypes.data_as(ctypes.c_void_p), xyz.shape[1],
+                                      p[3], None, n, None, None, None, ctypes.c_void_p(out[row].data_ptr()), None,
+                                      None, None) == 0
+        e.sync()
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+    Engine(protein_small.copy()).close()
+    with Engine(protein_small.copy()) as e:
+        call(e, 0)  # (the kernel's one-time device memory)
+        held = 32 * n * xyz.shape[1]
+        assert 8 << 20 < held < 64 << 20
+        before = free()
+        assert lib().gcmc_release_cache() == 0
+        e.sync()
+        assert free() - before > held // 2
+        call(e, 1)
+        assert lib().gcmc_release_cache() == 0  # while its launches may run
+        call(e, 2)
+    assert lib().gcmc_release_cache() == 0
+    a, b, c = (v.cpu().numpy() for v in out)
+    assert np.array_equal(a, b, equal_nan=True) and np.array_equal(a, c, equal_nan=True)
