@@ -254,7 +254,7 @@ def run_ours(args, ws, rank, local, kind="protein"):
     # replica) re-prepare + completion + accept + speculative prepare + speculative
     # energies; per run call: run-end update + start-step set-up
     speculating = opts.speculate >= 0 and opts.branches <= 1
-    launches = args.steps * (2 + (5 if speculating else 2) * 32 * ((chunk + 31) // 32))
+    launches = args.steps * run_launches(chunk, 5 if speculating else 2)
     out = {
         "metric": METRIC, "value": round(value, 1), "unit": "moves/s", "n_gpus": ws, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(ms / args.steps, 3), "higher_is_better": True,
@@ -386,7 +386,8 @@ def run_ours_batched(args, ws, rank, local):
     sm_max = (clk or {}).get("sm_max_mhz") or 1965.0
     peak, sms = nominal_fp32_tflops(sm_max)
     achieved = pairs_prof * FLOPS_PER_PAIR / (e_ms / 1e3) / 1e12
-    launches = args.steps * (2 + 2 * 32 * best.branches * ((chunk + 31) // 32))
+    # (the persistent loop is one launch)
+    launches = args.steps * (3 if best.persistent > 0 else run_launches(chunk, 2 * best.branches))
     out = {
         "metric": METRIC, "value": round(moves_all / (ms / 1e3), 1), "unit": "moves/s", "n_gpus": ws,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms / args.steps, 3),
@@ -815,7 +816,7 @@ def run_ours_large(args, ws, rank, local):
         # per chunk: k_set_run_end, k_prepare; per graph step and branch: three mesh-update
         # launches (which return at once when no charge moved), then per branch two force-bias
         # pose-energy launches and the accept kernel
-        "gpu_launches": args.steps * (2 + 32 * ((chunk + 31) // 32) * 6 * opt.branches),
+        "gpu_launches": args.steps * run_launches(chunk, 6 * opt.branches),
         "clocks": clk,
     }
 
@@ -956,6 +957,15 @@ def run_probe(args):
         print(json.dumps({"move": (mv % 4).tolist(), "energy_us": [round(float(x) * 1e3, 2) for x in te],
                           "accept_us": [round(float(x) * 1e3, 2) for x in ta], "counters": eng.counters(),
                           "accept_phase_cycles": eng.phase_cycles().tolist()}))
+
+
+def run_launches(nsteps, per_step):
+    """Kernels a run call of the step loop launches: two for its start, then per_step for every step of
+    its graphs, the 32-step one while more than 24 steps remain and the 8-step one after that."""
+    captured = 0
+    while captured < nsteps:
+        captured += 32 if nsteps - captured > 24 else 8
+    return 2 + per_step * captured
 
 
 def barrier(ws):
