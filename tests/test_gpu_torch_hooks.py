@@ -49,7 +49,8 @@ def test_compiled_whole(backend):
     par = [0.1 + torch.rand(9, generator=g, dtype=torch.float64).cuda() for _ in range(2)]
     frag = type("Frag", (), {"template": tpl})
     for f, ref, inputs in (
-            (lambda c, q: grad.RigidFragment.sites(frag, c, q), lambda c, q: grad._sites_expression(c, q, tpl), (com, quat)),
+            (lambda c, q: grad.RigidFragment.sites(frag, c, q), lambda c, q: grad._sites_expression(c, q, tpl),
+             (com, quat)),
             (lambda e, r: grad.lj_table(e, r, 4), lambda e, r: grad._lj_expression(e, r, 4), par)):
         got = []
         for fn in (torch.compile(f, backend=backend, fullgraph=True), ref):
